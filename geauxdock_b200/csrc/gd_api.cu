@@ -1063,15 +1063,33 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
   TileConfig tc{8, o.kpl, o.ab};
   default_pair_tile(1, tc.kpl, tc.ab);
   if (precision == GD_PREC_FP64) tc.kpl = 1, tc.ab = 8;
-  int kst = precision == GD_PREC_FP64 ? J.nkde : 0;  // FP32: KDE points through L1
-  int P = e->Pmax;
-  if (kernel_smem_bytes(P, 0, e->lig_slots, tc.warps_per_cta, precision) > kSmemLimit) P = 0;  // through L1
-  size_t smem = kernel_smem_bytes(P, kst, e->lig_slots, tc.warps_per_cta, precision);
-  if (smem > kSmemLimit) {
-    kst = 0;
-    smem = kernel_smem_bytes(P, kst, e->lig_slots, tc.warps_per_cta, precision);
-  }
-  if (smem > kSmemLimit) return fail(GD_E_CAPACITY, "ligand slots too large for shared memory");
+  // The pocket staged in shared memory or read through L1, and the poses per CTA: what keeps
+  // the most poses in flight (ties: staged, 8 poses).  A 64-atom ligand against 3000 points
+  // staged is 136 KB a CTA, so one CTA of 8 warps per SM: 16384 poses 6.26 ms; through L1
+  // three CTAs fit, 24 warps: 3.96 ms (FP64, 2048 poses on 8 and 16 warps: 8.89 and 5.12 ms).
+  int nsm = 0;
+  GD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device));
+  int kst = 0, P = 0, occ = 0;
+  long long flight = 0;
+  for (const bool staged : {true, false})
+    for (int w : {8, 12, 16, 4, 2, 1}) {
+      TileConfig t = tc;
+      t.warps_per_cta = w;
+      const int tp = staged ? e->Pmax : 0;
+      int tk = precision == GD_PREC_FP64 ? J.nkde : 0;  // FP32: KDE points through L1
+      size_t ts = kernel_smem_bytes(tp, tk, e->lig_slots, w, precision);
+      if (ts > kSmemLimit) ts = kernel_smem_bytes(tp, tk = 0, e->lig_slots, w, precision);
+      if (ts > kSmemLimit) continue;
+      const int to = kernel_occupancy(1, precision, t, ts);
+      const long long fl = std::min<long long>(n, (long long)to * w * nsm);
+      if (fl <= flight) continue;
+      flight = fl;
+      tc = t;
+      occ = to;
+      P = tp;
+      kst = tk;
+    }
+  if (occ < 1) return fail(GD_E_CAPACITY, "ligand slots too large for shared memory");
   // poses grouped by protein conformation so that a CTA stages one conformation
   std::vector<int> ord(n);
   std::iota(ord.begin(), ord.end(), 0);
@@ -1134,9 +1152,6 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
   a.out = d_out;
   a.out64 = d_out64;
   a.raw = d_raw;
-  int nsm = 0;
-  EV_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device));
-  const int occ = std::max(1, kernel_occupancy(1, precision, tc, smem));
   const int grid = std::max(1, std::min((int)items.size(), occ * nsm));
   EV_CUDA(launch_kernel(1, precision, tc, a, grid, e->st));
   std::vector<float> hout(10 * (size_t)n), hraw(raw ? 9 * (size_t)n : 0);
