@@ -28,7 +28,7 @@ struct Options {
   int dock_cache = 1;  // Dock keeps its device state per GPU between calls
   int dock_device_pack = 1;  // Dock refills that state on the GPU from the Complex CopyH2D put there
   int dock_record_direct = 1;  // Dock's kernels write Records straight into a GPU-mapped host array
-  int replica_warps = 1;     // warps per replica (1, 2, 4, 8): latency mode of the batched FP32 kernel
+  int replica_warps = 1;     // warps per replica: 1 the library's choice, else fixed at 2, 4 or 8
   int device_base = 0;        // the drop-in API's GPU g is CUDA device device_base + g
   long long wait_limit = 0;   // microseconds of a bounded shared-memory wait (0: one second)
   int stall_test = 0;         // test hook: staging barriers that never complete (bounded waits run out)
@@ -61,8 +61,6 @@ bool same_options(const Options &a, const Options &b)
          a.dock_device_pack == b.dock_device_pack && a.replica_warps == b.replica_warps &&
          a.device_base == b.device_base && a.wait_limit == b.wait_limit && a.stall_test == b.stall_test;
 }
-
-constexpr size_t kSmemLimit = 227 * 1024;
 
 }  // namespace
 
@@ -98,7 +96,7 @@ struct gd_ensemble {
   TileConfig tc{8, 1, 8};
   int grid = 0;
   size_t smem = 0;
-  int Pmax = 0, Kmax = 0, Kst = 0, lig_slots = 0;
+  int Pmax = 0, lig_slots = 0;
   int step = 0;
   // replica exchange over all jobs: pair-count prefix sums per parity
   int *d_xoff = nullptr;
@@ -159,30 +157,25 @@ int build_items(gd_ensemble *e)
   return GD_OK;
 }
 
-size_t smem_for(const gd_ensemble *e, int warps, int kst, int stage = 1, int group = 1)
+size_t smem_for(const gd_ensemble *e, const TileConfig &tc)
 {
-  return kernel_smem_bytes(stage ? e->Pmax : 0, kst, e->lig_slots, warps, e->precision, group);
+  return kernel_smem_bytes(tc.stage ? e->Pmax : 0, e->Pmax, e->lig_slots, e->precision, tc);
 }
 
-// Pick the KDE staging, the grid and (if not given) the replicas per CTA.
+// Check a tile shape, fix its staging, work items and grid.
 int configure(gd_ensemble *e, TileConfig tc)
 {
-  // the split (latency) form exists for the FP32 atom-pair loop of the batched kernel
-  if (e->precision == GD_PREC_FP64 || e->kernel == GD_KERNEL_PLAIN || tc.kpl % 2) tc.group = 1;
-  if (tc.group != 1 && tc.group != 2 && tc.group != 4 && tc.group != 8)
-    return fail(GD_E_INVALID, "warps per replica = %d (1, 2, 4 or 8)", tc.group);
+  if (e->kernel == GD_KERNEL_PLAIN) tc.group = 1;
+  if (tc.group != 1 && tc.group != 2 && tc.group != 4 && tc.group != 8 && tc.group != 16)
+    return fail(GD_E_INVALID, "warps per replica = %d (1, 2, 4, 8 or 16)", tc.group);
   if (tc.warps_per_cta < 1 || tc.warps_per_cta * 32 > kMaxCtaThreads || tc.warps_per_cta % tc.group)
     return fail(GD_E_INVALID, "warps per CTA = %d outside [1, %d] or not a multiple of the %d warps per replica",
                 tc.warps_per_cta, kMaxCtaThreads / 32, tc.group);
-  // a pocket too large to stage is read through L1; KDE points that do not fit are read from global memory
-  if (tc.stage && smem_for(e, tc.warps_per_cta, 0, 1, tc.group) > kSmemLimit) tc.stage = 0;
-  // FP32 reads the KDE points through L1 (the shared memory left to L1 pays more than
-  // staging them); FP64 stages them
-  e->Kst = e->precision == GD_PREC_FP64 ? e->Kmax : 0;
-  if (smem_for(e, tc.warps_per_cta, e->Kst, tc.stage, tc.group) > kSmemLimit) e->Kst = 0;
-  const size_t smem = smem_for(e, tc.warps_per_cta, e->Kst, tc.stage, tc.group);
+  // a pocket too large to stage is read through L1
+  if (tc.stage && smem_for(e, tc) > kSmemLimit) tc.stage = 0;
+  const size_t smem = smem_for(e, tc);
   if (smem > kSmemLimit)
-    return fail(GD_E_CAPACITY, "%d replicas per CTA need %zu B of shared memory (limit %zu)", tc.warps_per_cta, smem,
+    return fail(GD_E_CAPACITY, "%d warps per CTA need %zu B of shared memory (limit %zu)", tc.warps_per_cta, smem,
                 kSmemLimit);
   const int occ = kernel_occupancy(0, e->precision, tc, smem);
   if (occ < 1) return fail(GD_E_INVALID, "tile (warps %d, kpl %d, ab %d) cannot launch", tc.warps_per_cta, tc.kpl, tc.ab);
@@ -199,16 +192,44 @@ int configure(gd_ensemble *e, TileConfig tc)
   return GD_OK;
 }
 
-// Replicas per CTA from occupancy: fewest waves of work items, then most
-// resident warps per SM.
+// Work items of R replicas at most (build_items).
+long long count_items(const gd_ensemble *e, int R)
+{
+  long long items = 0;
+  for (const std::vector<int> &pr : e->rep_prt)
+    for (size_t r = 0, k; r < pr.size(); r += k) {
+      for (k = 1; r + k < pr.size() && (int)k < R && pr[r + k] == pr[r]; ++k) {}
+      ++items;
+    }
+  return items;
+}
+
+ShapeQuery shape_query(const gd_ensemble *e, int stage_opt, int nsm)
+{
+  ShapeQuery q;
+  q.precision = e->precision;
+  q.Pmax = e->Pmax;
+  q.lig_slots = e->lig_slots;
+  q.nsm = nsm;
+  q.stage_opt = stage_opt;
+  q.items = [e](int R) { return count_items(e, R); };
+  return q;
+}
+
+// Warps per replica and replicas per CTA from occupancy: a team each where one
+// wave holds them, else base.group warps each, fewest waves of work items, then
+// most resident warps per SM.
 // stage_opt: -1 chooses between staging the pocket and reading it through L1.
 int choose_warps(gd_ensemble *e, TileConfig base, int stage_opt = -1)
 {
   int nsm = 0;
   GD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device));
+  int grid = 0;
+  const ShapeQuery q = shape_query(e, stage_opt, nsm);
+  if (e->kernel == GD_KERNEL_BATCHED && choose_team(q, base, grid)) return configure(e, base);
+  if (base.group == 1 && choose_spread(q, base, grid)) return configure(e, base);
   double best = 1e300;
-  const int G = (e->precision == GD_PREC_FP64 || e->kernel == GD_KERNEL_PLAIN || base.kpl % 2) ? 1
-                                                                                         : std::max(1, base.group);
+  const int G = e->kernel == GD_KERNEL_PLAIN ? 1 : std::max(1, base.group);
   int best_w = std::max(8, G), best_stage = 1;
   for (int stage = 1; stage >= 0; --stage)
   for (int w = std::max(2, G); w <= kMaxCtaThreads / 32; w += (w < G ? 1 : G)) {
@@ -218,31 +239,23 @@ int choose_warps(gd_ensemble *e, TileConfig base, int stage_opt = -1)
     tc.warps_per_cta = w;
     tc.stage = stage;
     tc.group = G;
-    int kst = e->Kmax;
-    if (smem_for(e, w, kst, stage, G) > kSmemLimit) kst = 0;
-    const size_t smem = smem_for(e, w, kst, stage, G);
+    const size_t smem = smem_for(e, tc);
     if (smem > kSmemLimit) continue;
     const int occ = kernel_occupancy(0, e->precision, tc, smem);
     if (occ < 1) continue;
     // items and the slowest SM's load (items are equal-cost within a job)
-    long long items = 0;
-    for (size_t j = 0; j < e->jobs.size(); ++j) {
-      const std::vector<int> &pr = e->rep_prt[j];
-      int r = 0;
-      while (r < (int)pr.size()) {
-        int k = 1;
-        while (r + k < (int)pr.size() && k < w / G && pr[r + k] == pr[r]) ++k;
-        ++items;
-        r += k;
-      }
-    }
+    const long long items = count_items(e, w / G);
     const long long slots = (long long)occ * nsm;
     const long long waves = (items + slots - 1) / slots;
     // time ~ waves * (warps resident per SM); fewer resident warps per SM than 16 also hurts latency hiding
     const int resident = occ * w;
     double t = (double)waves * std::max(resident, 16) / (double)std::min(resident, 32);
     if (!stage) t *= 1.05;  // L1 reads of the pocket: prefer staging when occupancy is equal
-    if (t < best - 1e-9) {
+    // of equal shapes up to 8 warps the largest: each CTA has its own pair tables, which L1 loses
+    // (3520 replicas, 24 warps per SM as 6 CTAs of 4 warps: 3.10 ms for 10 steps, as 3 of 8: 2.96 ms);
+    // above, smaller items balance uneven ligands better (32 ligands x 400 replicas, 4 steps, 12 warps
+    // 5.60 ms, 8 warps 5.32 ms)
+    if (w <= 8 ? t < best + 1e-9 : t < best - 1e-9) {
       best = t;
       best_w = w;
       best_stage = stage;
@@ -268,13 +281,11 @@ int upload_jobs(gd_ensemble *e)
 int finish_create(gd_ensemble *e)
 {
   e->Pmax = 0;
-  e->Kmax = 0;
   int Lmax = 1;
   e->rep_prt.resize(e->jobs.size());
   for (size_t j = 0; j < e->jobs.size(); ++j) {
     const DevJob &J = e->jobs[j].dj;
     e->Pmax = std::max(e->Pmax, J.npoint_pad);
-    e->Kmax = std::max(e->Kmax, J.nkde);
     Lmax = std::max(Lmax, J.natom);
   }
   e->lig_slots = (Lmax + 3) & ~3;
@@ -305,8 +316,10 @@ int finish_create(gd_ensemble *e)
   e->wait_limit = (uint32_t)o.wait_limit;
   e->stall_bytes = o.stall_test ? 16u : 0u;
   TileConfig tc{o.warps > 0 ? o.warps : 8, o.kpl, o.ab, o.stage != 0 ? 1 : 0, o.replica_warps};
-  default_pair_tile(tc.group, tc.kpl, tc.ab);
+  default_pair_tile(tc.kpl, tc.ab);
   if (e->precision == GD_PREC_FP64) tc.kpl = 1, tc.ab = 8, tc.group = 1;
+  // replica_warps > 1 names the order the sums are combined in; FP64 and the plain kernel have one
+  if (e->kernel == GD_KERNEL_BATCHED) tc.split = tc.group;
   if (o.warps > 0) return configure(e, tc);
   return choose_warps(e, tc, o.stage);
 }
@@ -378,9 +391,8 @@ KArgs mc_args(gd_ensemble *e, int s_begin, int nsteps, int flags, const int *d_s
   a.flags = flags;
   a.d_step = d_step;
   a.P = e->tc.stage ? e->Pmax : 0;
-  a.Kst = e->Kst;
+  a.Pall = e->Pmax;
   a.lig_slots = e->lig_slots;
-  a.group = (uint16_t)e->tc.group;
   a.wait_limit = e->wait_limit;
   a.stall_bytes = (uint16_t)e->stall_bytes;
   return a;
@@ -1061,35 +1073,8 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
       return fail(GD_E_INVALID, "pose %d: conformation (%d, %d) out of range", i, conf[2 * i], conf[2 * i + 1]);
   const Options o = opts();
   TileConfig tc{8, o.kpl, o.ab};
-  default_pair_tile(1, tc.kpl, tc.ab);
+  default_pair_tile(tc.kpl, tc.ab);
   if (precision == GD_PREC_FP64) tc.kpl = 1, tc.ab = 8;
-  // The pocket staged in shared memory or read through L1, and the poses per CTA: what keeps
-  // the most poses in flight (ties: staged, 8 poses).  A 64-atom ligand against 3000 points
-  // staged is 136 KB a CTA, so one CTA of 8 warps per SM: 16384 poses 6.26 ms; through L1
-  // three CTAs fit, 24 warps: 3.96 ms (FP64, 2048 poses on 8 and 16 warps: 8.89 and 5.12 ms).
-  int nsm = 0;
-  GD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device));
-  int kst = 0, P = 0, occ = 0;
-  long long flight = 0;
-  for (const bool staged : {true, false})
-    for (int w : {8, 12, 16, 4, 2, 1}) {
-      TileConfig t = tc;
-      t.warps_per_cta = w;
-      const int tp = staged ? e->Pmax : 0;
-      int tk = precision == GD_PREC_FP64 ? J.nkde : 0;  // FP32: KDE points through L1
-      size_t ts = kernel_smem_bytes(tp, tk, e->lig_slots, w, precision);
-      if (ts > kSmemLimit) ts = kernel_smem_bytes(tp, tk = 0, e->lig_slots, w, precision);
-      if (ts > kSmemLimit) continue;
-      const int to = kernel_occupancy(1, precision, t, ts);
-      const long long fl = std::min<long long>(n, (long long)to * w * nsm);
-      if (fl <= flight) continue;
-      flight = fl;
-      tc = t;
-      occ = to;
-      P = tp;
-      kst = tk;
-    }
-  if (occ < 1) return fail(GD_E_CAPACITY, "ligand slots too large for shared memory");
   // poses grouped by protein conformation so that a CTA stages one conformation
   std::vector<int> ord(n);
   std::iota(ord.begin(), ord.end(), 0);
@@ -1101,10 +1086,49 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
     sconf[2 * i + 1] = conf[2 * ord[i] + 1];
     for (int k = 0; k < 6; ++k) smm[6 * i + k] = mm[6 * (size_t)ord[i] + k];
   }
+  // A team of warps per pose where one wave holds the poses, else one warp each, with the
+  // pocket staged in shared memory or read through L1 and the poses per CTA that keep the most
+  // poses in flight (ties: staged, 8 poses).  A 64-atom ligand against 3000 points staged is
+  // 136 KB a CTA, so one CTA of 8 warps per SM: 16384 poses 6.26 ms; through L1 three CTAs
+  // fit, 24 warps: 3.96 ms (FP64, 2048 poses on 8 and 16 warps: 8.89 and 5.12 ms).
+  ShapeQuery q;
+  GD_CUDA(cudaDeviceGetAttribute(&q.nsm, cudaDevAttrMultiProcessorCount, e->device));
+  q.mode = 1;
+  q.precision = precision;
+  q.Pmax = e->Pmax;
+  q.lig_slots = e->lig_slots;
+  q.items = [&](int R) {
+    long long m = 0;
+    for (int i = 0, k; i < n; i += k, ++m)
+      for (k = 1; i + k < n && k < R && sconf[2 * (i + k) + 1] == sconf[2 * i + 1]; ++k) {}
+    return m;
+  };
+  int grid = 0;
+  if (n > 16 * q.nsm || !choose_team(q, tc, grid)) {  // one wave holds at most 12 teams of two per SM
+    long long flight = 0;
+    int occ = 0;
+    for (const int staged : {1, 0})
+      for (int w : {8, 12, 16, 4, 2, 1}) {
+        TileConfig t = tc;
+        t.warps_per_cta = w;
+        t.stage = staged;
+        const size_t ts = q.smem(t);
+        if (ts > kSmemLimit) continue;
+        const int to = kernel_occupancy(1, precision, t, ts);
+        const long long fl = std::min<long long>(n, (long long)to * w * q.nsm);
+        if (fl <= flight) continue;
+        flight = fl;
+        tc = t;
+        occ = to;
+      }
+    if (occ < 1) return fail(GD_E_CAPACITY, "ligand slots too large for shared memory");
+    grid = occ * q.nsm;
+  }
+  const int R = tc.warps_per_cta / tc.group;  // poses per CTA
   std::vector<WorkItem> items;
   for (int i = 0; i < n;) {
     int k = 1;
-    while (i + k < n && k < tc.warps_per_cta && sconf[2 * (i + k) + 1] == sconf[2 * i + 1]) ++k;
+    while (i + k < n && k < R && sconf[2 * (i + k) + 1] == sconf[2 * i + 1]) ++k;
     items.push_back(WorkItem{job, sconf[2 * i + 1], i, k});
     i += k;
   }
@@ -1144,15 +1168,15 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
   a.n_items = (int)items.size();
   a.queue = e->d_queue;
   a.err = e->d_err;
-  a.P = P;
-  a.Kst = kst;
+  a.P = tc.stage ? e->Pmax : 0;
+  a.Pall = e->Pmax;
   a.lig_slots = e->lig_slots;
   a.conf = d_conf;
   a.mm = d_mm;
   a.out = d_out;
   a.out64 = d_out64;
   a.raw = d_raw;
-  const int grid = std::max(1, std::min((int)items.size(), occ * nsm));
+  grid = std::max(1, std::min((int)items.size(), grid));
   EV_CUDA(launch_kernel(1, precision, tc, a, grid, e->st));
   std::vector<float> hout(10 * (size_t)n), hraw(raw ? 9 * (size_t)n : 0);
   std::vector<double> hout64(out64 ? 10 * (size_t)n : 0);
@@ -1196,7 +1220,6 @@ int gd_eval_poses(const Complex *c, int n, const int *conf, const float *mm, int
     const DevJob &J = e->jobs[0].dj;
     e->precision = precision;
     e->Pmax = J.npoint_pad;
-    e->Kmax = J.nkde;
     e->lig_slots = (J.natom + 3) & ~3;
     rc = upload_jobs(e);
   }
@@ -1457,21 +1480,22 @@ int gd_ensemble_autotune(gd_ensemble_t *e, int steps, char *report, int report_l
   double best_t = 1e300;
   const int shapes[][2] = {{1, 8}, {2, 4}, {2, 8}, {4, 4}, {4, 8}};
   const int warps[] = {4, 6, 8, 10, 12, 14, 16};
-  const bool can_stage = smem_for(e, std::max(4, e->tc.group), 0, 1, e->tc.group) <= kSmemLimit;
+  const int group = e->tc.group;  // kept
+  const TileConfig smallest{std::max(4, group), e->tc.kpl, e->tc.ab, 1, group, e->tc.split};
+  const bool can_stage = smem_for(e, smallest) <= kSmemLimit;
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);
   for (int stage = can_stage ? 1 : 0; stage >= 0; --stage)
   for (const auto &sh : shapes) {
-    if (e->precision == GD_PREC_FP64 && !(sh[0] == 1 && sh[1] == 8)) continue;
-    // FP32: kpl 1 is the per-type-group scalar loop, which the atom-pair loop of
-    // the even kpl shapes outruns on every workload measured; not worth tuning time
-    if (e->precision != GD_PREC_FP64 && sh[0] == 1) continue;
+    // FP64 has the shape (1, 8), FP32 the others; a team's kernel has one shape whatever these say
+    if ((e->precision == GD_PREC_FP64) != (sh[0] == 1)) continue;
+    if (group > 1 && (sh[0] != e->tc.kpl || sh[1] != e->tc.ab)) continue;
     for (int w : warps) {
       if (rc != GD_OK) break;
       // the warps per replica are kept; the candidates are the multiples of it
-      if (w % e->tc.group) continue;
-      TileConfig tc{w, sh[0], sh[1], stage, e->tc.group};
+      if (w % group) continue;
+      TileConfig tc{w, sh[0], sh[1], stage, group, e->tc.split};
       if (configure(e, tc) != GD_OK || e->tc.stage != stage) continue;
       // a strided sample of the work items (heaviest-first order kept), about two
       // waves of the grid, so that a candidate runs the full chunk length

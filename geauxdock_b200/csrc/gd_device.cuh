@@ -87,7 +87,7 @@ __device__ __forceinline__ T warp_sum(T v)
 
 // Compensated butterfly: each level adds two partial sums with Knuth's
 // TwoSum and carries the rounding error; the result is (sum, compensation).
-__device__ __forceinline__ float warp_sum_comp(float s, float c)
+__device__ __forceinline__ void warp_sum_pair(float &s, float &c)
 {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -99,6 +99,10 @@ __device__ __forceinline__ float warp_sum_comp(float s, float c)
     s = t;
     c = c + co + err;
   }
+}
+__device__ __forceinline__ float warp_sum_comp(float s, float c)
+{
+  warp_sum_pair(s, c);
   return s + c;
 }
 

@@ -280,7 +280,7 @@ __global__ void dp_setup_kernel(const Complex *__restrict__ cx, PackDst D)
       const float4 p = D.kde[s_kbeg[t] + (q - s_go[g])];
       const float inv = 1.0f / (float)s_kcnt[t];
       D.kslot[2 * q] = make_int4(__float_as_int(p.x), __float_as_int(p.y), __float_as_int(p.z), __float_as_int(inv));
-      D.kslot[2 * q + 1] = make_int4(s_ga[g] | (s_ge[g] << 16), 0, 0, 0);
+      D.kslot[2 * q + 1] = make_int4(s_ga[g] | (s_ge[g] << 16), s_kcnt[t], 0, 0);
     }
     __syncthreads();
   }

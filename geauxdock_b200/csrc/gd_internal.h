@@ -136,8 +136,8 @@ struct DevJob {
   int kcnt[kLigTypes];
   // the same as a list of (KDE point, ligand type group) slots, one per KDE point of a type the
   // ligand has, in the grouped ligand's type order: slot s is the int4 pair kslot[2 s + {0, 1}] =
-  // (bits of x, y, z of the point and of 1/(points of its type)), (beg | end << 16, 0, 0, 0),
-  // [beg, end) the group's atoms; nkslot <= nkde (the atom-pair form's KDE pass)
+  // (bits of x, y, z of the point and of 1/(points of its type)), (beg | end << 16, points of
+  // the type, 0, 0), [beg, end) the group's atoms; nkslot <= nkde
   int nkslot;
   const int4 *kslot;
   // MCS
@@ -180,23 +180,23 @@ struct WorkItem {
 // Kernel configuration chosen by the autotuner.
 struct TileConfig {
   int warps_per_cta;   // replicas per CTA (one warp each)
-  int kpl;             // pocket points per lane per row (1, 2 or 4)
+  int kpl;             // pocket points per lane per row (2 or 4; FP64: 1, its only shape)
   int ab;              // ligand atoms per register block (4 or 8)
   int stage = 1;       // 1: stage the protein conformation in shared memory, 0: read it through L1
-  int group = 1;       // warps per replica (1, 2, 4 or 8; FP32 only): a replica's pair rows, KDE points and
-                       // hydrophobic sums split over them (latency mode)
+  int group = 1;       // warps per replica (1, 2, 4, 8 or 16): with more than one, the team form (gd_team.cuh)
+  int split = 1;       // order the sums are combined in: 1 the one-warp kernel's, 2, 4 or 8 the order of a replica
+                       // split over that many warps (option replica_warps; group > 1); whatever the group, a
+                       // replica's results depend on this alone
 };
 
-// Pair-tile shape where the caller leaves it to the library (option value 0):
-// 4 points per lane with one warp per replica, 2 in latency mode, whose warps
-// share a replica's rows (shorter rows deal out more evenly); 8-atom
-// hydrophobic blocks.  Measured on the batched FP32 kernel: 4 x 8 runs the
-// 3520-replica Dock call 1.8 % and a one-replica 600-point complex 10 %
-// faster than 2 x 8, and 4 points per lane make a replica on 4 or 8 warps
-// 14-25 % slower.
-inline void default_pair_tile(int group, int &kpl, int &ab)
+// Pair-tile shape where the caller leaves it to the library (option value 0).
+// Measured on the one-warp FP32 kernel: 4 x 8 runs the 3520-replica Dock call
+// 1.8 % and a one-replica 600-point complex 10 % faster than 2 x 8.  The team
+// form has one shape of its own.  One point per lane (kpl 1) runs as two.
+inline void default_pair_tile(int &kpl, int &ab)
 {
-  if (kpl == 0) kpl = group > 1 ? 2 : 4;
+  if (kpl == 0) kpl = 4;
+  if (kpl == 1) kpl = 2;
   if (ab == 0) ab = 8;
 }
 
@@ -224,13 +224,13 @@ struct KArgs {
   int *err;
   int s_begin, nsteps, flags;
   const int *d_step;       // if set, steps start at *d_step + s_begin (graph replay)
-  int P, Kst, lig_slots;   // smem layout (maxima over the launched jobs); P = 0: pocket read from global memory
+  int P, Pall, lig_slots;  // smem layout (maxima over the launched jobs): points staged (0: pocket read from
+                           // global memory), points of the largest conformation, ligand atoms
   uint32_t wait_limit;     // microseconds a bounded shared-memory wait lasts before it gives up (0: one second)
   uint16_t stall_bytes;    // test hook: bytes announced to the staging barrier that no copy delivers, so
                            // that its bounded wait runs out (0 in normal use)
-  uint16_t group;          // warps per replica (TileConfig::group); 0 reads as 1.  Two 16-bit fields in the
-                           // place of one 32-bit one: the size of this struct changes the kernels' register
-                           // allocation (measured), so it is kept
+  uint8_t group, split;    // TileConfig::group and split, set by launch_kernel.  Fields of one 32-bit word: the
+                           // size of this struct changes the kernels' register allocation (measured), so it is kept
   // pose evaluation
   const int *conf;
   const float *mm;
@@ -239,9 +239,10 @@ struct KArgs {
   float *raw;
 };
 
-// Shared-memory bytes of the batched kernel for pocket conformations of P
-// points, Kst KDE points staged, lig_slots ligand atoms and `warps` replicas per CTA.
-size_t kernel_smem_bytes(int P, int Kst, int lig_slots, int warps, int precision, int group = 1);
+// Shared-memory bytes of the batched kernel with P points staged (0: none),
+// conformations of at most Pall points, lig_slots ligand atoms and the warps per
+// CTA and per replica of the tile shape.
+size_t kernel_smem_bytes(int P, int Pall, int lig_slots, int precision, const TileConfig &tc);
 
 // Resident CTAs per SM of the batched kernel for this configuration (0 if it cannot launch).
 int kernel_occupancy(int mode, int precision, const TileConfig &tc, size_t smem);

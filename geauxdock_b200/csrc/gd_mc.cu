@@ -111,82 +111,78 @@ __device__ __forceinline__ long long check_at(long long i, long long n, int site
 enum CheckSite { kSiteLig = 1, kSiteApt, kSiteAph, kSiteAhd, kSitePos, kSitePsp, kSiteKde, kSiteMcs, kSiteLgrp,
                  kSiteTcc, kSiteLigConf, kSitePrtConf, kSiteRep, kSiteTmp, kSiteTab = 16 };
 
+}  // namespace gd
+
+#include "gd_energy.cuh"
+
+namespace gd {
+
 // ----------------------------------------------------------- smem layout --
 struct SmemLayout {
-  uint32_t params, lgrp, pos, aux, kde, apt, aph, ahd, warp0, warp_bytes, lig_bytes, parts, total;
+  uint32_t params, lgrp, pos, aux, apt, aph, ahd, warp0, warp_bytes, lig_bytes, total;
+  uint32_t team0, team_bytes, parts;  // teams of warps (gd_team.cuh)
 };
-
-// Per-warp partial sums of a replica split over several warps (latency mode):
-// the dense terms, then the hydrophobic sum of every atom.
-constexpr int kPartTerms = 8;    // vdw, ele, pmf, psp, hdb, kde, mcs, (1 unused)
-constexpr uint32_t kPartBytes = 4u * (kPartTerms + kMaxAtoms);
 
 __host__ __device__ inline uint32_t align16(uint32_t x) { return (x + 15u) & ~15u; }
 
-__host__ __device__ inline SmemLayout smem_layout(int P, int Kst, int lig_slots, int warps, bool fp64,
-                                                   int group = 1)
+constexpr int kDrawSteps = 16;  // Monte Carlo steps whose random numbers a warp of a team draws at once
+// 32-point chunks of each of the KDE and pocket-specific walks whose terms a team of 8 or more warps keeps in shared
+// memory; a smaller team gives each walk to one warp
+__host__ __device__ inline int team_chunks(int G) { return G >= 8 ? 24 : 0; }
+
+// Values per lane and row that pass 1 leaves in shared memory, times 32: four sums, or in the one-warp order of a
+// team of 8 or more warps the two components' seven (HalfRow).
+__host__ __device__ inline int team_row_reals(int G, int V, bool fp64) { return G >= 8 && V == 1 && !fp64 ? 448 : 128; }
+
+// Points of a pass 1 row, the unit a team deals out: the one-warp kernel's, or with the split order (V > 1) half.
+__host__ __device__ inline int team_row(int V) { return V > 1 ? kHalfPoints : kRowPoints; }
+
+// P: points staged (0: none); Pall: points of the largest conformation.
+__host__ __device__ inline SmemLayout smem_layout(int P, int Pall, int lig_slots, int warps, bool fp64, int group = 1,
+                                                   int split = 1)
 {
   SmemLayout s;
   uint32_t off = 0;
-  s.params = off;  // FP64: the whole DevParams; FP32: its scalar prefix
-  off = align16(off + (uint32_t)(fp64 ? sizeof(DevParams) : kParamScalarBytes));
+  s.params = off;  // the scalar prefix of DevParams
+  off = align16(off + (uint32_t)kParamScalarBytes);
   s.lgrp = off;
   off = align16(off + (uint32_t)sizeof(int2) * kMaxAtoms);
   s.pos = off;
   off = align16(off + 16u * (uint32_t)P);
   s.aux = off;
   off = align16(off + 8u * (uint32_t)P);
-  s.kde = off;
-  off = align16(off + 16u * (uint32_t)Kst);
-  // FP32: per (atom pair, point type) tables of the atom-pair pair loop
-  const uint32_t npairs = fp64 ? 0u : (uint32_t)(lig_slots + 1) / 2u;
+  // FP32: per (atom pair, point type) tables of the atom-pair pair loop; FP64: per (type group, point type)
+  const uint32_t npairs = (uint32_t)(lig_slots + 1) / 2u;
+  const uint32_t entries = (uint32_t)kTabCols * (fp64 ? (uint32_t)(lig_slots < kLigTypes ? lig_slots : kLigTypes) : npairs);
   s.apt = off;
-  off = align16(off + 32u * (uint32_t)kTabCols * npairs);
+  off = align16(off + (fp64 ? 16u : 32u) * entries);
   s.aph = off;
-  off = align16(off + 16u * (uint32_t)kTabCols * npairs);
+  off = align16(off + 16u * entries);
   s.ahd = off;
-  off = align16(off + 16u * npairs);
+  if (!fp64) off = align16(off + 16u * npairs);
   s.lig_bytes = (uint32_t)lig_slots * (fp64 ? 32u : 16u);  // V4<double> per atom, or LigPair per two atoms
-  // per warp: rotated ligand, ReplicaMC state, EnergyScratch (192 B), WarpStats (64 B), and with
-  // several warps per replica its partial sums
-  s.parts = s.lig_bytes + (uint32_t)sizeof(ReplicaMC) + 192u + 64u;
-  s.warp_bytes = align16(s.parts + (group > 1 ? kPartBytes : 0u));
+  // per replica: ReplicaMC state, EnergyScratch (192 B), WarpStats (64 B); per warp the rotated ligand
+  const uint32_t state = (uint32_t)sizeof(ReplicaMC) + 192u + 64u;
+  s.team0 = off;
+  s.team_bytes = 0;
+  s.parts = 0;
+  if (group > 1) {
+    // per team: the state, the rows' sums per lane, the contact sums per atom and share of the split order, the
+    // walks' terms (chunks) or sums per lane
+    const uint32_t real = fp64 ? 8u : 4u, V = (uint32_t)split;
+    const uint32_t walk = 64u * (V > 1 ? 0u : (uint32_t)team_chunks(group)) + 32u * V;
+    s.parts = (uint32_t)sizeof(ReplicaMC) + 64u + real * 72u;
+    s.team_bytes = align16(s.parts + real * ((uint32_t)team_row_reals(group, split, fp64) * (uint32_t)(Pall / team_row(split)) + V * (uint32_t)kMaxAtoms + 2u * walk));
+    off += s.team_bytes * (uint32_t)(warps / group);
+  }
+  s.warp_bytes = align16(s.lig_bytes + (group > 1 ? (uint32_t)kDrawSteps * 40u : state));
   s.warp0 = off;
   off += s.warp_bytes * (uint32_t)warps;
   s.total = off;
   return s;
 }
 
-// warps per replica a launch runs with: pose evaluation and FP64 use one
-template <int MODE, int PREC>
-__host__ __device__ inline int kernel_group(const KArgs &a)
-{
-  return (MODE == 1 || PREC == kFP64 || a.group < 1) ? 1 : a.group;
-}
-
-// Barrier of the G warps of one replica (named barrier 1 + index of the group).
-__device__ __forceinline__ void group_sync(int bar_id, int G)
-{
-  asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(G * 32) : "memory");
-}
-
-// A replica's place in a group of G warps (latency mode): warp `sub` of the
-// group takes pair rows sub, sub + G, ... and KDE points likewise; its partial
-// sums go to its own part area (gparts + sub * pstride floats) and warp 0 of
-// the group combines them in warp order, so that the result depends on G but
-// on nothing else.  G = 1 is the plain one-warp-per-replica evaluation.
-struct Split {
-  int sub, G, bar_id;
-  float *gparts;
-  uint32_t pstride;
-};
-struct NoSplit {};  // the one-warp-per-replica instantiation takes no split argument
-
-// ------------------------------------------------------------- energy --
-// Energy of ligand conformation ilig at pose mm in protein conformation iprt.
-// Called by all 32 lanes of a warp; on return every lane holds e[0..9]
-// (normalised terms and total) and raw[0..8] (terms before normalisation).
-// Per-warp results of energy_warp (written by lane 0 after the reductions).
+// Per-warp results of energy_warp, and the pose it is given.
 struct EnergyScratch {
   double e[10];    // normalised terms and total
   double raw[9];   // terms before the per-atom division and normalisation
@@ -195,6 +191,85 @@ struct EnergyScratch {
 };
 static_assert(sizeof(EnergyScratch) == 192, "EnergyScratch size is part of the smem layout");
 
+// ------------------------------------------------------------- energy --
+// Energy of ligand conformation ilig at pose out->mm in protein conformation
+// iprt, by one warp; writes e[0..9] (normalised terms and total) and raw[0..8].
+template <int PREC, int KPL, int AB>
+__device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__restrict__ par,
+                                         const float4 *__restrict__ pos, const float2 *__restrict__ aux,
+                                         const int2 *__restrict__ lgrp, const float4 *__restrict__ apt,
+                                         const float4 *__restrict__ aph, const int4 *__restrict__ ahd, void *ligbuf,
+                                         int ilig, int iprt, EnergyScratch *out)
+{
+  using T = RealOf<PREC>;
+  const int lane = lane_id();
+  const int L = J.natom, P = J.npoint_pad;
+  LigOf<PREC> *lig = reinterpret_cast<LigOf<PREC> *>(ligbuf);
+  rotate_ligand<PREC>(J, ilig, lane < 6 ? out->mm[lane] : 0.0f, lig);
+
+  // pass 1, row by row
+  RowSums<PREC> rs;
+  if constexpr (PREC == kFP64) {
+    for (int row = 0; row < P; row += kRowPoints) {
+      double h[4];
+      pass1_row64(lig, L, lgrp, par, reinterpret_cast<const double2 *>(apt), aph, row, P, pos, aux, h);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) rs.add(t, h[t]);
+    }
+  } else {
+    const PairConst kc = PairConst::load(par);
+    for (int row = 0; row < P; row += 32 * KPL) {
+      const float4 r = pass1_row<KPL, false>(lig, (L + 1) >> 1, row, P, pos, aux, apt, aph, ahd, kc);
+      rs.add(0, r.x);
+      rs.add(1, r.y);
+      rs.add(2, r.z);
+      rs.add(3, r.w);
+    }
+  }
+  const T s_psp = psp_walk<PREC>(J, iprt, lig, 0, 1);
+
+  // pass 2: one lane per atom applies the restraint
+  T ehpc = 0;
+  {
+    const int rows = contact_rows(J, iprt);
+    for (int a0 = 0; a0 < L; a0 += AB) {
+      const T S = contact_block<PREC, AB>(lig, L, a0, 0, kHalfPoints, rows, pos, aux, P);
+      const int a = a0 + lane / (32 / AB);
+      if (a < L && (lane & (32 / AB - 1)) == 0) ehpc = add_(ehpc, contact_restraint(par, lgrp, a, L, S));
+    }
+    ehpc = warp_sum(ehpc);
+  }
+
+  const T vdw = rs.total(0), ele = rs.total(1), pmf = rs.total(2), psp = warp_sum(s_psp), hdb = rs.total(3);
+  const T ekde = warp_sum(kde_walk<PREC>(J, par, lig, 0, 1));
+  const T elhm = mcs_sums<PREC>(J, lig, 1, nullptr);
+  const T dst = centre_dist2<T>(J, ilig, iprt, lane < 6 ? out->mm[lane] : 0.0f);
+
+  // lane i finishes term i; the weighted total in term order
+  T x = dst;
+  x = lane == 0 ? vdw : x;
+  x = lane == 1 ? ele : x;
+  x = lane == 2 ? pmf : x;
+  x = lane == 3 ? psp : x;
+  x = lane == 4 ? hdb : x;
+  x = lane == 5 ? ehpc : x;
+  x = lane == 6 ? ekde : x;
+  x = lane == 7 ? elhm : x;
+  const int term = lane < 9 ? lane : 8;
+  const T raw = raw_term<PREC>(term, scaled_sum<PREC>(term, x, par), J.nmcs);
+  const T v = norm_term(term, raw, par, L);
+  T tot = 0;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) tot = fma_((T)par->w[i], __shfl_sync(0xffffffffu, v, i), tot);
+  if (lane < 9) {
+    out->raw[lane] = (double)raw;
+    out->e[lane] = (double)v;
+  }
+  if (lane == 9) out->e[9] = (double)tot;
+  __syncwarp();
+}
+
+// ------------------------------------------------ per-type-group form --
 // Running sums of the pair terms of one point row.  The electrostatic term
 // q_a q_p g(d) is summed per point as q_p * sum_a q_a g(d), one sum per point
 // the lane holds, and multiplied by q_p at the end of the row.
@@ -205,11 +280,11 @@ struct PairAcc {
 };
 
 // Scalar force-field constants of the pair terms, read once per pose.
-struct PairConst {
+struct TypedConst {
   float lj0, lj1, lj01, el0, el1, inv_el1, a1, b1, ea, eb, ed2;
-  __device__ static PairConst load(const DevParams *p)
+  __device__ static TypedConst load(const DevParams *p)
   {
-    PairConst c;
+    TypedConst c;
     c.lj0 = p->lj0; c.lj1 = p->lj1; c.lj01 = p->lj01; c.el0 = p->el0; c.el1 = p->el1; c.inv_el1 = p->inv_el1;
     c.a1 = p->a1; c.b1 = p->b1; c.ea = p->ele_a; c.eb = p->ele_b; c.ed2 = p->ele_d2max;
     return c;
@@ -230,7 +305,7 @@ template <int PREC, int KPL, bool HDB, bool PSP, typename T, typename LA>
 __device__ __forceinline__ void pair_atoms(const LA *lig, int a, int aend, const T (&px)[KPL],
                                            const T (&py)[KPL], const T (&pz)[KPL], const float4 (&t4)[KPL],
                                            const float2 (&t2)[KPL], const float4 (&rf)[KPL], const T (&tps)[KPL],
-                                           const PairConst &c, PairAcc<T, KPL> &acc)
+                                           const TypedConst &c, PairAcc<T, KPL> &acc)
 {
   if constexpr (PREC == kFP64) {
     const double lj0 = c.lj0, lj1 = c.lj1, el0 = c.el0, el1 = c.el1, a1 = c.a1, b1 = c.b1;
@@ -288,112 +363,16 @@ __device__ __forceinline__ void pair_atoms(const LA *lig, int a, int aend, const
   }
 }
 
-// Running sums of one point row in the atom-pair form: component k of each
-// float2 belongs to atom 2i + k of the pair being visited; the electrostatic
-// sums are kept per point (they are multiplied by the point charge at the end
-// of the row).
-template <int KPL>
-struct PairAccP {
-  float2 vdw, pmf, hdb;
-  float2 ele[KPL];
-};
-
-// Per work item, shared-memory tables of the atom-pair pair loop, built from
-// the per-type tables (read from global memory): for pair i (atoms a = 2i,
-// b = 2i + 1) and point type pt, e = i * kTabCols + pt,
-//   apt[2e]     = (1/p1a, -p2a/p1a) of a and b interleaved: (a.x, b.x, a.y, b.y)
-//   apt[2e + 1] = (-pmf0, pmf1) interleaved
-//   aph[e]      = (hdb1 c, -hdb0 hdb1 c) interleaved
-//   ahd[i]      = (point types with hydrogen-bond parameters for a or b,
-//                  bit set of the types of a and b, type of a, type of b or 31).
-// The dummy half of an odd atom count gets the padding column and no types:
-// every term of it is exactly 0.
-__device__ void build_pair_tables(int L, const DevParams *par, const int2 *lg, float4 *apt, float4 *aph, int4 *ahd)
-{
-  const int npairs = (L + 1) >> 1;
-  for (int e = threadIdx.x; e < npairs * kTabCols; e += blockDim.x) {
-    const int i = e / kTabCols, pt = e % kTabCols;
-    const int a = 2 * i, b = a + 1;
-    const int lta = GD_AT(lg[GD_AT(a, L, kSiteLgrp)].x, kLigTypes, kSiteTab), ltb = b < L ? lg[b].x : -1;
-    const float4 ta = par->tab4[lta][pt];
-    const float4 tb = ltb >= 0 ? par->tab4[ltb][pt] : tab4_padding();
-    apt[2 * e] = make_float4(ta.x, tb.x, ta.y, tb.y);
-    apt[2 * e + 1] = make_float4(ta.z, tb.z, ta.w, tb.w);
-    const float2 ha = par->tab2[lta][pt], hb = ltb >= 0 ? par->tab2[ltb][pt] : make_float2(0.f, 0.f);
-    aph[e] = make_float4(ha.x, hb.x, ha.y, hb.y);
-    if (pt == 0) {
-      const uint32_t hm = par->hdbmask[lta] | (ltb >= 0 ? par->hdbmask[ltb] : 0u);
-      const uint32_t tb_bits = (1u << lta) | (ltb >= 0 ? 1u << ltb : 0u);
-      ahd[i] = make_int4((int)hm, (int)tb_bits, lta, ltb >= 0 ? ltb : 31);
-    }
-  }
-}
-
-// Pair terms of ligand atom pair i against the lane's KPL points
-// (energy_prt_v1.cu:56-139 except the hydrophobic contact), the FP32 forms of
-// pair_atoms with two atoms per packed f32x2 instruction (__ffma2_rn /
-// __fadd2_rn / __fmul2_rn, sm_100); the special functions stay per component.
-// HDB: evaluate the hydrogen-bond term (some point of the row has a parameter
-// for one of the two atoms); the pocket-specific term is walked over its
-// non-zero cells after the loop.  npx/npy/npz hold the lane's negated point
-// coordinates twice (x_atom - x_point is x_atom + (-x_point), exactly); the
-// charges are read from shared memory where they are used, which keeps the
-// loop within its registers.
-template <int KPL, bool HDB>
-__device__ __forceinline__ void pair_atom_pair(const LigPair *__restrict__ lig, int i GD_CHECK_ARG(int npairs), const float2 &lx,
-                                               const float2 &ly, const float2 &lz, const float4 *__restrict__ apt,
-                                               const float4 *__restrict__ aph, const int (&pt)[KPL],
-                                               const float2 (&npx)[KPL], const float2 (&npy)[KPL],
-                                               const float2 (&npz)[KPL], const PairConst &c, PairAccP<KPL> &acc)
-{
-  const float2 lj01 = f2(c.lj01), lj0 = f2(c.lj0), one = f2(1.0f), inv_el1 = f2(c.inv_el1);
-  const float2 za = f2(-0.5f * kLog2e), zb = f2(6.0f * kLog2e);
-#pragma unroll
-  for (int j = 0; j < KPL; ++j) {
-    const int e = i * kTabCols + pt[j];
-    const float4 ta = apt[2 * e], tb = apt[GD_AT(2 * e + 1, 2 * npairs * kTabCols, kSiteApt)];
-    const float2 dx = __fadd2_rn(lx, npx[j]), dy = __fadd2_rn(ly, npy[j]), dz = __fadd2_rn(lz, npz[j]);
-    const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-    const float2 r = make_float2(rsqrt_approx(d2.x), rsqrt_approx(d2.y));
-    const float2 d = __fmul2_rn(d2, r);
-    const float2 d3 = __fmul2_rn(d2, d);
-    const float2 d6 = __fmul2_rn(d3, d3);
-    const float2 den = __ffma2_rn(__fmul2_rn(d6, d3), make_float2(ta.x, ta.y), __ffma2_rn(lj01, d2, lj0));
-    const float2 num = __ffma2_rn(make_float2(ta.z, ta.w), d3, one);
-    acc.vdw = __ffma2_rn(num, make_float2(rcp_approx(den.x), rcp_approx(den.y)), acc.vdw);
-    float2 g = __fmul2_rn(r, inv_el1);
-    if (d2.x < c.ed2) g.x = fmaf(d2.x, fmaf(c.eb, d.x, c.ea), c.el0);
-    if (d2.y < c.ed2) g.y = fmaf(d2.y, fmaf(c.eb, d.y, c.ea), c.el0);
-    acc.ele[j] = __ffma2_rn(lig[GD_AT(i, npairs, kSiteLig)].q, g, acc.ele[j]);
-    const float2 dmp = __fadd2_rn(d, make_float2(tb.x, tb.y));
-    const float2 z = __fmul2_rn(__ffma2_rn(za, d, zb), dmp);
-    const float2 e1 = __fadd2_rn(make_float2(ex2_approx(z.x), ex2_approx(z.y)), one);
-    acc.pmf = __ffma2_rn(make_float2(tb.z, tb.w), make_float2(rcp_approx(e1.x), rcp_approx(e1.y)), acc.pmf);
-    if constexpr (HDB) {
-      const float4 th = aph[GD_AT(e, npairs * kTabCols, kSiteAph)];
-      const float2 h = __ffma2_rn(d, make_float2(th.x, th.y), make_float2(th.z, th.w));
-      const float2 hh = __fmul2_rn(h, h);
-      acc.hdb = __ffma2_rn(make_float2(th.x, th.y), make_float2(ex2_approx(-hh.x), ex2_approx(-hh.y)), acc.hdb);
-    }
-  }
-}
-
-template <int PREC, int KPL, int AB, bool SPLIT = false>
-__device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__restrict__ par,
+template <int PREC, int KPL, int AB>
+__device__ __noinline__ void energy_typed(const DevJob &J, const DevParams *__restrict__ par,
                                          const float4 *__restrict__ pos, const float2 *__restrict__ aux,
                                          const float4 *__restrict__ kde, const int2 *__restrict__ lgrp,
                                          const float4 *__restrict__ apt, const float4 *__restrict__ aph,
                                          const int4 *__restrict__ ahd, void *ligbuf, int ilig, int iprt,
-                                         const float *mm, EnergyScratch *out,
-                                         typename std::conditional<SPLIT, Split, NoSplit>::type sp = {})
+                                         const float *mm, EnergyScratch *out)
 {
   using T = typename std::conditional<PREC == kFP64, double, float>::type;
-  // SPLIT: the latency-mode instantiation (G warps per replica); otherwise G is 1 at compile time
-  int G = 1, my_sub = 0;
-  if constexpr (SPLIT && PREC != kFP64) {
-    G = sp.G;
-    my_sub = sp.sub;
-  }
+  constexpr int G = 1, my_sub = 0;
   const int row0 = 32 * KPL * my_sub, rstep = 32 * KPL * G;
   const int lane = lane_id();
   const int L = J.natom;
@@ -468,98 +447,9 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
   float c_vdw = 0.f, c_ele = 0.f, c_pmf = 0.f;
   const float *pspc = J.psp + (size_t)iprt * kLigTypes * P;
   const uint32_t *pmc = J.pspmask + (size_t)iprt * P;
-  const PairConst kc = PairConst::load(par);
+  const TypedConst kc = TypedConst::load(par);
 
-  if constexpr (PREC != kFP64 && KPL % 2 == 0) {
-    // atom-pair form: atoms 2i and 2i+1 share one register pair and the
-    // table entries come per atom pair, so there is no loop over type groups
-    // (the pocket-specific term is not in this loop: it walks the potential's
-    // non-zero cells after it)
-    const LigPair *lp = lig;
-    const int npairs = (L + 1) >> 1;
-    for (int row = row0; row < P; row += rstep) {
-      float2 npx[KPL], npy[KPL], npz[KPL];
-      int pt[KPL];
-      uint32_t ptbits = 0u;
-#pragma unroll
-      for (int j = 0; j < KPL; ++j) {
-        const int p = GD_AT(row + 32 * j + lane, P, kSitePos);
-        const float4 q = pos[p];
-        npx[j] = f2(-q.x);
-        npy[j] = f2(-q.y);
-        npz[j] = f2(-q.z);
-        pt[j] = __float_as_int(aux[p].y);
-        ptbits |= 1u << pt[j];
-      }
-      // point types present in the row: decide per atom pair, for the whole
-      // warp, whether the hydrogen-bond term is evaluated
-      ptbits = __reduce_or_sync(0xffffffffu, ptbits);
-      PairAccP<KPL> acc;
-      acc.vdw = acc.pmf = acc.hdb = f2(0.0f);
-#pragma unroll
-      for (int j = 0; j < KPL; ++j) acc.ele[j] = f2(0.0f);
-      for (int i = 0; i < npairs; ++i) {
-        const int2 fl = *reinterpret_cast<const int2 *>(&ahd[GD_AT(i, npairs, kSiteAhd)].x);
-        const bool any_hdb = ((uint32_t)fl.x & ptbits) != 0u;
-        const float4 l01 = *reinterpret_cast<const float4 *>(&lp[GD_AT(i, npairs, kSiteLig)].x);
-        const float2 lx = make_float2(l01.x, l01.y), ly = make_float2(l01.z, l01.w), lz = lp[i].z;
-        if (any_hdb)
-          pair_atom_pair<KPL, true>(lp, i GD_CHECK_ARG(npairs), lx, ly, lz, apt, aph, pt, npx, npy, npz, kc, acc);
-        else
-          pair_atom_pair<KPL, false>(lp, i GD_CHECK_ARG(npairs), lx, ly, lz, apt, aph, pt, npx, npy, npz, kc, acc);
-      }
-      float row_ele = 0.f;
-#pragma unroll
-      for (int j = 0; j < KPL; ++j) {
-        // the point charges are read again here rather than held through the atom loop
-        row_ele += pos[row + 32 * j + lane].w * (acc.ele[j].x + acc.ele[j].y);
-      }
-      const float row_vdw = acc.vdw.x + acc.vdw.y, row_pmf = acc.pmf.x + acc.pmf.y;
-      const float row_hdb = acc.hdb.x + acc.hdb.y;
-      if constexpr (PREC == kFP32Kahan) {
-        kahan_add(s_vdw, c_vdw, row_vdw);
-        kahan_add(s_ele, c_ele, row_ele);
-        kahan_add(s_pmf, c_pmf, row_pmf);
-        s_hdb += row_hdb;
-      } else {
-        s_vdw += row_vdw;
-        s_ele += row_ele;
-        s_pmf += row_pmf;
-        s_hdb += row_hdb;
-      }
-    }
-    // Pocket-specific term (energy_prt_v1.cu:109-115) over the conformation's
-    // non-zero cells (point p, ligand type t, value v; only types the ligand
-    // has), ordered by type: lane k takes cell k and counts the atoms of type t
-    // (the contiguous range [beg, end) of the type-grouped ligand) with
-    // d - pmf0 <= 0.  d, -pmf0 (the value the pair tables hold) and the
-    // comparison are the pair loop's operations in the same order, so an atom
-    // counts here exactly where that loop would count it.
-    {
-      const int4 *cell = J.pcell + (size_t)iprt * J.pcell_stride * 2;
-      const int ncell = J.pcell_cnt[iprt];
-      float acc_psp = 0.0f;
-      for (int k = 32 * my_sub + lane; k < ncell; k += 32 * G) {
-        // the point's coordinates and value, and the atom range with -pmf0 of
-        // (t, point type), the pair table's value: two independent 16-byte loads
-        const int4 c0 = __ldg(cell + 2 * GD_AT(k, J.pcell_stride, kSitePsp));
-        const int4 c1 = __ldg(cell + 2 * k + 1);
-        const int beg = c1.x & 0xffff, end = c1.x >> 16;
-        const float thr = __int_as_float(c1.y);
-        const float nx = -__int_as_float(c0.x), ny = -__int_as_float(c0.y), nz = -__int_as_float(c0.z);
-        int hits = 0;
-        for (int a = beg; a < end; ++a) {
-          const V4<float> la = atom_at(lp, GD_AT(a, L, kSiteLig));
-          const float dx = __fadd_rn(la.x, nx), dy = __fadd_rn(la.y, ny), dz = __fadd_rn(la.z, nz);
-          const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-          const float d = __fmul_rn(d2, rsqrt_approx(d2));
-          hits += __fadd_rn(d, thr) <= 0.0f ? 1 : 0;
-        }
-        acc_psp = fmaf((float)hits, __int_as_float(c0.w), acc_psp);
-      }
-      s_psp += acc_psp;
-    }
-  } else {
+  {
     for (int row = row0; row < P; row += rstep) {
       T px[KPL], py[KPL], pz[KPL], pe[KPL];
       int pt[KPL];
@@ -652,54 +542,7 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
     const int rows = ((J.ncdc[iprt] + 32 * KPL - 1) / (32 * KPL)) * (32 * KPL);
     for (int a0 = 0; a0 < L; a0 += AB) {
       T hpc[AB];
-      if constexpr (PREC != kFP64 && KPL % 2 == 0) {
-        // atom-pair form, the same operations per component: h2[k] holds the
-        // sums of atoms a0 + 2k and a0 + 2k + 1 (AB is even) of hpp (y^2 (y + y^2)),
-        // twice the contact sum (halved exactly at the end)
-        const float2 one = f2(1.0f), c1 = f2(-1.0f / 81.0f);
-        // rows of at most 64 points here: the last row of the hydrophobic-contact
-        // points then carries at most 63 others (hpp 0) where 128-point rows
-        // would carry up to 127
-        constexpr int K2 = KPL > 2 ? 2 : KPL;
-        const int rows2 = ((J.ncdc[iprt] + 32 * K2 - 1) / (32 * K2)) * (32 * K2);
-        float2 h2[AB / 2];
-#pragma unroll
-        for (int k = 0; k < AB / 2; ++k) h2[k] = f2(0.0f);
-        for (int row = 32 * K2 * my_sub; row < rows2; row += 32 * K2 * G) {
-          float2 npx[K2], npy[K2], npz[K2], ph2[K2];
-#pragma unroll
-          for (int j = 0; j < K2; ++j) {
-            const int p = GD_AT(row + 32 * j + lane, P, kSitePos);
-            const float4 q = pos[p];
-            npx[j] = f2(-q.x);
-            npy[j] = f2(-q.y);
-            npz[j] = f2(-q.z);
-            ph2[j] = f2(aux[p].x);
-          }
-#pragma unroll
-          for (int k = 0; k < AB / 2; ++k) {
-            const int a = a0 + 2 * k;
-            if (a >= L) break;
-            const LigPair la = lig[GD_AT(a >> 1, (L + 1) >> 1, kSiteLig)];
-#pragma unroll
-            for (int j = 0; j < K2; ++j) {
-              const float2 dx = __fadd2_rn(la.x, npx[j]), dy = __fadd2_rn(la.y, npy[j]), dz = __fadd2_rn(la.z, npz[j]);
-              const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-              float2 y = __ffma2_rn(d2, c1, one);
-              y.x = fmaxf(y.x, 0.0f);
-              y.y = fmaxf(y.y, 0.0f);
-              const float2 yy = __fmul2_rn(y, y);
-              const float2 w = __fmul2_rn(yy, __fadd2_rn(y, yy));
-              h2[k] = __ffma2_rn(ph2[j], w, h2[k]);
-            }
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < AB / 2; ++k) {
-          hpc[2 * k] = 0.5f * h2[k].x;
-          hpc[2 * k + 1] = 0.5f * h2[k].y;
-        }
-      } else {
+      {
 #pragma unroll
         for (int k = 0; k < AB; ++k) hpc[k] = 0;
         for (int row = row0; row < rows; row += rstep) {
@@ -733,46 +576,7 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
           }
         }
       }
-      if constexpr (PREC != kFP64 && KPL % 2 == 0) {
-        // the block's AB contact sums reduced across the warp together: each
-        // butterfly step halves the sums a lane carries (it keeps the half its
-        // lane bit selects and adds its partner's copy of it), then plain steps
-        // finish; lane l ends with atom a0 + base's sum, as do the lanes that
-        // differ from it below bit log2(32 / AB).  One lane per atom applies the
-        // restraint; its per-lane terms are summed once after the last block.
-        float v[AB];
-#pragma unroll
-        for (int k = 0; k < AB; ++k) v[k] = hpc[k];
-        int base = 0;
-#pragma unroll
-        for (int n = AB, off = 16; n > 1; n >>= 1, off >>= 1) {
-          const bool hi = (lane & off) != 0;
-#pragma unroll
-          for (int i = 0; i < n / 2; ++i) {
-            const float keep = hi ? v[n / 2 + i] : v[i], give = hi ? v[i] : v[n / 2 + i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
-          }
-          base += hi ? n / 2 : 0;
-        }
-#pragma unroll
-        for (int off = 16 / AB; off > 0; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
-        const int a = a0 + base;
-        if (a < L && (lane & (32 / AB - 1)) == 0) {
-          bool restraint = true;
-          if constexpr (SPLIT) {
-            if (G > 1) {
-              // this warp's share of atom a's contact sum; the restraint comes after the combination
-              sp.gparts[sp.sub * sp.pstride + kPartTerms + a] = v[0];
-              restraint = false;
-            }
-          }
-          if (restraint) {
-            const int lt = GD_AT(lgrp[GD_AT(a, L, kSiteLgrp)].x, kLigTypes, kSiteTab);
-            const float h2 = (v[0] - par->hpl0[lt]) / par->hpl1[lt];
-            ehpc += 0.5f * h2 * h2 - par->hpl2[lt];
-          }
-        }
-      } else {
+      {
 #pragma unroll
         for (int k = 0; k < AB; ++k) {
           const int a = a0 + k;
@@ -785,7 +589,6 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
       }
     }
     // the atom-pair form's restraint terms sit on one lane per atom
-    if constexpr (PREC != kFP64 && KPL % 2 == 0) ehpc = warp_sum(ehpc);
   }
 
   T vdw, ele, pmf, psp, hdb;
@@ -813,27 +616,7 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
   // replica split over G warps deals the slots or the type groups out to its
   // warps in turn.
   T kacc = 0;
-  if constexpr (PREC != kFP64 && KPL % 2 == 0) {
-    // the atom-pair form walks the job's KDE slots: lane k takes slot k (one
-    // KDE point of one of the ligand's type groups) and sums over the group's
-    // atoms, weighted by 1/(points of the type): every lane busy, one
-    // coalesced pair of loads per slot, no division
-    const float k2 = par->kde2 * kLog2e;
-    for (int q = 32 * my_sub + lane; q < J.nkslot; q += 32 * G) {
-      const int4 c0 = __ldg(J.kslot + 2 * GD_AT(q, J.nkde, kSiteKde));
-      const int4 c1 = __ldg(J.kslot + 2 * q + 1);
-      const float qx = __int_as_float(c0.x), qy = __int_as_float(c0.y), qz = __int_as_float(c0.z);
-      float sk = 0.0f;
-      const int end = c1.x >> 16;
-      for (int b = c1.x & 0xffff; b < end; ++b) {
-        const V4<float> la = atom_at(lig, GD_AT(b, L, kSiteLig));
-        const float dx = la.x - qx, dy = la.y - qy, dz = la.z - qz;
-        const float d2 = dx * dx + dy * dy + dz * dz;
-        sk += ex2_approx(k2 * d2);
-      }
-      kacc += sk * __int_as_float(c0.w);
-    }
-  } else {
+  {
     const T kde2 = par->kde2;
     int tg = 0;
     for (int a = 0; a < L; ++tg) {
@@ -910,55 +693,6 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
   }
   T elhm = warp_sum(macc);
 
-  if constexpr (SPLIT && PREC != kFP64) {
-    if (G > 1) {
-      // one replica over G warps: publish this warp's partial sums, and let warp
-      // 0 of the group combine them in warp order (compensated for the dense
-      // terms with the FP32-Kahan policy) and finish the evaluation
-      float *part = sp.gparts + sp.sub * sp.pstride;
-      if (lane == 0) {
-        part[0] = vdw;
-        part[1] = ele;
-        part[2] = pmf;
-        part[3] = psp;
-        part[4] = hdb;
-        part[5] = ekde;
-        part[6] = elhm;
-      }
-      group_sync(sp.bar_id, G);
-      if (sp.sub != 0) return;
-      float cv = 0.f, ce = 0.f, cp = 0.f;
-      for (int g = 1; g < G; ++g) {
-        const float *o = sp.gparts + g * sp.pstride;
-        if constexpr (PREC == kFP32Kahan) {
-          kahan_add(vdw, cv, o[0]);
-          kahan_add(ele, ce, o[1]);
-          kahan_add(pmf, cp, o[2]);
-        } else {
-          vdw += o[0];
-          ele += o[1];
-          pmf += o[2];
-        }
-        psp += o[3];
-        hdb += o[4];
-        ekde += o[5];
-        elhm += o[6];
-      }
-      vdw += cv;
-      ele += ce;
-      pmf += cp;
-      // the hydrophobic restraint on each atom's combined contact sum (energy_prt_v1.cu:162-169)
-      float eh = 0.f;
-      for (int a = lane; a < L; a += 32) {
-        float S = sp.gparts[kPartTerms + a];
-        for (int g = 1; g < G; ++g) S += sp.gparts[g * sp.pstride + kPartTerms + a];
-        const int lt = GD_AT(lgrp[GD_AT(a, L, kSiteLgrp)].x, kLigTypes, kSiteTab);
-        const float h2 = (S - par->hpl0[lt]) / par->hpl1[lt];
-        eh += 0.5f * h2 * h2 - par->hpl2[lt];
-      }
-      ehpc = warp_sum(eh);
-    }
-  }
 
   // ---- distance to the pocket centre, kernel_cuda_l1_montecarlo.cu:439-454
   const float *pc = J.pcenter + 3 * GD_AT(iprt, J.nprt, kSitePrtConf);
@@ -999,29 +733,23 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
 
 // ------------------------------------------------------------ kernels --
 
-
 // Stage the shared data of work item `wi` into shared memory.  Returns false,
 // in every thread of the CTA alike, if the bulk copies did not complete within
 // the wait limit; the barrier phase is then left open (see stage_abandon).
-template <bool FP64>
 __device__ bool stage_item(const KArgs &A, const DevJob &J, const WorkItem &wi, unsigned char *smem,
                            const SmemLayout &sl, uint64_t *bar, uint32_t &phase)
 {
   const int P = J.npoint_pad;
-  const bool kde_in_smem = J.nkde <= A.Kst;
   const bool pocket_in_smem = A.P > 0;
   if (threadIdx.x == 0) {
     fence_proxy_async_smem();
-    const uint32_t pbytes = (uint32_t)(FP64 ? sizeof(DevParams) : kParamScalarBytes);
-    uint32_t bytes = pbytes + (pocket_in_smem ? 24u * (uint32_t)P : 0u);
-    if (kde_in_smem) bytes += 16u * (uint32_t)J.nkde;
-    mbar_expect_tx(bar, bytes + A.stall_bytes);
+    const uint32_t pbytes = (uint32_t)kParamScalarBytes;
+    mbar_expect_tx(bar, pbytes + (pocket_in_smem ? 24u * (uint32_t)P : 0u) + A.stall_bytes);
     bulk_g2s(smem + sl.params, J.par, pbytes, bar);
     if (pocket_in_smem) {
       bulk_g2s(smem + sl.pos, J.pos + (size_t)wi.prt * P, 16u * (uint32_t)P, bar);
       bulk_g2s(smem + sl.aux, J.aux + (size_t)wi.prt * P, 8u * (uint32_t)P, bar);
     }
-    if (kde_in_smem && J.nkde > 0) bulk_g2s(smem + sl.kde, J.kde, 16u * (uint32_t)J.nkde, bar);
   }
   int2 *lg = reinterpret_cast<int2 *>(smem + sl.lgrp);
   for (int a = threadIdx.x; a < J.natom; a += blockDim.x) lg[a] = J.lgrp[a];
@@ -1044,7 +772,36 @@ __device__ void stage_abandon(const KArgs &A, uint64_t *bar, uint32_t phase)
   (void)__syncthreads_and(mbar_wait(bar, phase ^ 1u, wait_limit_ns(A.wait_limit)) ? 1 : 0);
 }
 
-// Per-warp FP64 statistics kept in shared memory during a chunk (lane 0).
+// The shared data of work item `wi`: staged, and its pair tables built, where the
+// CTA's previous item had another job or protein conformation.  Returns false
+// in every thread alike after a wait gave up (the kernel then returns).
+template <int PREC>
+__device__ bool load_item(const KArgs &A, const DevJob &J, const WorkItem &wi, unsigned char *smem,
+                          const SmemLayout &sl, uint64_t *bar, uint32_t &phase, int &prev_job, int &prev_prt)
+{
+  if (wi.job != prev_job || wi.prt != prev_prt) {
+    if (!stage_item(A, J, wi, smem, sl, bar, phase)) {
+      if (threadIdx.x == 0) atomicOr(A.err, kErrTimeout);
+      stage_abandon(A, bar, phase);
+      return false;
+    }
+    __syncthreads();  // type groups are in shared memory
+    if (wi.job != prev_job) {
+      const int2 *lg = reinterpret_cast<const int2 *>(smem + sl.lgrp);
+      if constexpr (PREC == kFP64)
+        build_pair_tables64(J, lg, reinterpret_cast<double2 *>(smem + sl.apt), reinterpret_cast<float4 *>(smem + sl.aph));
+      else
+        build_pair_tables(J.natom, J.par, lg, reinterpret_cast<float4 *>(smem + sl.apt),
+                          reinterpret_cast<float4 *>(smem + sl.aph), reinterpret_cast<int4 *>(smem + sl.ahd));
+    }
+    prev_job = wi.job;
+    prev_prt = wi.prt;
+  }
+  __syncthreads();
+  return true;
+}
+
+// Per-replica FP64 statistics kept in shared memory during a chunk (one lane).
 struct WarpStats {
   double e_sum, e_sum2, best_e;
   long long n_acc;
@@ -1053,18 +810,49 @@ struct WarpStats {
   int pad_;
 };
 
-template <int MODE, int PREC, int KPL, int AB, bool SPLIT = false>
+__device__ __forceinline__ void load_stats(WarpStats *w, const RepStats &S)
+{
+  w->e_sum = 0.0;
+  w->e_sum2 = 0.0;
+  w->n_acc = 0;
+  w->best_e = S.best_e;
+  w->best_step = S.best_step;
+  for (int i = 0; i < 6; ++i) w->best_mm[i] = S.best_mm[i];
+}
+
+// Step s ended with total energy ecur at pose mm.
+__device__ __forceinline__ void step_stats(WarpStats *w, int accept, double ecur, int s, const float *mm)
+{
+  w->n_acc += accept;
+  w->e_sum += ecur;
+  w->e_sum2 = fma_(ecur, ecur, w->e_sum2);
+  if (w->best_step < 0 || ecur < w->best_e) {
+    w->best_e = ecur;
+    w->best_step = s;
+    for (int i = 0; i < 6; ++i) w->best_mm[i] = mm[i];
+  }
+}
+
+__device__ __forceinline__ void store_stats(RepStats &S, const WarpStats *w, int nsteps)
+{
+  S.e_sum += w->e_sum;
+  S.e_sum2 += w->e_sum2;
+  S.n_steps += nsteps;
+  S.n_accept += w->n_acc;
+  S.best_e = w->best_e;
+  S.best_step = w->best_step;
+  for (int i = 0; i < 6; ++i) S.best_mm[i] = w->best_mm[i];
+}
+
+template <int MODE, int PREC, int KPL, int AB>
 __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
 {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ int s_item;
-  // G warps per replica (latency mode, the SPLIT instantiation): warp `sub` of replica slot `gi`
-  const int G = SPLIT ? kernel_group<MODE, PREC>(A) : 1;
-  const SmemLayout sl = smem_layout(A.P, A.Kst, A.lig_slots, blockDim.x / 32, PREC == kFP64, G);
+  const SmemLayout sl = smem_layout(A.P, A.Pall, A.lig_slots, blockDim.x / 32, PREC == kFP64);
   const int warp = threadIdx.x >> 5;
   const int lane = lane_id();
-  const int gi = warp / G, sub = warp - gi * G;
   // a Complex the device packer refused (gd_devpack.cu) leaves its job unread
   if (*(volatile int *)A.err & kErrPack) return;
   if (threadIdx.x == 0) mbar_init(&bar, 1);
@@ -1079,56 +867,32 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
     if (it >= A.n_items) break;
     const WorkItem wi = A.items[it];
     const DevJob &J = A.jobs[wi.job];
-    if (wi.job != prev_job || wi.prt != prev_prt) {
-      if (!stage_item<PREC == kFP64>(A, J, wi, smem, sl, &bar, phase)) {
-        if (threadIdx.x == 0) atomicOr(A.err, kErrTimeout);
-        stage_abandon(A, &bar, phase);
-        return;
-      }
-      if constexpr (PREC != kFP64 && KPL % 2 == 0) {
-        __syncthreads();  // type groups are in shared memory
-        if (wi.job != prev_job)
-          build_pair_tables(J.natom, J.par,
-                            reinterpret_cast<const int2 *>(smem + sl.lgrp), reinterpret_cast<float4 *>(smem + sl.apt),
-                            reinterpret_cast<float4 *>(smem + sl.aph), reinterpret_cast<int4 *>(smem + sl.ahd));
-      }
-      prev_job = wi.job;
-      prev_prt = wi.prt;
-    }
-    __syncthreads();
+    if (!load_item<PREC>(A, J, wi, smem, sl, &bar, phase, prev_job, prev_prt)) return;
     const float4 *apt = reinterpret_cast<const float4 *>(smem + sl.apt);
     const float4 *aph = reinterpret_cast<const float4 *>(smem + sl.aph);
     const int4 *ahd = reinterpret_cast<const int4 *>(smem + sl.ahd);
 
-    // FP32: only the scalar prefix of DevParams is in shared memory (no table is read through par)
-    const DevParams *par = reinterpret_cast<const DevParams *>(smem + sl.params);
+    const DevParams *par = reinterpret_cast<const DevParams *>(smem + sl.params);  // its scalar prefix
     // the protein conformation: staged in shared memory, or read through L1
     const float4 *pos = A.P > 0 ? reinterpret_cast<const float4 *>(smem + sl.pos)
                                 : J.pos + (size_t)wi.prt * J.npoint_pad;
     const float2 *aux = A.P > 0 ? reinterpret_cast<const float2 *>(smem + sl.aux)
                                 : J.aux + (size_t)wi.prt * J.npoint_pad;
-    const float4 *kde = (J.nkde <= A.Kst) ? reinterpret_cast<const float4 *>(smem + sl.kde) : J.kde;
     const int2 *lgrp = reinterpret_cast<const int2 *>(smem + sl.lgrp);
-    // each warp rotates the ligand into its own buffer; the replica's state, its
-    // proposal and the evaluation's result live in the group's first warp
     unsigned char *wbase = smem + sl.warp0 + (size_t)warp * sl.warp_bytes;
-    unsigned char *gbase = smem + sl.warp0 + (size_t)(gi * G) * sl.warp_bytes;
     void *ligbuf = wbase;
-    ReplicaMC *srep = reinterpret_cast<ReplicaMC *>(gbase + sl.lig_bytes);
-    EnergyScratch *esc = reinterpret_cast<EnergyScratch *>(gbase + sl.lig_bytes + sizeof(ReplicaMC));
-    WarpStats *wst = reinterpret_cast<WarpStats *>(gbase + sl.lig_bytes + sizeof(ReplicaMC) + sizeof(EnergyScratch));
-    typename std::conditional<SPLIT, Split, NoSplit>::type sp{};
-    if constexpr (SPLIT) sp = Split{sub, G, 1 + gi, reinterpret_cast<float *>(gbase + sl.parts), sl.warp_bytes / 4u};
-    const bool lead = sub == 0;  // the group's first warp: proposal, Metropolis, state
+    ReplicaMC *srep = reinterpret_cast<ReplicaMC *>(wbase + sl.lig_bytes);
+    EnergyScratch *esc = reinterpret_cast<EnergyScratch *>(wbase + sl.lig_bytes + sizeof(ReplicaMC));
+    WarpStats *wst = reinterpret_cast<WarpStats *>(wbase + sl.lig_bytes + sizeof(ReplicaMC) + sizeof(EnergyScratch));
 
-    if (gi < wi.count) {
-      const int r = wi.rep0 + gi;  // job-local index
+    if (warp < wi.count) {
+      const int r = wi.rep0 + warp;  // job-local index
       if constexpr (MODE == 1) {
         // ---- pose evaluation
         const int ilig = A.conf[2 * r], iprt = A.conf[2 * r + 1];
         if (lane < 6) esc->mm[lane] = A.mm[6 * r + lane];
         __syncwarp();
-        energy_warp<PREC, KPL, AB>(J, par, pos, aux, kde, lgrp, apt, aph, ahd, ligbuf, ilig, iprt, esc->mm, esc);
+        energy_warp<PREC, KPL, AB>(J, par, pos, aux, lgrp, apt, aph, ahd, ligbuf, ilig, iprt, esc);
         if (lane < 10) {
           A.out[10 * (size_t)r + lane] = (float)esc->e[lane];
           if (A.out64) A.out64[10 * (size_t)r + lane] = esc->e[lane];
@@ -1139,25 +903,16 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
         // ---- Monte Carlo chunk for replica r
         const int gr = J.rid_base + r;
         int *sw = reinterpret_cast<int *>(srep);
-        if (lead) sw[lane] = reinterpret_cast<const int *>(J.rep + GD_AT(r, J.nrep, kSiteRep))[lane];
-        if (lead && lane == 0) {
-          const RepStats &S = J.stats[r];
-          wst->e_sum = 0.0;
-          wst->e_sum2 = 0.0;
-          wst->n_acc = 0;
-          wst->best_e = S.best_e;
-          wst->best_step = S.best_step;
-          for (int i = 0; i < 6; ++i) wst->best_mm[i] = S.best_mm[i];
-        }
+        sw[lane] = reinterpret_cast<const int *>(J.rep + GD_AT(r, J.nrep, kSiteRep))[lane];
+        if (lane == 0) load_stats(wst, J.stats[r]);
         __syncwarp();
-        if (G > 1) group_sync(1 + gi, G);  // the replica's state is in shared memory
         int acc = J.run_acc[r];
         const int ilig = srep->idx_lig, iprt = srep->idx_prt;
         const double mbeta = (double)J.minus_beta[GD_AT(srep->idx_tmp, J.ntmp, kSiteTmp)];
         Record *rec = (J.rec && (A.flags & kMcRecord)) ? J.rec + r : nullptr;
         int ne = 0;
         if (J.rec && (A.flags & kMcResetRecord)) {
-          if (lead && lane == 0) J.rec[r].next_entry = 0;
+          if (lane == 0) J.rec[r].next_entry = 0;
         } else if (rec) {
           ne = rec->next_entry;
         }
@@ -1166,7 +921,7 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
         const int s0 = (A.d_step ? *A.d_step + A.s_begin : A.s_begin) + J.step0;
         const int nsteps = J.nsteps > 0 ? min(J.nsteps, A.nsteps) : A.nsteps;
         for (int s = s0; s < s0 + nsteps; ++s) {
-          if (acc && lead) {
+          if (acc) {
             // record the old state, kernel_cuda_l1_montecarlo.cu:290-297
             if (lane == 0) srep->step = s;
             __syncwarp();
@@ -1176,9 +931,7 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
           // draws of step s: counter {s, replica, 0, 0} -> move x y z, rot x;
           // {s, replica, 0, 1} -> rot y z, accept (lane 0 and lane 1 compute one each)
           float u_acc = 0.0f;
-          if (!lead) {
-            // the proposal is the group's first warp's
-          } else if (!initial) {
+          if (!initial) {
             const Philox4 d = philox4x32_10((uint32_t)s, (uint32_t)gr, 0u, (uint32_t)(lane & 1), J.key0, J.key1);
             float u[7];
 #pragma unroll
@@ -1196,10 +949,7 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
             esc->mm[lane] = __fmaf_rn(par->move_scale[lane], 0.0f, srep->movematrix[lane]);
           }
           __syncwarp();
-          if (G > 1) group_sync(1 + gi, G);  // the proposal is in shared memory
-          energy_warp<PREC, KPL, AB, SPLIT>(J, par, pos, aux, kde, lgrp, apt, aph, ahd, ligbuf, ilig, iprt, esc->mm, esc,
-                                            sp);
-          if (!lead) continue;  // the group's first warp holds the result
+          energy_warp<PREC, KPL, AB>(J, par, pos, aux, lgrp, apt, aph, ahd, ligbuf, ilig, iprt, esc);
           const float etot = (float)esc->e[9];
 
           // Metropolis test in FP64, kernel_cuda_l1_montecarlo.cu:485-507
@@ -1214,42 +964,29 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
             if (lane < 6) srep->movematrix[lane] = esc->mm[lane];
           }
           __syncwarp();
-          if (lane == 0) {
-            const double ecur = (double)srep->energy[9];
-            wst->n_acc += accept;
-            wst->e_sum += ecur;
-            wst->e_sum2 += ecur * ecur;
-            if (wst->best_step < 0 || ecur < wst->best_e) {
-              wst->best_e = ecur;
-              wst->best_step = s;
-              for (int i = 0; i < 6; ++i) wst->best_mm[i] = srep->movematrix[i];
-            }
-          }
+          if (lane == 0) step_stats(wst, accept, (double)srep->energy[9], s, srep->movematrix);
           acc = accept;
         }
 
-        if (lead) {
-          if (lane == 0) {
-            J.run_acc[r] = acc;
-            if (A.flags & kMcStoreAccept) srep->is_accept = acc;
-            if (rec) rec->next_entry = ne;
-            RepStats &S = J.stats[r];
-            S.e_sum += wst->e_sum;
-            S.e_sum2 += wst->e_sum2;
-            S.n_steps += nsteps;
-            S.n_accept += wst->n_acc;
-            S.best_e = wst->best_e;
-            S.best_step = wst->best_step;
-            for (int i = 0; i < 6; ++i) S.best_mm[i] = wst->best_mm[i];
-          }
-          __syncwarp();
-          reinterpret_cast<int *>(J.rep + r)[lane] = sw[lane];
+        if (lane == 0) {
+          J.run_acc[r] = acc;
+          if (A.flags & kMcStoreAccept) srep->is_accept = acc;
+          if (rec) rec->next_entry = ne;
+          store_stats(J.stats[r], wst, nsteps);
         }
+        __syncwarp();
+        reinterpret_cast<int *>(J.rep + r)[lane] = sw[lane];
       }
     }
     __syncthreads();
   }
 }
+
+}  // namespace gd
+
+#include "gd_team.cuh"
+
+namespace gd {
 
 // Replica exchange between adjacent temperatures.  Sweep x pairs (t, t+1) for
 // t = x mod 2, x mod 2 + 2, ... in every (protein conf p, ligand conf l)
@@ -1357,7 +1094,7 @@ __global__ void __launch_bounds__(256) eval_global_kernel(const DevJob *jobp, co
     __syncwarp();
     const size_t P = (size_t)J.npoint_pad;
     // KPL = 1: the per-type-group form, which needs no per-work-item tables
-    energy_warp<PREC, KPL, AB>(J, J.par, J.pos + iprt * P, J.aux + iprt * P, J.kde, J.lgrp, nullptr, nullptr, nullptr,
+    energy_typed<PREC, KPL, AB>(J, J.par, J.pos + iprt * P, J.aux + iprt * P, J.kde, J.lgrp, nullptr, nullptr, nullptr,
                                wb, ilig, iprt, esc->mm, esc);
     if (lane < 10) out[10 * (size_t)i + lane] = (float)esc->e[lane];
     if (raw && lane < 9) raw[9 * (size_t)i + lane] = (float)esc->raw[lane];
@@ -1383,65 +1120,61 @@ cudaError_t launch_eval_global(int precision, const DevJob *d_job, const int *co
 }
 
 // ---------------------------------------------------------- launchers --
-size_t kernel_smem_bytes(int P, int Kst, int lig_slots, int warps, int precision, int group)
+size_t kernel_smem_bytes(int P, int Pall, int lig_slots, int precision, const TileConfig &tc)
 {
-  return smem_layout(P, Kst, lig_slots, warps, precision == kFP64, group).total;
+  return smem_layout(P, Pall, lig_slots, tc.warps_per_cta, precision == kFP64, tc.group, tc.split).total;
 }
 
-template <int MODE, int PREC, int KPL, int AB>
-static cudaError_t launch_t(const KArgs &a, int warps, int grid, cudaStream_t st)
-{
-  const int group = kernel_group<MODE, PREC>(a);
-  const size_t smem = kernel_smem_bytes(a.P, a.Kst, a.lig_slots, warps, PREC, group);
-  auto k = mc_kernel<MODE, PREC, KPL, AB, false>;
-  if constexpr (MODE == 0 && PREC != kFP64 && KPL % 2 == 0)
-    if (group > 1) k = mc_kernel<MODE, PREC, KPL, AB, true>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k<<<grid, warps * 32, smem, st>>>(a);
-  return cudaGetLastError();
-}
+using McKernel = void (*)(KArgs);
 
+// The kernel of a launch: the team form with several warps per replica, else
+// the one-warp form of the tile shape.  FP64 has one shape, (1, 8).
 template <int MODE, int PREC>
-static cudaError_t launch_p(const KArgs &a, const TileConfig &tc, int grid, cudaStream_t st)
+static McKernel pick_kernel(const TileConfig &tc)
 {
-  const int w = tc.warps_per_cta;
-  if (tc.kpl == 1 && tc.ab == 8) return launch_t<MODE, PREC, 1, 8>(a, w, grid, st);
-  if (tc.kpl == 2 && tc.ab == 4) return launch_t<MODE, PREC, 2, 4>(a, w, grid, st);
-  if (tc.kpl == 2 && tc.ab == 8) return launch_t<MODE, PREC, 2, 8>(a, w, grid, st);
-  if (tc.kpl == 4 && tc.ab == 4) return launch_t<MODE, PREC, 4, 4>(a, w, grid, st);
-  if (tc.kpl == 4 && tc.ab == 8) return launch_t<MODE, PREC, 4, 8>(a, w, grid, st);
-  return cudaErrorInvalidValue;
+  if (tc.group >= 8 && PREC != kFP64) return team_kernel<MODE, PREC, PREC != kFP64>;
+  if (tc.group > 1) return team_kernel<MODE, PREC, false>;
+  if constexpr (PREC == kFP64) return tc.kpl == 1 && tc.ab == 8 ? mc_kernel<MODE, PREC, 1, 8> : nullptr;
+  else {
+    if (tc.kpl == 2 && tc.ab == 4) return mc_kernel<MODE, PREC, 2, 4>;
+    if (tc.kpl == 2 && tc.ab == 8) return mc_kernel<MODE, PREC, 2, 8>;
+    if (tc.kpl == 4 && tc.ab == 4) return mc_kernel<MODE, PREC, 4, 4>;
+    if (tc.kpl == 4 && tc.ab == 8) return mc_kernel<MODE, PREC, 4, 8>;
+    return nullptr;
+  }
+}
+
+static McKernel pick_kernel(int mode, int precision, const TileConfig &tc)
+{
+  if (mode == 0) {
+    if (precision == kFP32) return pick_kernel<0, kFP32>(tc);
+    if (precision == kFP32Kahan) return pick_kernel<0, kFP32Kahan>(tc);
+    if (precision == kFP64) return pick_kernel<0, kFP64>(tc);
+  } else {
+    if (precision == kFP32) return pick_kernel<1, kFP32>(tc);
+    if (precision == kFP32Kahan) return pick_kernel<1, kFP32Kahan>(tc);
+    if (precision == kFP64) return pick_kernel<1, kFP64>(tc);
+  }
+  return nullptr;
 }
 
 cudaError_t launch_kernel(int mode, int precision, const TileConfig &tc, const KArgs &a, int grid, cudaStream_t st)
 {
-  if (mode == 0) {
-    if (precision == kFP32) return launch_p<0, kFP32>(a, tc, grid, st);
-    if (precision == kFP32Kahan) return launch_p<0, kFP32Kahan>(a, tc, grid, st);
-    if (precision == kFP64) return launch_p<0, kFP64>(a, tc, grid, st);
-  } else {
-    if (precision == kFP32) return launch_p<1, kFP32>(a, tc, grid, st);
-    if (precision == kFP32Kahan) return launch_p<1, kFP32Kahan>(a, tc, grid, st);
-    if (precision == kFP64) return launch_p<1, kFP64>(a, tc, grid, st);
-  }
-  return cudaErrorInvalidValue;
+  const McKernel k = pick_kernel(mode, precision, tc);
+  if (!k) return cudaErrorInvalidValue;
+  const size_t smem = kernel_smem_bytes(a.P, a.Pall, a.lig_slots, precision, tc);
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  KArgs b = a;
+  b.group = (uint8_t)tc.group;
+  b.split = (uint8_t)tc.split;
+  k<<<grid, tc.warps_per_cta * 32, smem, st>>>(b);
+  return cudaGetLastError();
 }
 
 int kernel_occupancy(int mode, int precision, const TileConfig &tc, size_t smem)
 {
-  const void *f = nullptr;
-  const bool split = mode == 0 && precision != kFP64 && tc.group > 1;
-#define GD_PICK(M, PR, K, A)                                                                  \
-  if (mode == M && precision == PR && tc.kpl == K && tc.ab == A)                              \
-    f = split ? (const void *)mc_kernel<M, PR, K, A, (M == 0 && PR != kFP64 && K % 2 == 0)> \
-              : (const void *)mc_kernel<M, PR, K, A, false>;
-#define GD_PICK_ALL(M, PR) \
-  GD_PICK(M, PR, 1, 8) GD_PICK(M, PR, 2, 4) GD_PICK(M, PR, 2, 8) GD_PICK(M, PR, 4, 4) GD_PICK(M, PR, 4, 8)
-  GD_PICK_ALL(0, kFP32) GD_PICK_ALL(0, kFP32Kahan) GD_PICK_ALL(0, kFP64)
-  GD_PICK_ALL(1, kFP32) GD_PICK_ALL(1, kFP32Kahan) GD_PICK_ALL(1, kFP64)
-#undef GD_PICK_ALL
-#undef GD_PICK
+  const McKernel f = pick_kernel(mode, precision, tc);
   if (!f) return 0;
   if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
   int nb = 0;

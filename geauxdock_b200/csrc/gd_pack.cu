@@ -516,7 +516,7 @@ int pack_job_impl(const JobData &jd, const DevPocket &pk, const EnePara &ep, boo
       const float inv = 1.0f / (float)kcnt[t];
       for (int k = kbeg[t]; k < kbeg[t] + kcnt[t]; ++k) {
         kslot.push_back(make_int4(as_int(kde[k].x), as_int(kde[k].y), as_int(kde[k].z), as_int(inv)));
-        kslot.push_back(make_int4(a | (e << 16), 0, 0, 0));
+        kslot.push_back(make_int4(a | (e << 16), kcnt[t], 0, 0));
       }
     }
     a = e;

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -174,6 +175,24 @@ enum { kFieldNLig = 1, kFieldNPrt, kFieldNatom, kFieldNatomConf, kFieldNpoint, k
 // Launches the packer on `st` (setup, pocket, ligand kernels); failures stay in D.err.
 cudaError_t device_pack(const Complex *d_cx, const PackDst &D, cudaStream_t st);
 const char *pack_field_name(int field);
+
+// What a launch's shape depends on (gd_shape.cu).
+constexpr size_t kSmemLimit = 227 * 1024;
+struct ShapeQuery {
+  int mode = 0, precision = 0;
+  int Pmax = 0, lig_slots = 0;   // largest conformation and ligand of the launch
+  int nsm = 0;
+  int stage_opt = -1;            // pocket staged: 1 always, 0 never, -1 by the shape
+  std::function<long long(int)> items;  // work items of at most R replicas
+  size_t smem(const TileConfig &tc) const
+  {
+    return kernel_smem_bytes(tc.stage ? Pmax : 0, Pmax, lig_slots, precision, tc);
+  }
+};
+// Several warps per replica (tc.group, warps_per_cta, stage set; tc.split kept),
+// or one: false where one wave does not hold the replicas.
+bool choose_team(const ShapeQuery &q, TileConfig &tc, int &grid);
+bool choose_spread(const ShapeQuery &q, TileConfig &tc, int &grid);
 
 void free_pocket(DevPocket &p);
 void free_job(DevJobBuf &j);

@@ -35,7 +35,6 @@ using namespace gd;
 
 namespace {
 
-constexpr size_t kSmemLimitServe = 227 * 1024;
 constexpr int kMaxServeSlots = 65535;  // exchange grid's y extent
 
 using Clock = std::chrono::steady_clock;
@@ -55,6 +54,7 @@ struct ServeReq {
   bool fresh = true;   // initial energies not evaluated yet
   bool done = false;   // final round enqueued, result not yet copied out
   int nstep_round = 0;
+  int items[kMaxCtaThreads / 32 + 1] = {0};  // work items of at most R replicas
 };
 
 void stats_to_out8(const RepStats &x, double *o)
@@ -83,17 +83,22 @@ struct gd_server {
   cudaEvent_t t_ev[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   TileConfig tc{8, 2, 8};
   int precision = GD_PREC_FP32;
-  int grid = 0, Pmax = 0, Kst = 0, lig_slots = 0;
+  int grid = 0, Pmax = 0, lig_slots = 0;
   size_t smem = 0;
-  // adaptive latency mode (replica_warps = -G): the launch shapes of G, G/2, ...
-  // 2 warps per replica, largest first, each with the replicas one wave holds
+  // adaptive split order (replica_warps = -V): V, V/2, ... 2, largest first, each
+  // with the replicas one wave of as many warps per replica holds
   struct Level {
     TileConfig tc{8, 2, 8};
-    int grid = 0, Kst = 0;
+    int grid = 0;
     long long wave = 0;
   };
   Level lv[3];
   int nlv = 0;
+  int nsm = 0;
+  // launch shape of the running rounds, chosen again when the admitted jobs change
+  TileConfig rtc{8, 2, 8};
+  int rgrid = 0, rPmax = 0, rslots = 0;
+  bool reshape = true;
   int max_items = 0;
   // device tables
   DevJob *d_jobs = nullptr;
@@ -217,6 +222,17 @@ void complete(gd_server *s, std::vector<ServeReq *> &done)
   done.clear();
 }
 
+// Work items a request's replicas make at each R (append_items).
+void count_request_items(ServeReq &r)
+{
+  const std::vector<ReplicaMC> &reps = r.jd.reps;
+  for (int R = 1; R <= kMaxCtaThreads / 32; ++R)
+    for (int i = 0, k; i < r.nrep; i += k) {
+      for (k = 1; i + k < r.nrep && k < R && reps[i + k].idx_prt == reps[i].idx_prt; ++k) {}
+      ++r.items[R];
+    }
+}
+
 // Items of one launch: runs of consecutive replicas with the same protein
 // conformation, at most warps_per_cta long, heaviest job first.
 void append_items(const TileConfig &tc, const ServeReq &r, std::vector<WorkItem> &out)
@@ -230,6 +246,49 @@ void append_items(const TileConfig &tc, const ServeReq &r, std::vector<WorkItem>
     out.push_back(WorkItem{r.slot, reps[i].idx_prt, i, k});
     i += k;
   }
+}
+
+// Launch shape for the admitted jobs: sized by the largest ligand and pocket
+// among them, a team of warps per replica where one wave holds them, else one
+// warp (or the split order's number) each.
+void round_shape(gd_server *s, const std::vector<ServeReq *> &act, long long nrep)
+{
+  s->reshape = false;
+  int slots = 1, P = 0;
+  for (const ServeReq *r : act) {
+    slots = std::max(slots, (r->jd.L + 7) & ~7);
+    P = std::max(P, r->buf.dj.npoint_pad);
+  }
+  s->rslots = std::min(slots, s->lig_slots);
+  s->rPmax = P;
+  // the order of the sums: fixed, or with the adaptive one the most shares whose one wave of warps holds the replicas
+  TileConfig tc = s->tc;
+  int grid = s->grid;
+  for (int i = 0; i < s->nlv; ++i)
+    if (nrep <= s->lv[i].wave) {
+      tc = s->lv[i].tc;
+      grid = s->lv[i].grid;
+      break;
+    }
+  ShapeQuery q;
+  q.precision = s->precision;
+  q.Pmax = P;
+  q.lig_slots = s->rslots;
+  q.nsm = s->nsm;
+  q.items = [&act](int R) {
+    long long n = 0;
+    for (const ServeReq *r : act) n += r->items[R];
+    return n;
+  };
+  if (s->cfg.warps == 0 && (choose_team(q, tc, grid) || (tc.group == 1 && choose_spread(q, tc, grid)))) {
+    s->rtc = tc;
+    s->rgrid = grid;
+    return;
+  }
+  // the shape chosen at creation, at this round's sizes
+  if (tc.stage && q.smem(tc) > kSmemLimit) tc.stage = 0;
+  s->rtc = tc;
+  s->rgrid = std::max(1, kernel_occupancy(0, s->precision, tc, q.smem(tc))) * s->nsm;
 }
 
 int enqueue_round(gd_server *s, long long k, std::vector<ServeReq *> &finishing, bool &enqueued)
@@ -253,14 +312,9 @@ int enqueue_round(gd_server *s, long long k, std::vector<ServeReq *> &finishing,
     any_fresh |= r->fresh;
     nrep_act += r->nrep;
   }
-  // adaptive latency mode: the most warps per replica whose one wave holds the
-  // round's replicas; one warp per replica when none does
-  int li = -1;
-  for (int i = 0; i < s->nlv && li < 0; ++i)
-    if (nrep_act <= s->lv[i].wave) li = i;
-  const bool lat = li >= 0;
-  const TileConfig &tc = lat ? s->lv[li].tc : s->tc;
-  const int grid = lat ? s->lv[li].grid : s->grid;
+  if (s->reshape) round_shape(s, act, nrep_act);
+  const TileConfig &tc = s->rtc;
+  const int grid = s->rgrid;
   // job table of this round
   DevJob *hj = s->h_jobs[b];
   for (int i = 0; i < nslot; ++i) hj[i] = DevJob{};
@@ -296,10 +350,9 @@ int enqueue_round(gd_server *s, long long k, std::vector<ServeReq *> &finishing,
   a.jobs = s->d_jobs;
   a.queue = s->d_queue;
   a.err = s->d_err;
-  a.P = tc.stage ? s->Pmax : 0;
-  a.Kst = lat ? s->lv[li].Kst : s->Kst;
-  a.lig_slots = s->lig_slots;
-  a.group = (uint16_t)tc.group;
+  a.P = tc.stage ? s->rPmax : 0;
+  a.Pall = s->rPmax;
+  a.lig_slots = s->rslots;
   int launches = 0;
   GD_CUDA(cudaEventRecord(s->t_ev[b][0], s->st));
   if (any_fresh) {
@@ -340,6 +393,7 @@ int enqueue_round(gd_server *s, long long k, std::vector<ServeReq *> &finishing,
                               cudaMemcpyDeviceToHost, s->st));
       free_job_async(r->buf, s->st);
       r->done = true;
+      s->reshape = true;
       finishing.push_back(r);
     }
   }
@@ -348,7 +402,7 @@ int enqueue_round(gd_server *s, long long k, std::vector<ServeReq *> &finishing,
   {
     std::lock_guard<std::mutex> lk(s->mu);
     s->stats.rounds += 1;
-    s->stats.latency_rounds += lat ? 1 : 0;
+    s->stats.latency_rounds += tc.group > 1 ? 1 : 0;
     s->stats.launches += launches;
     s->stats.pose_evals += evals;
     for (ServeReq *r : finishing) s->active_reps -= r->nrep;
@@ -396,6 +450,8 @@ int admit(gd_server *s)
     r.jd.lxyz.clear();  // host copies no longer needed (replica layout is kept for the items)
     r.jd.psp.clear();
     r.jd.mxyz.clear();
+    count_request_items(r);
+    s->reshape = true;
     s->slots[r.slot] = std::move(p);
   }
   GD_CUDA(cudaEventRecord(s->up_ev, s->up));
@@ -419,6 +475,7 @@ void retire_cancelled(gd_server *s)
     for (auto &p : s->slots)
       if (p && p->ticket == t && !p->done) {
         free_job_async(p->buf, s->st);
+        s->reshape = true;
         std::lock_guard<std::mutex> lk(s->mu);
         s->active_reps -= p->nrep;
         release(s, *p);
@@ -482,14 +539,14 @@ void serve_loop(gd_server *s)
 }
 
 // Launch shape of tile tc's group: warps per CTA and pocket staging from the
-// resident replica-warps per SM; sets tc, grid, Kst, smem and the CTAs per SM.
-int choose_shape(gd_server *s, TileConfig &tc_out, int &grid, int &Kst, size_t &smem_out, int &occ_out)
+// resident replica-warps per SM; sets tc, grid, smem and the CTAs per SM.
+int choose_shape(gd_server *s, TileConfig &tc_out, int &grid, size_t &smem_out, int &occ_out)
 {
-  int nsm = 0;
-  GD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
+  GD_CUDA(cudaDeviceGetAttribute(&s->nsm, cudaDevAttrMultiProcessorCount, s->device));
+  const int nsm = s->nsm;
   const int G = tc_out.group;
   const int w0 = s->cfg.warps, wlo = w0 > 0 ? w0 : std::max(2, G), whi = w0 > 0 ? w0 : kMaxCtaThreads / 32;
-  int best_w = 0, best_res = 0, best_occ = 0, best_kst = 0, best_stage = 1;
+  int best_w = 0, best_res = 0, best_occ = 0, best_stage = 1;
   size_t best_smem = 0;
   // resident replica-warps per SM decide; the pocket is staged in shared
   // memory unless reading it through L1 lets more replicas be resident
@@ -500,29 +557,22 @@ int choose_shape(gd_server *s, TileConfig &tc_out, int &grid, int &Kst, size_t &
     tc.warps_per_cta = w;
     tc.stage = stage;
     const int P = stage ? s->Pmax : 0;
-    int kst = s->cfg.kde_stage;
-    size_t smem = kernel_smem_bytes(P, kst, s->lig_slots, w, s->precision, G);
-    if (smem > kSmemLimitServe) {
-      kst = 0;
-      smem = kernel_smem_bytes(P, kst, s->lig_slots, w, s->precision, G);
-    }
-    if (smem > kSmemLimitServe) continue;
+    const size_t smem = kernel_smem_bytes(P, s->Pmax, s->lig_slots, s->precision, tc);
+    if (smem > kSmemLimit) continue;
     const int occ = kernel_occupancy(0, s->precision, tc, smem);
     if (occ < 1) continue;
     const int resident = std::min(occ * w, 32);
-    if (resident > best_res || (resident == best_res && stage == best_stage && kst > best_kst)) {
+    if (resident > best_res) {
       best_res = resident;
       best_w = w;
       best_occ = occ;
       best_smem = smem;
-      best_kst = kst;
       best_stage = stage;
     }
   }
   if (best_w == 0) return fail(GD_E_CAPACITY, "no launch shape fits shared memory");
   tc_out.warps_per_cta = best_w;
   tc_out.stage = best_stage;
-  Kst = best_kst;
   smem_out = best_smem;
   grid = best_occ * nsm;
   occ_out = best_occ;
@@ -532,7 +582,7 @@ int choose_shape(gd_server *s, TileConfig &tc_out, int &grid, int &Kst, size_t &
 int server_configure(gd_server *s)
 {
   int occ = 0;
-  GD_TRY(choose_shape(s, s->tc, s->grid, s->Kst, s->smem, occ));
+  GD_TRY(choose_shape(s, s->tc, s->grid, s->smem, occ));
   // four waves of resident replica-warps per round: more balanced rounds (items
   // of uneven jobs) than two, with the same latency below saturation
   if (s->cfg.max_active_replicas <= 0)
@@ -541,7 +591,7 @@ int server_configure(gd_server *s)
     gd_server::Level &l = s->lv[i];
     size_t smem_l = 0;
     int occ_l = 0;
-    GD_TRY(choose_shape(s, l.tc, l.grid, l.Kst, smem_l, occ_l));
+    GD_TRY(choose_shape(s, l.tc, l.grid, smem_l, occ_l));
     l.wave = (long long)l.grid * (l.tc.warps_per_cta / l.tc.group);
   }
   return GD_OK;
@@ -590,21 +640,22 @@ int server_create(const gd_pocket_desc_t *pockets, int npocket, const EnePara *e
   s->precision = (int)gd_get_option("precision");
   s->tc = TileConfig{8, (int)o_kpl, (int)o_ab};
   const int rw = s->cfg.replica_warps;
+  // 1: the one-warp order of the sums; 2, 4 or 8: the order of a replica split over that many warps; -2, -4 or -8: up
+  // to that many by the load.  The warps per replica are chosen per round whatever the order.
   const int adapt = rw < 0 ? -rw : 0;
   s->tc.group = rw > 0 ? rw : 1;
   if (s->tc.group != 1 && s->tc.group != 2 && s->tc.group != 4 && s->tc.group != 8)
     return fail(GD_E_INVALID, "replica_warps = %d (1, 2, 4 or 8; -2, -4 or -8: adaptive)", rw);
   if (adapt && adapt != 2 && adapt != 4 && adapt != 8)
     return fail(GD_E_INVALID, "replica_warps = %d (1, 2, 4 or 8; -2, -4 or -8: adaptive)", rw);
-  default_pair_tile(s->tc.group, s->tc.kpl, s->tc.ab);
-  if (s->precision == GD_PREC_FP64) s->tc.kpl = 1, s->tc.ab = 8, s->tc.group = 1;
-  if (s->tc.kpl % 2) s->tc.group = 1;  // the split form exists for the FP32 atom-pair loop
+  default_pair_tile(s->tc.kpl, s->tc.ab);
+  const bool fp64 = s->precision == GD_PREC_FP64;  // one order
+  if (fp64) s->tc.kpl = 1, s->tc.ab = 8, s->tc.group = 1;
+  s->tc.split = s->tc.group;
   s->nlv = 0;
-  for (int g = adapt; g >= 2 && s->precision != GD_PREC_FP64; g /= 2) {
-    TileConfig t{8, (int)o_kpl, (int)o_ab};
-    t.group = g;
-    default_pair_tile(g, t.kpl, t.ab);
-    if (t.kpl % 2) break;  // the split form exists for the FP32 atom-pair loop
+  for (int g = adapt; g >= 2 && !fp64; g /= 2) {
+    TileConfig t = s->tc;
+    t.group = t.split = g;
     s->lv[s->nlv++].tc = t;
   }
   GD_TRY(server_configure(s));

@@ -1,0 +1,63 @@
+// gd_shape.cu -- launch shapes of the batched kernel: the warps a replica gets.
+#include <algorithm>
+
+#include "gd_pack.h"
+
+namespace gd {
+
+// A team is the best use of a warp that no replica needs.  Measured per step of
+// an ensemble of n replicas (40 atoms x 1500 points) on 1, 2, 4, 8 and 16 warps
+// each, where one wave holds the teams: n = 48 128 / 77 / 44 / 22 / 19 us;
+// n = 160 129 / 79 / 48 / 33 us; n = 400 130 / 91 / 57 us; n = 880
+// 151 / 109 / 84 us; n = 1760 179 / 166 us; and in the same order of G for 24
+// atoms x 600 points and 60 x 2000.  The larger team always wins while its wave
+// holds, so the line is where the wave ends.
+bool choose_team(const ShapeQuery &q, TileConfig &tc, int &grid)
+{
+  // a team's sums are those of the pair tile 4 x 8 (or of a split order): another tile asked for runs on one warp
+  if (tc.split == 1 && q.precision != kFP64 && (tc.kpl != 4 || tc.ab != 8)) return false;
+  for (int G = 16; G >= 2; G /= 2)
+    for (int R = 1; R * G <= kMaxCtaThreads / 32; ++R) {  // the fewest teams per CTA: they spread over the SMs
+      TileConfig t = tc;
+      t.group = G;
+      t.warps_per_cta = R * G;
+      // teams of 8 and 16 read the pocket from shared memory (one CTA per SM whatever it stages)
+      t.stage = q.stage_opt > 0 || (q.stage_opt < 0 && G >= 8) ? 1 : 0;
+      if (t.stage && q.smem(t) > kSmemLimit) t.stage = 0;
+      const size_t smem = q.smem(t);
+      if (smem > kSmemLimit) continue;
+      const long long items = q.items(R), wave = (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm;
+      if (items > wave) continue;
+      tc = t;
+      grid = (int)std::max(1LL, items);
+      return true;
+    }
+  return false;
+}
+
+// One warp per replica where one wave holds them all: the replicas per CTA that
+// load the fullest SM least, since a step takes about as long as that SM needs
+// (2816 replicas of 40 atoms x 1500 points: 32 warps on the fullest SM 281 us a
+// step, 20 warps 248 us).
+bool choose_spread(const ShapeQuery &q, TileConfig &tc, int &grid)
+{
+  long long best = -1;
+  for (int w = kMaxCtaThreads / 32; w >= 2; --w) {
+    TileConfig t = tc;
+    t.group = 1;
+    t.warps_per_cta = w;
+    t.stage = q.stage_opt > 0 ? 1 : 0;
+    const size_t smem = q.smem(t);
+    if (smem > kSmemLimit) continue;
+    const long long items = q.items(w);
+    if (items > (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm) continue;
+    const long long load = (items + q.nsm - 1) / q.nsm * w;
+    if (best >= 0 && load >= best) continue;
+    best = load;
+    tc = t;
+    grid = (int)std::max(1LL, items);
+  }
+  return best >= 0;
+}
+
+}  // namespace gd

@@ -95,8 +95,11 @@ int Dock(Complex *ch, Record *rh, Complex **cd, Record **rd, ParaT **pt, gd_rng_
 /* Options: "kernel" (GD_KERNEL_*), "precision" (GD_PREC_*, default
  * GD_PREC_FP32_KAHAN), "warps" (replicas
  * per CTA, 0 = autotune), "kpl", "ab" (pair-tile shape: pocket points per
- * lane 1, 2 or 4, atoms per hydrophobic block 4 or 8; default 0, the
- * library's choice: 4, 8 with one warp per replica, 2, 8 in latency mode),
+ * lane 1 (run as 2), 2 or 4, atoms per hydrophobic block 4 or 8; default 0,
+ * the library's choice: 4, 8), "replica_warps" (order the energy sums are
+ * combined in: 1, the default, the one-warp kernel's; 2, 4 or 8 that of a
+ * replica split over so many warps; the warps that run a replica are the
+ * library's choice either way, with the same results, unless "warps" is set),
  * "graph" (1: replay whole exchange intervals from a captured CUDA graph,
  * 0: launch them one by one), "stage" (1: stage each protein conformation in
  * shared memory, 0: read it through L1, -1: choose by occupancy; pockets too
@@ -301,16 +304,19 @@ typedef struct gd_server_config {
   int max_replicas_per_job; /* default 1024 */
   int max_atoms;            /* largest ligand accepted (sizes the per-warp buffers), default 128 */
   int steps_per_round;      /* MC steps between scheduling decisions, default 50 */
-  int kde_stage;            /* KDE points staged in shared memory (more: read through L1), default 0 */
+  int kde_stage;            /* accepted, without effect: KDE points are read through L1 */
   int warps;                /* warps per CTA, 0: occupancy model */
   int device;
-  int replica_warps;        /* warps per replica, 1 (default), 2, 4 or 8: latency mode, every
-                               replica's pair rows and KDE points split over that many warps;
-                               -2, -4 or -8: adaptive, each round on the most warps per replica
-                               (that many, or a power of two below it) for which one wave of
-                               the grid holds its active replicas, else one warp per replica (a
-                               request's results then depend on the load it met, within the
-                               parity tolerance either way) */
+  int replica_warps;        /* order the energy sums are combined in: 1 (default) the one-warp
+                               kernel's; 2, 4 or 8 that of a replica split over so many warps;
+                               -2, -4 or -8: adaptive, each round the order of the most shares
+                               (that many, or a power of two below it) for which one wave of as
+                               many warps per replica holds its active replicas, else the
+                               one-warp order (a request's results then depend on the load it
+                               met, within the parity tolerance either way).  The warps that
+                               run a replica are chosen per round whatever the order: the most,
+                               up to 16, for which one wave holds the round's replicas, with
+                               the same results */
 } gd_server_config_t;
 
 typedef struct gd_request {
@@ -337,7 +343,7 @@ typedef struct gd_server_stats {
   unsigned long long used_bytes, peak_bytes;
   int warps_per_cta, grid, max_active_replicas;
   int pocket_staged;                /* 1: pockets staged in shared memory, 0: read through L1 */
-  long long latency_rounds;         /* rounds run in latency mode           */
+  long long latency_rounds;         /* rounds run with several warps per replica */
 } gd_server_stats_t;
 
 void gd_server_config_default(gd_server_config_t *cfg);
