@@ -600,7 +600,7 @@ int dock_refill_device(gd_ensemble *e, const Complex *d_cx, int rb, int re, int 
   D.key1 = (uint32_t)(seed >> 32);
   GD_CUDA(cudaMemsetAsync(e->d_err, 0, 4 * sizeof(int), e->st));
   GD_CUDA(device_pack(d_cx, D, e->st));
-  e->all_launches += 3;
+  e->all_launches += 1;
   e->jobs[0].dj.key0 = D.key0;  // the host copy of the header follows the device one
   e->jobs[0].dj.key1 = D.key1;
   e->jobs[0].dj.rec = rec;

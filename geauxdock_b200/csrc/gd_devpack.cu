@@ -19,7 +19,7 @@
 // scratch array, gd_noalloc.cu) and Dock's refill of its resident state after
 // CopyH2D put the next Complex on the GPU (destination: the arenas of the
 // cached ensemble, gd_api.cu).  Invalid input sets the destination's error
-// words and no header is written; the kernels downstream check the flag.
+// words; the kernels downstream check the flag and leave the job unread.
 #include "gd_pack.h"
 
 namespace gd {
@@ -34,117 +34,141 @@ __device__ void dp_fail(const PackDst &D, int kind, int field, int value)
   atomicOr(&D.err[0], kErrPack);
 }
 
-__device__ __forceinline__ float dp_as_float(int i) { return __int_as_float(i); }
+// Sizes of the Complex, the same in every block; ok only where they are valid and
+// those the destination holds.  Block 0 reports what is wrong.
+struct DpSizes {
+  int ok, nlig, nprt, ntmp, L, K, M, P;  // P: padded points per conformation
+};
 
-// The host packer's order of the ligand type groups: the types with a
-// hydrogen-bond parameter for some point type first, each part by type.
-__device__ void dp_ligand_type_order(const Complex *cx, int *order)
+__device__ void dp_sizes(const Complex *cx, const PackDst &D, DpSizes &s)
 {
-  uint32_t m = 0;
-  for (int lt = 0; lt < kLigTypes; ++lt)
-    for (int pt = 0; pt < kPadType; ++pt)
-      if (cx->enepara.hdb0[lt][pt] > 0.1f) m |= 1u << lt;
-  int q = 0;
-  for (int t = 0; t < kLigTypes; ++t)
-    if ((m >> t) & 1u) order[q++] = t;
-  for (int t = 0; t < kLigTypes; ++t)
-    if (!((m >> t) & 1u)) order[q++] = t;
-}
-
-// Ligand atoms grouped by type in that order (stable): perm[k] = input index
-// of grouped atom k.
-__device__ void dp_ligand_order(const Complex *cx, int L, int *perm, int *ltype)
-{
-  int order[kLigTypes];
-  dp_ligand_type_order(cx, order);
-  int k = 0;
-  for (int q = 0; q < kLigTypes; ++q) {
-    const int t = order[q];
-    for (int a = 0; a < L; ++a)
-      if (cx->lig[0].t2[a] == t) {
-        perm[k] = a;
-        ltype[k] = t;
-        ++k;
-      }
-  }
-}
-
-// Sizes, validation, force-field tables, ligand atom order, KDE points sorted
-// by type with per-type ranges, and (when everything is valid) the DevJob
-// header.  One CTA of 256 threads.
-__global__ void dp_setup_kernel(const Complex *__restrict__ cx, PackDst D)
-{
-  __shared__ int s_ok, s_L, s_P, s_K, s_M, s_nlig, s_nprt, s_ntmp, s_nk;
-  __shared__ int s_kcnt[kLigTypes], s_kbeg[kLigTypes];
-  __shared__ int s_perm[GD_MAXLIG], s_ltype[GD_MAXLIG];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ int s_conf, s_point, s_max;  // first ligand conformation of another atom count, first bad point count
+  const int tid = threadIdx.x;
   if (tid == 0) {
-    const int nlig = cx->size.n_lig, nprt = cx->size.n_prt, K = cx->size.kde_npoint, M = cx->size.mcs_nrow;
-    const int ntmp = cx->size.n_tmp;
-    const int L = cx->lig[0].lig_natom;
-    int ok = 1, P = 0;
-    if (nlig < 1 || nlig > GD_MAX_CONF_LIG) dp_fail(D, nlig < 1 ? kPackFailInput : kPackFailCapacity, kFieldNLig, nlig), ok = 0;
-    else if (nprt < 1 || nprt > GD_MAX_CONF_PRT) dp_fail(D, nprt < 1 ? kPackFailInput : kPackFailCapacity, kFieldNPrt, nprt), ok = 0;
-    else if (L < 1 || L > GD_MAXLIG) dp_fail(D, L < 1 ? kPackFailInput : kPackFailCapacity, kFieldNatom, L), ok = 0;
-    else if (K < 0 || K > GD_MAXKDE) dp_fail(D, K < 0 ? kPackFailInput : kPackFailCapacity, kFieldKde, K), ok = 0;
-    else if (M < 1 || M > GD_MAX_MCS_ROW) dp_fail(D, M < 1 ? kPackFailInput : kPackFailCapacity, kFieldMcs, M), ok = 0;
-    else if (D.rep && (ntmp < 1 || ntmp > GD_MAX_TMP)) dp_fail(D, kPackFailInput, kFieldNTmp, ntmp), ok = 0;
-    if (ok)
-      for (int i = 0; i < nlig; ++i)
-        if (cx->lig[i].lig_natom != L) {
-          dp_fail(D, kPackFailInput, kFieldNatomConf, i);
-          ok = 0;
-          break;
-        }
-    if (ok)
-      for (int i = 0; i < nprt; ++i) {
-        const int n = cx->prt[i].prt_npoint;
-        if (n < 1 || n > GD_MAXPRO) {
-          dp_fail(D, n < 1 ? kPackFailInput : kPackFailCapacity, kFieldNpoint, n);
-          ok = 0;
-          break;
-        }
-        P = max(P, n);
-      }
-    const int Ppad = ((P + kPointAlign - 1) / kPointAlign) * kPointAlign;
-    if (ok && D.Ppad > 0 && Ppad != D.Ppad) dp_fail(D, kPackFailShape, kFieldNpoint, P), ok = 0;
-    if (ok && D.expect_L >= 0 && L != D.expect_L) dp_fail(D, kPackFailShape, kFieldNatom, L), ok = 0;
-    if (ok && D.expect_nlig >= 0 && nlig != D.expect_nlig) dp_fail(D, kPackFailShape, kFieldNLig, nlig), ok = 0;
-    if (ok && D.expect_nprt >= 0 && nprt != D.expect_nprt) dp_fail(D, kPackFailShape, kFieldNPrt, nprt), ok = 0;
-    if (ok && D.expect_M >= 0 && M != D.expect_M) dp_fail(D, kPackFailShape, kFieldMcs, M), ok = 0;
-    if (ok && D.rep && D.expect_ntmp >= 0 && ntmp != D.expect_ntmp) dp_fail(D, kPackFailShape, kFieldNTmp, ntmp), ok = 0;
-    if (ok && D.rep && (D.rep_begin < 0 || D.rep_begin + D.nrep > cx->size.n_rep))
-      dp_fail(D, kPackFailShape, kFieldReplica, D.rep_begin + D.nrep), ok = 0;
-    s_ok = ok;
-    s_L = L;
-    s_P = D.Ppad > 0 ? D.Ppad : Ppad;
-    s_K = K;
-    s_M = M;
-    s_nlig = nlig;
-    s_nprt = nprt;
-    s_ntmp = ntmp;
+    s.nlig = cx->size.n_lig;
+    s.nprt = cx->size.n_prt;
+    s.ntmp = cx->size.n_tmp;
+    s.K = cx->size.kde_npoint;
+    s.M = cx->size.mcs_nrow;
+    s.L = cx->lig[0].lig_natom;
+    s_conf = s_point = 1 << 30;
+    s_max = 0;
   }
   __syncthreads();
-  if (!s_ok) return;
-  const int L = s_L, K = s_K, M = s_M, nlig = s_nlig, nprt = s_nprt;
+  if (tid < s.nlig && tid < GD_MAX_CONF_LIG && cx->lig[tid].lig_natom != s.L) atomicMin(&s_conf, tid);
+  if (tid < s.nprt && tid < GD_MAX_CONF_PRT) {
+    const int n = cx->prt[tid].prt_npoint;
+    if (n < 1 || n > GD_MAXPRO) atomicMin(&s_point, tid);
+    else atomicMax(&s_max, n);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    int kind = 0, field = 0, value = 0;
+    auto bad = [&](int k, int f, int v) {
+      if (kind == 0) kind = k, field = f, value = v;
+    };
+    auto range = [&](int v, int lo, int hi, int f) {
+      if (v < lo || v > hi) bad(v < lo ? kPackFailInput : kPackFailCapacity, f, v);
+    };
+    auto want = [&](int v, int expect, int f, int tell) {
+      if (expect >= 0 && v != expect) bad(kPackFailShape, f, tell);
+    };
+    range(s.nlig, 1, GD_MAX_CONF_LIG, kFieldNLig);
+    range(s.nprt, 1, GD_MAX_CONF_PRT, kFieldNPrt);
+    range(s.L, 1, GD_MAXLIG, kFieldNatom);
+    range(s.K, 0, GD_MAXKDE, kFieldKde);
+    range(s.M, 1, GD_MAX_MCS_ROW, kFieldMcs);
+    if (D.rep && (s.ntmp < 1 || s.ntmp > GD_MAX_TMP)) bad(kPackFailInput, kFieldNTmp, s.ntmp);
+    if (kind == 0 && s_conf < s.nlig) bad(kPackFailInput, kFieldNatomConf, s_conf);
+    if (kind == 0 && s_point < s.nprt) range(cx->prt[s_point].prt_npoint, 1, GD_MAXPRO, kFieldNpoint);
+    s.P = ((s_max + kPointAlign - 1) / kPointAlign) * kPointAlign;
+    want(s.P, D.Ppad > 0 ? D.Ppad : -1, kFieldNpoint, s_max);
+    want(s.L, D.expect_L, kFieldNatom, s.L);
+    want(s.nlig, D.expect_nlig, kFieldNLig, s.nlig);
+    want(s.nprt, D.expect_nprt, kFieldNPrt, s.nprt);
+    want(s.M, D.expect_M, kFieldMcs, s.M);
+    if (D.rep) want(s.ntmp, D.expect_ntmp, kFieldNTmp, s.ntmp);
+    if (D.rep && (D.rep_begin < 0 || D.rep_begin + D.nrep > cx->size.n_rep))
+      bad(kPackFailShape, kFieldReplica, D.rep_begin + D.nrep);
+    s.ok = kind == 0;
+    if (kind && blockIdx.x == 0) dp_fail(D, kind, field, value);
+  }
+  __syncthreads();
+}
 
-  // type and index validation
+// Bit pt of point[lt]'s union: the point types, and bit lt the ligand types, with
+// a hydrogen-bond parameter (hdb0 > 0.1).
+__device__ void dp_hdb_types(const Complex *cx, uint32_t &points, uint32_t &ligands)
+{
+  __shared__ uint32_t s_p, s_l;
+  if (threadIdx.x == 0) s_p = s_l = 0u;
+  __syncthreads();
+  for (int q = threadIdx.x; q < kLigTypes * kPadType; q += blockDim.x) {
+    const int lt = q / kPadType, pt = q % kPadType;
+    if (cx->enepara.hdb0[lt][pt] > 0.1f) {
+      atomicOr(&s_p, 1u << pt);
+      atomicOr(&s_l, 1u << lt);
+    }
+  }
+  __syncthreads();
+  points = s_p;
+  ligands = s_l;
+}
+
+// Ligand atoms grouped by type, the types with a hydrogen-bond parameter first,
+// each part by type (stable): perm[k] = input index of grouped atom k; and each
+// type's atoms [range & 0xffff, range >> 16).  An atom of an invalid type keeps
+// its place in the order of the others (block 0 reports it).
+__device__ void dp_ligand_order(const Complex *cx, int L, uint32_t hdb_ligands, int *perm, int *ltype, int *range)
+{
+  __shared__ int s_type[GD_MAXLIG];
+  const int a = threadIdx.x;
+  if (a < kLigTypes) range[a] = 0;
+  if (a < L) {
+    const int t = cx->lig[0].t2[a];
+    s_type[a] = t >= 0 && t < kLigTypes ? t : 0;
+  }
+  __syncthreads();
+  auto key = [&](int t) { return (((hdb_ligands >> t) & 1u) ? 0 : 32) + t; };
+  int t = 0, r = 0, beg = 0, end = 0;
+  if (a < L) {
+    t = s_type[a];
+    const int k = key(t);
+    for (int b = 0; b < L; ++b) {
+      const int kb = key(s_type[b]);
+      r += kb < k || (kb == k && b < a);
+      beg += kb < k;
+      end += kb <= k;
+    }
+    perm[r] = a;
+    ltype[r] = t;
+    range[t] = beg | (end << 16);
+  }
+  __syncthreads();
+}
+
+// Block 0: validation of the ligand and the templates, force-field tables, ligand
+// atom groups, centres, KDE slots, and the DevJob header (read only where the
+// error flag stays clear).
+__device__ void dp_setup(const Complex *cx, const PackDst &D, const DpSizes &s)
+{
+  __shared__ int s_kcnt[kLigTypes], s_kbeg[kLigTypes], s_slot[kLigTypes], s_nk, s_nslot;
+  __shared__ int s_perm[GD_MAXLIG], s_ltype[GD_MAXLIG], s_range[kLigTypes];
+  __shared__ unsigned char s_kt[GD_MAXKDE];  // KDE point types (255: none of the ligand's types)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int L = s.L, K = s.K, M = s.M, nlig = s.nlig, nprt = s.nprt;
   for (int a = tid; a < L; a += blockDim.x) {
     const int t = cx->lig[0].t2[a];
     if (t < 0 || t >= kLigTypes) dp_fail(D, kPackFailInput, kFieldLigType, a);
   }
-  for (int q = tid; q < nprt * GD_MAXPRO; q += blockDim.x) {
-    const int i = q / GD_MAXPRO, k = q % GD_MAXPRO;
-    const Protein &pr = cx->prt[i];
-    if (k >= pr.prt_npoint) continue;
-    if (pr.t[k] < 0 || pr.t[k] >= kPadType) dp_fail(D, kPackFailInput, kFieldPrtType, k);
-    if (pr.c[k] == 2 && (pr.seq3r[k] < 0 || pr.seq3r[k] >= GD_MAXPRO)) dp_fail(D, kPackFailInput, kFieldSeq3r, k);
+  for (int m = warp; m < M; m += nwarps) {
+    bool any = false;
+    for (int a = lane; a < L; a += 32) any |= cx->mcs[m].x[a] != GD_MCS_INVALID_COORD;
+    if (!__any_sync(0xffffffffu, any) && lane == 0) dp_fail(D, kPackFailInput, kFieldMcsRow, m);
   }
-  for (int m = tid; m < M; m += blockDim.x) {
-    int n = 0;
-    for (int a = 0; a < L; ++a) n += cx->mcs[m].x[a] != GD_MCS_INVALID_COORD;
-    if (n == 0) dp_fail(D, kPackFailInput, kFieldMcsRow, m);
-  }
+  uint32_t hp, hl;
+  dp_hdb_types(cx, hp, hl);
+  dp_ligand_order(cx, L, hl, s_perm, s_ltype, s_range);
 
   // force-field tables, as the host packer's build_params
   const EnePara &ep = cx->enepara;
@@ -165,13 +189,14 @@ __global__ void dp_setup_kernel(const Complex *__restrict__ cx, PackDst D)
       D.ref4[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
-  for (int q = tid; q < kLigTypes; q += blockDim.x) {
-    par.hpl0[q] = ep.hpl0[q];
-    par.hpl1[q] = ep.hpl1[q];
-    par.hpl2[q] = ep.hpl2[q];
-    uint32_t m = 0;
-    for (int pt = 0; pt < kPadType; ++pt) m |= (ep.hdb0[q][pt] > 0.1f ? 1u : 0u) << pt;
-    par.hdbmask[q] = m;
+  for (int q = warp; q < kLigTypes; q += nwarps) {
+    const uint32_t m = __ballot_sync(0xffffffffu, lane < kPadType && ep.hdb0[q][lane] > 0.1f);
+    if (lane == 0) {
+      par.hpl0[q] = ep.hpl0[q];
+      par.hpl1[q] = ep.hpl1[q];
+      par.hpl2[q] = ep.hpl2[q];
+      par.hdbmask[q] = m;
+    }
   }
   for (int q = tid; q < 12; q += blockDim.x) {
     par.a_para[q] = q < GD_MAXWEI ? ep.a_para[q] : 0.f;
@@ -193,107 +218,79 @@ __global__ void dp_setup_kernel(const Complex *__restrict__ cx, PackDst D)
     par.ele_b = (float)((double)ep.b1 * ep.el1 * ep.el1 * ep.el1);
     par.ele_d2max = (float)(1.0 / ((double)ep.el1 * ep.el1));
     par.hdb_cinv = (float)(1.0 / kHdbC);
-    for (int i = 0; i < 6; ++i) par.move_scale[i] = cx->mcpara.move_scale[i];
     par.kde3 = ep.kde3;
     par.pad_ = 0.f;
-    // ligand atoms grouped by type, stable (the host packer's order)
-    dp_ligand_order(cx, L, s_perm, s_ltype);
-    int end = L;
-    for (int a = L - 1; a >= 0; --a) {
-      if (a + 1 < L && s_ltype[a + 1] != s_ltype[a]) end = a + 1;
-      D.lgrp[a] = make_int2(s_ltype[a], end);
-    }
   }
+  for (int q = tid; q < 6; q += blockDim.x) par.move_scale[q] = cx->mcpara.move_scale[q];
+  for (int a = tid; a < L; a += blockDim.x) D.lgrp[a] = make_int2(s_ltype[a], s_range[s_ltype[a]] >> 16);
   for (int q = tid; q < nlig * 3; q += blockDim.x) D.lcenter[q] = cx->lig[q / 3].center[q % 3];
   for (int q = tid; q < nprt * 3; q += blockDim.x) D.pcenter[q] = cx->prt[q / 3].pocket_center[q % 3];
   for (int q = tid; q < M; q += blockDim.x) D.tcc[q] = cx->mcs[q].tcc;
 
-  // KDE points of ligand types, sorted by type (stable): count, prefix, scatter
-  const int nwarps = blockDim.x >> 5;
+  // KDE points of ligand types, sorted by type (stable), and slots in the grouped
+  // ligand's type order, one per KDE point of a type the ligand has: count, prefix, scatter
+  for (int k = tid; k < K; k += blockDim.x) {
+    const int t = cx->kde.t[k];
+    s_kt[k] = t >= 0 && t < kLigTypes ? (unsigned char)t : (unsigned char)255;
+  }
+  __syncthreads();
   for (int t = warp; t < kLigTypes; t += nwarps) {
     int cnt = 0;
-    for (int k0 = 0; k0 < K; k0 += 32) {
-      const int k = k0 + lane;
-      cnt += __popc(__ballot_sync(0xffffffffu, k < K && cx->kde.t[k] == t));
-    }
+    for (int k0 = 0; k0 < K; k0 += 32) cnt += __popc(__ballot_sync(0xffffffffu, k0 + lane < K && s_kt[k0 + lane] == t));
     if (lane == 0) s_kcnt[t] = cnt;
   }
   __syncthreads();
   if (tid == 0) {
-    int b = 0;
+    int b = 0, o = 0;
     for (int t = 0; t < kLigTypes; ++t) {
       s_kbeg[t] = s_kcnt[t] ? b : 0;
       b += s_kcnt[t];
     }
+    for (int a = 0; a < L; a = s_range[s_ltype[a]] >> 16) {
+      s_slot[s_ltype[a]] = o;
+      o += s_kcnt[s_ltype[a]];
+    }
     s_nk = b;
+    s_nslot = o;
     if (D.nkde_expect >= 0 && b != D.nkde_expect) dp_fail(D, kPackFailShape, kFieldKde, b);
   }
   __syncthreads();
   for (int t = warp; t < kLigTypes; t += nwarps) {
-    int at = s_kbeg[t];
+    int at = 0;
+    const int range = s_range[t];
+    const float inv = 1.0f / (float)s_kcnt[t];
     for (int k0 = 0; k0 < K; k0 += 32) {
       const int k = k0 + lane;
-      const bool m = k < K && cx->kde.t[k] == t;
+      const bool m = k < K && s_kt[k] == t;
       const unsigned b = __ballot_sync(0xffffffffu, m);
-      if (m && at + __popc(b & ((1u << lane) - 1u)) < D.kde_cap) {
-        const int o = at + __popc(b & ((1u << lane) - 1u));
-        D.kde[o] = make_float4(cx->kde.x[k], cx->kde.y[k], cx->kde.z[k], dp_as_float(t));
+      const int rank = at + __popc(b & ((1u << lane) - 1u)), o = s_kbeg[t] + rank;
+      if (m && o < D.kde_cap) {
+        const float x = cx->kde.x[k], y = cx->kde.y[k], z = cx->kde.z[k];
+        if (D.kde) D.kde[o] = make_float4(x, y, z, __int_as_float(t));
+        const int q = s_slot[t] + rank;
+        if (range && q < D.kde_cap) {
+          D.kslot[2 * q] = make_int4(__float_as_int(x), __float_as_int(y), __float_as_int(z), __float_as_int(inv));
+          D.kslot[2 * q + 1] = make_int4(range, s_kcnt[t], 0, 0);
+        }
       }
       at += __popc(b);
     }
   }
-  if (tid == 0 && s_nk == 0 && D.kde_cap > 0) D.kde[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-  __syncthreads();
-  // KDE slots (the host packer's order): for each ligand type group, each KDE
-  // point of its type, with the group's atom range and 1/(points of the type)
-  __shared__ int s_ga[kLigTypes], s_ge[kLigTypes], s_gt[kLigTypes], s_go[kLigTypes + 1], s_ng, s_valid;
-  // (only for a valid Complex: with an out-of-range ligand type the grouped
-  // order does not cover every atom)
-  if (tid == 0) s_valid = (*(volatile int *)D.err & kErrPack) == 0;
-  __syncthreads();
-  if (D.kslot && s_valid) {
-    if (tid == 0) {
-      int ng = 0, off = 0;
-      for (int a = 0; a < L;) {
-        const int t = s_ltype[a];
-        int e = a;
-        while (e < L && s_ltype[e] == t) ++e;
-        if (s_kcnt[t] > 0) {
-          s_ga[ng] = a;
-          s_ge[ng] = e;
-          s_gt[ng] = t;
-          s_go[ng] = off;
-          off += s_kcnt[t];
-          ++ng;
-        }
-        a = e;
-      }
-      s_go[ng] = off;
-      s_ng = ng;
-    }
-    __syncthreads();
-    const int nslot = s_go[s_ng];
-    for (int q = tid; q < nslot && q < D.kde_cap; q += blockDim.x) {
-      int g = 0;
-      while (q >= s_go[g + 1]) ++g;
-      const int t = s_gt[g];
-      const float4 p = D.kde[s_kbeg[t] + (q - s_go[g])];
-      const float inv = 1.0f / (float)s_kcnt[t];
-      D.kslot[2 * q] = make_int4(__float_as_int(p.x), __float_as_int(p.y), __float_as_int(p.z), __float_as_int(inv));
-      D.kslot[2 * q + 1] = make_int4(s_ga[g] | (s_ge[g] << 16), s_kcnt[t], 0, 0);
-    }
-    __syncthreads();
+  if (tid == 0 && s_nk == 0 && D.kde && D.kde_cap > 0) D.kde[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (tid < kLigTypes) {
+    D.job->kbeg[tid] = s_kbeg[tid];
+    D.job->kcnt[tid] = s_kcnt[tid];
+    D.job->trange[tid] = s_range[tid];
   }
-  // the header only for a valid Complex: the kernels that read it run only then
-  if (tid == 0 && (*(volatile int *)D.err & kErrPack) == 0) {
-    DevJob J;
+  if (tid == 0) {
+    DevJob &J = *D.job;
     J.natom = L;
     J.nlig = nlig;
     J.lstride = (L + 3) & ~3;
     J.lig = D.lig;
     J.lgrp = D.lgrp;
     J.lcenter = D.lcenter;
-    J.npoint_pad = s_P;
+    J.npoint_pad = s.P;
     J.nprt = nprt;
     J.pos = D.pos;
     J.aux = D.aux;
@@ -304,18 +301,16 @@ __global__ void dp_setup_kernel(const Complex *__restrict__ cx, PackDst D)
     J.pcell = D.pcell;
     J.pcell_cnt = D.pcell_cnt;
     J.pcell_stride = D.pcell_stride;
-    for (int t = 0; t < kLigTypes; ++t) {
-      J.kbeg[t] = s_kbeg[t];
-      J.kcnt[t] = s_kcnt[t];
-    }
+    J.pcell4 = D.pcell4;
+    J.psp_table = &cx->psp.psp[0][0];
     J.nkde = s_nk;
     J.kde = D.kde;
-    J.nkslot = (D.kslot && s_valid) ? min(s_go[s_ng], D.kde_cap) : 0;
+    J.nkslot = min(s_nslot, D.kde_cap);
     J.kslot = D.kslot;
     J.nmcs = M;
     J.mcs = D.mcs;
     J.tcc = D.tcc;
-    J.ntmp = D.rep ? s_ntmp : 0;
+    J.ntmp = D.rep ? s.ntmp : 0;
     J.minus_beta = D.minus_beta;
     J.par = D.par;
     J.ref4 = D.ref4;
@@ -332,126 +327,114 @@ __global__ void dp_setup_kernel(const Complex *__restrict__ cx, PackDst D)
     J.nsteps = 0;
     J.xsweep = -1;
     J.pad_ = 0;
-    *D.job = J;
   }
 }
 
-// One CTA per protein conformation: points ordered as the host packer orders
-// them (hydrophobic-contact points first, each part by hydrogen-bond group and point type,
-// stable; 60 buckets (cdc, type), two per warp, counted and scattered with
-// warp ballots), inert padding, the pocket-specific potential gathered with
-// its non-zero type mask, and its non-zero cells for the ligand's types, by
-// type then point (one warp per type, counted and scattered the same way).
-__global__ void __launch_bounds__(1024) dp_pocket_kernel(const Complex *__restrict__ cx, PackDst D)
+// One block per protein conformation: points ordered as the host packer orders
+// them (hydrophobic-contact points first, each part by hydrogen-bond group and
+// point type, stable: 60 buckets counted and ranked with warp ballots), inert
+// padding, the pocket-specific potential gathered with its non-zero type mask,
+// and its non-zero cells for the ligand's types, by type then point.
+__device__ void dp_pocket(const Complex *cx, const PackDst &D, const DpSizes &s, int i)
 {
   constexpr int kBuckets = 2 * kPadType;
-  __shared__ int s_cnt[kBuckets], s_beg[kBuckets], s_rank[kPadType];
-  if (*(volatile int *)D.err & kErrPack) return;
-  const int i = blockIdx.x;
-  const int nprt = cx->size.n_prt;
-  if (i >= nprt) return;
+  __shared__ unsigned char s_key[GD_MAXPRO];
+  __shared__ short s_src[GD_MAXPRO];       // input index of sorted point j
+  __shared__ uint32_t s_mask[GD_MAXPRO];   // ligand types with a potential at sorted point j
+  __shared__ int s_cnt[kBuckets], s_beg[kBuckets], s_ccnt[kLigTypes], s_cbeg[kLigTypes];
+  __shared__ int s_perm[GD_MAXLIG], s_ltype[GD_MAXLIG], s_range[kLigTypes];
   const Protein &pr = cx->prt[i];
-  int P = 0;
-  for (int c = 0; c < nprt; ++c) P = max(P, cx->prt[c].prt_npoint);
-  const int np = pr.prt_npoint;
-  const int Pp = D.Ppad > 0 ? D.Ppad : ((P + kPointAlign - 1) / kPointAlign) * kPointAlign;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  // the host packer's order: per part (cdc == 1 first) the point types with a
-  // hydrogen-bond parameter first, each group by type: rank of each type
-  if (threadIdx.x == 0) {
-    uint32_t m = 0;
-    for (int lt = 0; lt < kLigTypes; ++lt)
-      for (int pt = 0; pt < kPadType; ++pt)
-        if (cx->enepara.hdb0[lt][pt] > 0.1f) m |= 1u << pt;
-    int r = 0;
-    for (int pt = 0; pt < kPadType; ++pt)
-      if ((m >> pt) & 1u) s_rank[pt] = r++;
-    for (int pt = 0; pt < kPadType; ++pt)
-      if (!((m >> pt) & 1u)) s_rank[pt] = r++;
+  const int np = pr.prt_npoint, Pp = s.P;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  uint32_t hp, hl;
+  dp_hdb_types(cx, hp, hl);
+  dp_ligand_order(cx, s.L, hl, s_perm, s_ltype, s_range);
+  for (int k = tid; k < np; k += blockDim.x) {
+    const int t = pr.t[k];
+    int rank = kBuckets;  // an invalid type: left out
+    if (t < 0 || t >= kPadType) {
+      dp_fail(D, kPackFailInput, kFieldPrtType, k);
+    } else {
+      const uint32_t below = (1u << t) - 1u;
+      rank = (pr.cdc[k] == 1 ? 0 : kPadType) +
+             (((hp >> t) & 1u) ? __popc(hp & below) : __popc(hp) + t - __popc(hp & below));
+    }
+    s_key[k] = (unsigned char)rank;
   }
+  for (int j = tid; j < Pp; j += blockDim.x) s_src[j] = -1;
   __syncthreads();
-  auto bucket = [&](int k) { return (pr.cdc[k] == 1 ? 0 : kPadType) + s_rank[pr.t[k]]; };
   for (int bk = warp; bk < kBuckets; bk += nwarps) {
     int cnt = 0;
-    for (int k0 = 0; k0 < np; k0 += 32) {
-      const int k = k0 + lane;
-      cnt += __popc(__ballot_sync(0xffffffffu, k < np && bucket(k) == bk));
-    }
+    for (int k0 = 0; k0 < np; k0 += 32) cnt += __popc(__ballot_sync(0xffffffffu, k0 + lane < np && s_key[k0 + lane] == bk));
     if (lane == 0) s_cnt[bk] = cnt;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int b = 0;
+  if (tid == 0) {
+    int b = 0, nc = 0;
     for (int q = 0; q < kBuckets; ++q) {
       s_beg[q] = b;
       b += s_cnt[q];
+      if (q < kPadType) nc += s_cnt[q];
     }
-    int nc = 0;
-    for (int q = 0; q < kPadType; ++q) nc += s_cnt[q];
     D.ncdc[i] = nc;
+  }
+  __syncthreads();
+  for (int bk = warp; bk < kBuckets; bk += nwarps) {
+    int at = s_beg[bk];
+    if (s_cnt[bk] == 0) continue;
+    for (int k0 = 0; k0 < np; k0 += 32) {
+      const int k = k0 + lane;
+      const bool m = k < np && s_key[k] == bk;
+      const unsigned b = __ballot_sync(0xffffffffu, m);
+      if (m) s_src[at + __popc(b & ((1u << lane) - 1u))] = (short)k;
+      at += __popc(b);
+    }
   }
   __syncthreads();
   float4 *pos = D.pos + (size_t)i * Pp;
   float2 *aux = D.aux + (size_t)i * Pp;
-  float *psp = D.psp + (size_t)i * kLigTypes * Pp;
-  uint32_t *pm = D.pspmask + (size_t)i * Pp;
-  for (int bk = warp; bk < kBuckets; bk += nwarps) {
-    int at = s_beg[bk];
-    for (int k0 = 0; k0 < np; k0 += 32) {
-      const int k = k0 + lane;
-      const bool m = k < np && bucket(k) == bk;
-      const unsigned b = __ballot_sync(0xffffffffu, m);
-      if (m) {
-        const int j = at + __popc(b & ((1u << lane) - 1u));
-        pos[j] = make_float4(pr.x[k], pr.y[k], pr.z[k], pr.ele[k]);
-        aux[j] = make_float2(pr.cdc[k] == 1 ? pr.hpp[k] : 0.f, dp_as_float(pr.t[k]));
-        const bool c2 = pr.c[k] == 2;
-        const int col = pr.seq3r[k];
-        uint32_t mask = 0;
-        for (int lt = 0; lt < kLigTypes; ++lt) {
-          const float v = c2 ? cx->psp.psp[lt][col] : 0.f;
-          psp[(size_t)lt * Pp + j] = v;
-          mask |= (v != 0.f ? 1u : 0u) << lt;
+  for (int j = tid; j < Pp; j += blockDim.x) {
+    const int k = s_src[j];
+    uint32_t mask = 0u;
+    if (k >= 0) {
+      pos[j] = make_float4(pr.x[k], pr.y[k], pr.z[k], pr.ele[k]);
+      aux[j] = make_float2(pr.cdc[k] == 1 ? pr.hpp[k] : 0.f, __int_as_float(pr.t[k]));
+      int col = -1;
+      if (pr.c[k] == 2) {
+        col = pr.seq3r[k];
+        if (col < 0 || col >= GD_MAXPRO) {
+          dp_fail(D, kPackFailInput, kFieldSeq3r, k);
+          col = -1;
         }
-        pm[j] = mask;
       }
-      at += __popc(b);
+      if (col >= 0)
+#pragma unroll
+        for (int lt = 0; lt < kLigTypes; ++lt) mask |= (cx->psp.psp[lt][col] != 0.f ? 1u : 0u) << lt;
+    } else {
+      pos[j] = make_float4(1.0e4f + (float)j, 1.0e4f, 1.0e4f, 0.f);
+      aux[j] = make_float2(0.f, __int_as_float(kPadType));
     }
-  }
-  for (int j = np + threadIdx.x; j < Pp; j += blockDim.x) {
-    pos[j] = make_float4(1.0e4f + (float)j, 1.0e4f, 1.0e4f, 0.f);
-    aux[j] = make_float2(0.f, dp_as_float(kPadType));
-    pm[j] = 0u;
-    for (int lt = 0; lt < kLigTypes; ++lt) psp[(size_t)lt * Pp + j] = 0.f;
-  }
-  if (!D.pcell) return;
-  // cells: the atoms of type t are [tbeg, tbeg + tcnt) of the type-grouped ligand
-  __shared__ int s_tcnt[kLigTypes], s_tbeg[kLigTypes], s_ccnt[kLigTypes], s_cbeg[kLigTypes];
-  __syncthreads();  // this CTA's mask writes above are read below
-  const int L = cx->lig[0].lig_natom;
-  if (warp < kLigTypes) {
-    int na = 0;
-    for (int a0 = 0; a0 < L; a0 += 32)
-      na += __popc(__ballot_sync(0xffffffffu, a0 + lane < L && cx->lig[0].t2[a0 + lane] == warp));
-    int nc = 0;
-    if (na > 0)
-      for (int j0 = 0; j0 < Pp; j0 += 32)
-        nc += __popc(__ballot_sync(0xffffffffu, j0 + lane < Pp && ((pm[j0 + lane] >> warp) & 1u)));
-    if (lane == 0) {
-      s_tcnt[warp] = na;
-      s_ccnt[warp] = nc;
-    }
+    s_mask[j] = mask;
+    if (D.pspmask) D.pspmask[(size_t)i * Pp + j] = mask;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    // atom ranges in the grouped ligand's type order, cells by type index
-    int order[kLigTypes];
-    dp_ligand_type_order(cx, order);
-    int a = 0, c = 0;
-    for (int q = 0; q < kLigTypes; ++q) {
-      s_tbeg[order[q]] = a;
-      a += s_tcnt[order[q]];
-    }
+  if (D.psp) {
+    float *psp = D.psp + (size_t)i * kLigTypes * Pp;
+    for (int lt = warp; lt < kLigTypes; lt += nwarps)
+      for (int j = lane; j < Pp; j += 32)
+        psp[(size_t)lt * Pp + j] = ((s_mask[j] >> lt) & 1u) ? cx->psp.psp[lt][pr.seq3r[s_src[j]]] : 0.f;
+  }
+  // cells of the ligand's types: the atoms of type t are s_range[t]
+  if (warp < kLigTypes) {
+    int nc = 0;
+    if (s_range[warp])
+      for (int j0 = 0; j0 < Pp; j0 += 32)
+        nc += __popc(__ballot_sync(0xffffffffu, (s_mask[j0 + lane] >> warp) & 1u));
+    if (lane == 0) s_ccnt[warp] = nc;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    int c = 0;
     for (int t = 0; t < kLigTypes; ++t) {
       s_cbeg[t] = c;
       c += s_ccnt[t];
@@ -460,58 +443,60 @@ __global__ void __launch_bounds__(1024) dp_pocket_kernel(const Complex *__restri
     if (c > D.pcell_stride) dp_fail(D, kPackFailCapacity, kFieldPcell, c);
   }
   __syncthreads();
-  if (warp < kLigTypes && s_tcnt[warp] > 0) {
-    int4 *cell = D.pcell + (size_t)i * D.pcell_stride * 2;
-    const int t = warp, rng = s_tbeg[t] | ((s_tbeg[t] + s_tcnt[t]) << 16);
+  if (warp < kLigTypes && s_ccnt[warp] > 0) {
+    const int t = warp;
     int at = s_cbeg[t];
     for (int j0 = 0; j0 < Pp; j0 += 32) {
       const int j = j0 + lane;
-      const bool m = j < Pp && ((pm[j] >> t) & 1u);
+      const bool m = (s_mask[j] >> t) & 1u;
       const unsigned b = __ballot_sync(0xffffffffu, m);
       const int o = at + __popc(b & ((1u << lane) - 1u));
       if (m && o < D.pcell_stride) {
-        const float4 q = pos[j];
-        const int pt = __float_as_int(aux[j].y);
-        cell[2 * o] = make_int4(__float_as_int(q.x), __float_as_int(q.y), __float_as_int(q.z),
-                                __float_as_int(psp[(size_t)t * Pp + j]));
-        cell[2 * o + 1] = make_int4(rng, __float_as_int(D.par->tab4[t][pt].z), t, j);
+        const int k = s_src[j], col = pr.seq3r[k];
+        if (D.pcell) {
+          int4 *cell = D.pcell + ((size_t)i * D.pcell_stride + o) * 2;
+          cell[0] = make_int4(__float_as_int(pr.x[k]), __float_as_int(pr.y[k]), __float_as_int(pr.z[k]),
+                              __float_as_int(cx->psp.psp[t][col]));
+          cell[1] = make_int4(s_range[t], __float_as_int(-cx->enepara.pmf0[t][pr.t[k]]), t, j);
+        } else {
+          D.pcell4[(size_t)i * D.pcell_stride + o] = pack_cell4(j, t, col);
+        }
       }
       at += __popc(b);
     }
   }
 }
 
-// Ligand conformations in grouped atom order, MCS templates atom-major; with a
-// replica destination also the replica range, accept flags, statistics and
-// the temperature ladder.
-__global__ void dp_ligand_kernel(const Complex *__restrict__ cx, PackDst D)
+// The other blocks: ligand conformations in grouped atom order, MCS templates
+// atom-major; with a replica destination also the replica range, accept flags,
+// statistics and the temperature ladder.
+__device__ void dp_ligand(const Complex *cx, const PackDst &D, const DpSizes &s, int block, int nblock)
 {
-  __shared__ int s_perm[GD_MAXLIG], s_ltype[GD_MAXLIG];
-  if (*(volatile int *)D.err & kErrPack) return;
-  const int L = cx->lig[0].lig_natom, M = cx->size.mcs_nrow, nlig = cx->size.n_lig;
+  __shared__ int s_perm[GD_MAXLIG], s_ltype[GD_MAXLIG], s_range[kLigTypes];
+  const int L = s.L, M = s.M, nlig = s.nlig, nprt = s.nprt, ntmp = s.ntmp;
   const int ls = (L + 3) & ~3;
-  if (threadIdx.x == 0) dp_ligand_order(cx, L, s_perm, s_ltype);
-  __syncthreads();
-  const int stride = gridDim.x * blockDim.x;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t hp, hl;
+  dp_hdb_types(cx, hp, hl);
+  dp_ligand_order(cx, L, hl, s_perm, s_ltype, s_range);
+  const int stride = nblock * blockDim.x;
+  const int g = block * blockDim.x + threadIdx.x;
   for (int q = g; q < nlig * ls; q += stride) {
     const int i = q / ls, a = q % ls;
     if (a < L) {
-      const int s = s_perm[a];
+      const int k = s_perm[a];
       const Ligand &lg = cx->lig[i];
-      D.lig[q] = make_float4(lg.x2[s], lg.y2[s], lg.z2[s], cx->lig[0].c2[s]);
+      D.lig[q] = make_float4(lg.x2[k], lg.y2[k], lg.z2[k], cx->lig[0].c2[k]);
     } else {
       D.lig[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
   for (int q = g; q < L * M; q += stride) {
     const int a = q / M, m = q % M;
-    const int s = s_perm[a];
-    const float x = cx->mcs[m].x[s];
-    D.mcs[q] = make_float4(x, cx->mcs[m].y[s], cx->mcs[m].z[s], x != GD_MCS_INVALID_COORD ? 1.f : 0.f);
+    const int k = s_perm[a];
+    const float x = cx->mcs[m].x[k];
+    D.mcs[q] = make_float4(x, cx->mcs[m].y[k], cx->mcs[m].z[k], x != GD_MCS_INVALID_COORD ? 1.f : 0.f);
   }
   if (!D.rep) return;
-  const int ntmp = cx->size.n_tmp, nprt = cx->size.n_prt;
   for (int t = g; t < ntmp; t += stride) D.minus_beta[t] = cx->temp[t].minus_beta;
   for (int r = g; r < D.nrep; r += stride) {
     ReplicaMC R = cx->replica[D.rep_begin + r];
@@ -532,18 +517,32 @@ __global__ void dp_ligand_kernel(const Complex *__restrict__ cx, PackDst D)
   }
 }
 
+// The whole packing in one launch: no block needs another's output (each works
+// out the sizes, the hydrogen-bond types and the ligand's order for itself, 720
+// parameters and up to 64 atoms), so nothing waits between them.  What bounds it
+// is the latency of each block's few dependent passes over global memory; as
+// three launches whose orders and checks ran on one thread it took 110 + 70 + 30
+// us for 40 atoms x 1500 points x 11 conformations, now 33 us
+// (as a refill of Dock's state, with replicas and the dense potential, 260 -> 44 us).
+constexpr int kPackLigBlocks = 16;
+__global__ void __launch_bounds__(1024) dp_pack_kernel(const Complex *__restrict__ cx, PackDst D)
+{
+  __shared__ DpSizes s;
+  dp_sizes(cx, D, s);
+  if (!s.ok) return;
+  const int b = blockIdx.x;
+  if (b == 0) dp_setup(cx, D, s);
+  else if (b <= GD_MAX_CONF_PRT) {
+    if (b <= s.nprt) dp_pocket(cx, D, s, b - 1);
+  } else dp_ligand(cx, D, s, b - 1 - GD_MAX_CONF_PRT, kPackLigBlocks);
+}
+
 }  // namespace
 
 cudaError_t device_pack(const Complex *d_cx, const PackDst &D, cudaStream_t st)
 {
   (void)cudaGetLastError();  // a failure an earlier call already reported is not this launch's
-  dp_setup_kernel<<<1, 256, 0, st>>>(d_cx, D);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  dp_pocket_kernel<<<GD_MAX_CONF_PRT, 1024, 0, st>>>(d_cx, D);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  dp_ligand_kernel<<<64, 256, 0, st>>>(d_cx, D);
+  dp_pack_kernel<<<1 + GD_MAX_CONF_PRT + kPackLigBlocks, 1024, 0, st>>>(d_cx, D);
   return cudaGetLastError();
 }
 

@@ -643,8 +643,32 @@ __device__ __forceinline__ WalkTerm<RealOf<PREC>> psp_cell(const int4 *cell, int
   return {(T)hits, (T)__int_as_float(c0.w)};
 }
 
-// The chunks c0, c0 + cstep, ... of 32 cells in turn.
+// The same of a 4-byte cell (pack_cell4), gathered through it.
 template <int PREC>
+__device__ __forceinline__ WalkTerm<RealOf<PREC>> psp_cell4(const DevJob &J, int iprt, const LigOf<PREC> *lig, int k)
+{
+  using T = RealOf<PREC>;
+  const int c = J.pcell4[(size_t)iprt * J.pcell_stride + GD_AT(k, J.pcell_stride, kSitePsp)];
+  const int j = c & 2047, t = (c >> 11) & 31, L = J.natom;
+  const size_t p = (size_t)iprt * J.npoint_pad + j;
+  const float4 q = J.pos[p];
+  const T thr = (T)J.par->tab4[t][__float_as_int(J.aux[p].y)].z;
+  const T nx = -(T)q.x, ny = -(T)q.y, nz = -(T)q.z;
+  const int range = J.trange[t];
+  int hits = 0;
+  for (int a = range & 0xffff; a < range >> 16; ++a) {
+    const V4<T> la = atom_at(lig, GD_AT(a, L, kSiteLig));
+    const T d2 = dist2(add_(la.x, nx), add_(la.y, ny), add_(la.z, nz));
+    T d;
+    if constexpr (PREC == kFP64) d = sqrt(d2);
+    else d = mul_(d2, rsqrt_approx(d2));
+    hits += add_(d, thr) <= (T)0 ? 1 : 0;
+  }
+  return {(T)hits, (T)J.psp_table[t * GD_MAXPRO + (c >> 16)]};
+}
+
+// The chunks c0, c0 + cstep, ... of 32 cells in turn (C4: 4-byte cells).
+template <int PREC, bool C4>
 __device__ __forceinline__ RealOf<PREC> psp_walk(const DevJob &J, int iprt, const LigOf<PREC> *lig, int c0, int cstep)
 {
   using T = RealOf<PREC>;
@@ -652,7 +676,9 @@ __device__ __forceinline__ RealOf<PREC> psp_walk(const DevJob &J, int iprt, cons
   const int n = J.pcell_cnt[iprt], L = J.natom, stride = J.pcell_stride;
   T acc = 0;
   for (int k = 32 * c0 + lane_id(); k < n; k += 32 * cstep) {
-    const WalkTerm<T> t = psp_cell<PREC>(cell, stride, L, lig, k);
+    WalkTerm<T> t;
+    if constexpr (C4) t = psp_cell4<PREC>(J, iprt, lig, k);
+    else t = psp_cell<PREC>(cell, stride, L, lig, k);
     acc = fma_(t.x, t.w, acc);
   }
   return acc;

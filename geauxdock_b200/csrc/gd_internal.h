@@ -129,6 +129,11 @@ struct DevJob {
   const int4 *pcell;
   const int *pcell_cnt;    // [nprt]
   int pcell_stride;        // cells per conformation
+  // the same cells in 4 bytes each (pack_cell4), the values read from the Complex's table, where pcell is null:
+  // the allocation-free entry point's fixed scratch
+  const int *pcell4;
+  const float *psp_table;  // [GD_MAXLIG][GD_MAXPRO]
+  int trange[kLigTypes];   // atoms of each type in the type-grouped ligand, beg | end << 16 (0: none)
   // KDE
   int nkde;
   const float4 *kde;       // [nkde]
@@ -167,6 +172,10 @@ struct DevJob {
   int xsweep;              // exchange sweep run for this job by exchange_jobs_kernel (< 0: none)
   int pad_;
 };
+
+// Cell of pcell4: sorted point, ligand type, column of the potential's table.
+__host__ __device__ inline int pack_cell4(int point, int type, int col) { return point | (type << 11) | (col << 16); }
+static_assert(GD_MAXPRO <= 2048 && kLigTypes <= 32, "pack_cell4's fields");
 
 // One unit of work of the batched kernel: `count` consecutive replicas of
 // one job that share protein conformation `prt`.
@@ -232,6 +241,7 @@ struct KArgs {
   uint8_t group, split;    // TileConfig::group and split, set by launch_kernel.  Fields of one 32-bit word: the
                            // size of this struct changes the kernels' register allocation (measured), so it is kept
   // pose evaluation
+  int n_poses;             // mode 2
   const int *conf;
   const float *mm;
   float *out;
@@ -247,12 +257,11 @@ size_t kernel_smem_bytes(int P, int Pall, int lig_slots, int precision, const Ti
 // Resident CTAs per SM of the batched kernel for this configuration (0 if it cannot launch).
 int kernel_occupancy(int mode, int precision, const TileConfig &tc, size_t smem);
 
-// mode 0: Monte Carlo chunk over the work items; mode 1: pose evaluation.
+// mode 0: Monte Carlo chunk over the work items; mode 1: pose evaluation over
+// work items; mode 2: pose evaluation of jobs[0] without an item list or queue
+// (n_items runs of the CTA's poses, any conformations), for a job packed on the
+// GPU with 4-byte pocket cells.
 cudaError_t launch_kernel(int mode, int precision, const TileConfig &tc, const KArgs &a, int grid, cudaStream_t st);
-
-// Pose evaluation reading the packed job from global memory (8 poses per 256-thread CTA, grid-stride).
-cudaError_t launch_eval_global(int precision, const DevJob *d_job, const int *conf, const float *mm, int n,
-                               float *out, float *raw, int *err, int grid, cudaStream_t st);
 
 // Replica-exchange sweep over all jobs (d_xoff: [2][njob+1] pair-count prefix sums per
 // parity; total: the larger of the two totals).  With d_step, the sweep index is

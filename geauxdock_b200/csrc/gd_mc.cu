@@ -194,7 +194,7 @@ static_assert(sizeof(EnergyScratch) == 192, "EnergyScratch size is part of the s
 // ------------------------------------------------------------- energy --
 // Energy of ligand conformation ilig at pose out->mm in protein conformation
 // iprt, by one warp; writes e[0..9] (normalised terms and total) and raw[0..8].
-template <int PREC, int KPL, int AB>
+template <int PREC, int KPL, int AB, bool C4>
 __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__restrict__ par,
                                          const float4 *__restrict__ pos, const float2 *__restrict__ aux,
                                          const int2 *__restrict__ lgrp, const float4 *__restrict__ apt,
@@ -226,7 +226,7 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
       rs.add(3, r.w);
     }
   }
-  const T s_psp = psp_walk<PREC>(J, iprt, lig, 0, 1);
+  const T s_psp = psp_walk<PREC, C4>(J, iprt, lig, 0, 1);
 
   // pass 2: one lane per atom applies the restraint
   T ehpc = 0;
@@ -266,468 +266,6 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
     out->e[lane] = (double)v;
   }
   if (lane == 9) out->e[9] = (double)tot;
-  __syncwarp();
-}
-
-// ------------------------------------------------ per-type-group form --
-// Running sums of the pair terms of one point row.  The electrostatic term
-// q_a q_p g(d) is summed per point as q_p * sum_a q_a g(d), one sum per point
-// the lane holds, and multiplied by q_p at the end of the row.
-template <typename T, int KPL>
-struct PairAcc {
-  T vdw, pmf, psp, hdb;
-  T ele[KPL];
-};
-
-// Scalar force-field constants of the pair terms, read once per pose.
-struct TypedConst {
-  float lj0, lj1, lj01, el0, el1, inv_el1, a1, b1, ea, eb, ed2;
-  __device__ static TypedConst load(const DevParams *p)
-  {
-    TypedConst c;
-    c.lj0 = p->lj0; c.lj1 = p->lj1; c.lj01 = p->lj01; c.el0 = p->el0; c.el1 = p->el1; c.inv_el1 = p->inv_el1;
-    c.a1 = p->a1; c.b1 = p->b1; c.ea = p->ele_a; c.eb = p->ele_b; c.ed2 = p->ele_d2max;
-    return c;
-  }
-};
-
-// Pair terms of ligand atoms [a, aend) (one type group) against the lane's
-// KPL points, energy_prt_v1.cu:56-139 except the hydrophobic contact.  HDB /
-// PSP: evaluate the hydrogen-bond / pocket-specific terms (some lane has a
-// non-zero parameter).  FP32 uses rearranged forms of the same formulas
-// (t4 = (1/p1a, p2a/p1a, pmf0, pmf1), tab4_entry):
-//   LJ = (1 - (p2a/p1a) d^3) / (lj0 + lj0 lj1 d^2 + d^9 / p1a)   (divided through by p1),
-//   g  = el0 + d^2 (a1 el1^2 + b1 el1^3 d) for el1 d < 1, else r/el1 with r = 1/d,
-//   hdb1 exp(-((d - hdb0) hdb1)^2 / 2) = (hdb1 c) 2^-(d hdb1 c - hdb0 hdb1 c)^2 / c
-// (t2 = (hdb1 c, -hdb0 hdb1 c)).  FP64 evaluates the reference's forms with
-// rf = (p1a, p2a, hdb0, hdb1).
-template <int PREC, int KPL, bool HDB, bool PSP, typename T, typename LA>
-__device__ __forceinline__ void pair_atoms(const LA *lig, int a, int aend, const T (&px)[KPL],
-                                           const T (&py)[KPL], const T (&pz)[KPL], const float4 (&t4)[KPL],
-                                           const float2 (&t2)[KPL], const float4 (&rf)[KPL], const T (&tps)[KPL],
-                                           const TypedConst &c, PairAcc<T, KPL> &acc)
-{
-  if constexpr (PREC == kFP64) {
-    const double lj0 = c.lj0, lj1 = c.lj1, el0 = c.el0, el1 = c.el1, a1 = c.a1, b1 = c.b1;
-    for (; a < aend; ++a) {
-      const V4<double> la = atom_at(lig, a);
-#pragma unroll
-      for (int j = 0; j < KPL; ++j) {
-        const double dx = la.x - px[j], dy = la.y - py[j], dz = la.z - pz[j];
-        const double d2 = dx * dx + dy * dy + dz * dz;
-        const double d4 = d2 * d2;
-        const double d = sqrt(d2);
-        const double p1 = (double)rf[j].x / (d4 * d4 * d);
-        const double p2 = (double)rf[j].y / (d4 * d2);
-        const double p4 = p1 * lj0 * (1.0 + lj1 * d2) + 1.0;
-        acc.vdw += (p1 - p2) / p4;
-        const double s1 = el1 * d;
-        const double g = (s1 < 1.0) ? el0 + a1 * s1 * s1 + b1 * s1 * s1 * s1 : 1.0 / s1;
-        acc.ele[j] += la.w * g;
-        const double dmp = d + (double)t4[j].z;   // t4.z = -pmf0
-        acc.pmf += (double)t4[j].w / (1.0 + exp((-0.5 * d + 6.0) * dmp));
-        if constexpr (PSP) acc.psp += (dmp <= 0.0) ? tps[j] : 0.0;
-        if constexpr (HDB) {
-          const double h3 = (d - (double)rf[j].z) * (double)rf[j].w;
-          acc.hdb += (double)rf[j].w * exp(-0.5 * h3 * h3);
-        }
-      }
-    }
-  } else {
-#pragma unroll 2
-    for (; a < aend; ++a) {
-      const V4<float> la = atom_at(lig, a);
-#pragma unroll
-      for (int j = 0; j < KPL; ++j) {
-        const float dx = la.x - px[j], dy = la.y - py[j], dz = la.z - pz[j];
-        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        const float r = rsqrt_approx(d2);
-        const float d = d2 * r;
-        const float d3 = d2 * d;
-        const float d6 = d3 * d3;
-        const float den = fmaf(d6 * d3, t4[j].x, fmaf(c.lj01, d2, c.lj0));
-        const float num = fmaf(t4[j].y, d3, 1.0f);
-        acc.vdw = fmaf(num, rcp_approx(den), acc.vdw);
-        const float g = (d2 < c.ed2) ? fmaf(d2, fmaf(c.eb, d, c.ea), c.el0) : r * c.inv_el1;
-        acc.ele[j] = fmaf(la.w, g, acc.ele[j]);
-        const float dmp = d + t4[j].z;
-        const float ex = ex2_approx(fmaf(-0.5f * kLog2e, d, 6.0f * kLog2e) * dmp);
-        acc.pmf = fmaf(t4[j].w, rcp_approx(1.0f + ex), acc.pmf);
-        if constexpr (PSP) acc.psp += (dmp <= 0.0f) ? tps[j] : 0.0f;
-        if constexpr (HDB) {
-          const float h = fmaf(d, t2[j].x, t2[j].y);
-          acc.hdb = fmaf(t2[j].x, ex2_approx(-(h * h)), acc.hdb);
-        }
-      }
-    }
-  }
-}
-
-template <int PREC, int KPL, int AB>
-__device__ __noinline__ void energy_typed(const DevJob &J, const DevParams *__restrict__ par,
-                                         const float4 *__restrict__ pos, const float2 *__restrict__ aux,
-                                         const float4 *__restrict__ kde, const int2 *__restrict__ lgrp,
-                                         const float4 *__restrict__ apt, const float4 *__restrict__ aph,
-                                         const int4 *__restrict__ ahd, void *ligbuf, int ilig, int iprt,
-                                         const float *mm, EnergyScratch *out)
-{
-  using T = typename std::conditional<PREC == kFP64, double, float>::type;
-  constexpr int G = 1, my_sub = 0;
-  const int row0 = 32 * KPL * my_sub, rstep = 32 * KPL * G;
-  const int lane = lane_id();
-  const int L = J.natom;
-  const int P = J.npoint_pad;
-  using LA = typename std::conditional<PREC == kFP64, V4<double>, LigPair>::type;
-  LA *lig = reinterpret_cast<LA *>(ligbuf);
-
-  // rotation + translation, kernel_cuda_l1_montecarlo.cu:336-380
-  T r00, r01, r02, r10, r11, r12, r20, r21, r22;
-  {
-    T s1, c1, s2, c2, s3, c3;
-    if constexpr (PREC == kFP64) {
-      sincos((double)mm[3], &s1, &c1);
-      sincos((double)mm[4], &s2, &c2);
-      sincos((double)mm[5], &s3, &c3);
-    } else {
-      sincosf(mm[3], &s1, &c1);
-      sincosf(mm[4], &s2, &c2);
-      sincosf(mm[5], &s3, &c3);
-    }
-    r00 = c1 * c2;
-    r01 = c1 * s2 * s3 - c3 * s1;
-    r02 = s1 * s3 + c1 * c3 * s2;
-    r10 = c2 * s1;
-    r11 = c1 * c3 + s1 * s2 * s3;
-    r12 = c3 * s1 * s2 - c1 * s3;
-    r20 = -s2;
-    r21 = c2 * s3;
-    r22 = c2 * c3;
-  }
-  const float *lc = J.lcenter + 3 * GD_AT(ilig, J.nlig, kSiteLigConf);
-  const T tx = (T)mm[0] + (T)lc[0], ty = (T)mm[1] + (T)lc[1], tz = (T)mm[2] + (T)lc[2];
-  const float4 *lsrc = J.lig + (size_t)ilig * J.lstride;
-  for (int a = lane; a < L; a += 32) {
-    const float4 v = lsrc[a];
-    V4<T> o;
-    o.x = r00 * (T)v.x + r01 * (T)v.y + r02 * (T)v.z + tx;
-    o.y = r10 * (T)v.x + r11 * (T)v.y + r12 * (T)v.z + ty;
-    o.z = r20 * (T)v.x + r21 * (T)v.y + r22 * (T)v.z + tz;
-    o.w = (T)v.w;
-    if constexpr (PREC == kFP64) {
-      lig[a] = o;
-    } else {
-      float *f = reinterpret_cast<float *>(lig + (a >> 1)) + (a & 1);
-      f[0] = o.x;
-      f[2] = o.y;
-      f[4] = o.z;
-      f[6] = o.w;
-    }
-  }
-  if constexpr (PREC != kFP64) {
-    // the dummy half of an odd atom count: far from every point (padding
-    // points sit near +1e4), no charge; its table entries make every term 0
-    if ((L & 1) && lane == 0) {
-      float *f = reinterpret_cast<float *>(lig + (L >> 1)) + 1;
-      f[0] = -1.0e4f;
-      f[2] = -1.0e4f;
-      f[4] = -1.0e4f;
-      f[6] = 0.0f;
-    }
-  }
-  __syncwarp();
-
-  // ---- protein-ligand pair terms, energy_prt_v1.cu:8-174
-  // Pass 1: every term but the hydrophobic contact.  Lane i holds points
-  // row + i + 32 j (j < KPL); atoms are visited one type group at a time, with
-  // the (atom type, point type) table entries loaded once per group.  The
-  // hydrogen-bond and pocket-specific terms are skipped for a group when no
-  // lane of the warp has a non-zero parameter for it (both are sparse).
-  T s_vdw = 0, s_ele = 0, s_pmf = 0, s_psp = 0, s_hdb = 0;
-  // Kahan compensations of the three dense sums (psp and hdb are short, sparse sums)
-  float c_vdw = 0.f, c_ele = 0.f, c_pmf = 0.f;
-  const float *pspc = J.psp + (size_t)iprt * kLigTypes * P;
-  const uint32_t *pmc = J.pspmask + (size_t)iprt * P;
-  const TypedConst kc = TypedConst::load(par);
-
-  {
-    for (int row = row0; row < P; row += rstep) {
-      T px[KPL], py[KPL], pz[KPL], pe[KPL];
-      int pt[KPL];
-      uint32_t pm[KPL];
-      uint32_t ptbits = 0u, pmbits = 0u;
-  #pragma unroll
-      for (int j = 0; j < KPL; ++j) {
-        const int p = GD_AT(row + 32 * j + lane, P, kSitePos);
-        const float4 q = pos[p];
-        px[j] = q.x; py[j] = q.y; pz[j] = q.z; pe[j] = q.w;
-        pt[j] = __float_as_int(aux[p].y);
-        pm[j] = __ldg(pmc + p);
-        ptbits |= 1u << pt[j];
-        pmbits |= pm[j];
-      }
-      // point types present in the row, and ligand types with a pocket-specific
-      // potential on some point of it: decide per type group, for the whole warp,
-      // whether the sparse terms are evaluated
-      ptbits = __reduce_or_sync(0xffffffffu, ptbits);
-      pmbits = __reduce_or_sync(0xffffffffu, pmbits);
-      PairAcc<T, KPL> acc;
-      acc.vdw = acc.pmf = acc.psp = acc.hdb = 0;
-  #pragma unroll
-      for (int j = 0; j < KPL; ++j) acc.ele[j] = 0;
-      int a = 0;
-      while (a < L) {
-        const int2 grp = lgrp[GD_AT(a, L, kSiteLgrp)];
-        const int lt = GD_AT(grp.x, kLigTypes, kSiteTab), aend = grp.y;
-        const bool any_hdb = (par->hdbmask[lt] & ptbits) != 0u;
-        const bool any_psp = ((pmbits >> lt) & 1u) != 0u;
-        float4 t4[KPL], rf[KPL];
-        float2 t2[KPL];
-        T tps[KPL];
-  #pragma unroll
-        for (int j = 0; j < KPL; ++j) {
-          t4[j] = (PREC == kFP64 ? par : J.par)->tab4[lt][pt[j]];  // FP32 stages no tables
-          if constexpr (PREC == kFP64) rf[j] = __ldg(J.ref4 + lt * kTabCols + pt[j]);
-          else rf[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-          t2[j] = make_float2(0.f, 0.f);
-          tps[j] = 0;
-        }
-        if constexpr (PREC != kFP64) {
-          if (any_hdb) {
-  #pragma unroll
-            for (int j = 0; j < KPL; ++j) t2[j] = J.par->tab2[lt][pt[j]];
-          }
-        }
-        if (any_psp) {
-  #pragma unroll
-          for (int j = 0; j < KPL; ++j)
-            if ((pm[j] >> lt) & 1u) tps[j] = __ldg(pspc + GD_AT((size_t)lt * P + row + 32 * j + lane, kLigTypes * P, kSitePsp));
-        }
-        if (any_hdb) {
-          if (any_psp) pair_atoms<PREC, KPL, true, true>(lig, a, aend, px, py, pz, t4, t2, rf, tps, kc, acc);
-          else pair_atoms<PREC, KPL, true, false>(lig, a, aend, px, py, pz, t4, t2, rf, tps, kc, acc);
-        } else {
-          if (any_psp) pair_atoms<PREC, KPL, false, true>(lig, a, aend, px, py, pz, t4, t2, rf, tps, kc, acc);
-          else pair_atoms<PREC, KPL, false, false>(lig, a, aend, px, py, pz, t4, t2, rf, tps, kc, acc);
-        }
-        a = aend;
-      }
-      T row_ele = 0;
-  #pragma unroll
-      for (int j = 0; j < KPL; ++j) row_ele += pe[j] * acc.ele[j];
-      if constexpr (PREC == kFP32Kahan) {
-        kahan_add(s_vdw, c_vdw, acc.vdw);
-        kahan_add(s_ele, c_ele, row_ele);
-        kahan_add(s_pmf, c_pmf, acc.pmf);
-        s_psp += acc.psp;
-        s_hdb += acc.hdb;
-      } else {
-        s_vdw += acc.vdw;
-        s_ele += row_ele;
-        s_pmf += acc.pmf;
-        s_psp += acc.psp;
-        s_hdb += acc.hdb;
-      }
-    }
-  }
-
-  // Pass 2: hydrophobic contact (energy_prt_v1.cu:42-49) over the rows that
-  // hold cdc == 1 points (placed first).  The polynomial
-  // 1 - 3.5x + 4.5x^2 - 2.5x^3 + 0.5x^4 (x = d^2/81) is (1-x)^3 (1-x/2), i.e.
-  // (y^3 + y^4) / 2 with y = 1 - x; clamping y at 0 applies the d^2 <= 81
-  // cut-off.  Per-atom sums stay in
-  // registers for AB atoms at a time, then the per-atom restraint
-  // (energy_prt_v1.cu:162-169).
-  T ehpc = 0;
-  {
-    const int rows = ((J.ncdc[iprt] + 32 * KPL - 1) / (32 * KPL)) * (32 * KPL);
-    for (int a0 = 0; a0 < L; a0 += AB) {
-      T hpc[AB];
-      {
-#pragma unroll
-        for (int k = 0; k < AB; ++k) hpc[k] = 0;
-        for (int row = row0; row < rows; row += rstep) {
-          T px[KPL], py[KPL], pz[KPL], ph[KPL];
-#pragma unroll
-          for (int j = 0; j < KPL; ++j) {
-            const int p = GD_AT(row + 32 * j + lane, P, kSitePos);
-            const float4 q = pos[p];
-            px[j] = q.x; py[j] = q.y; pz[j] = q.z;
-            ph[j] = aux[p].x;
-          }
-#pragma unroll
-          for (int k = 0; k < AB; ++k) {
-            const int a = a0 + k;
-            if (a >= L) break;
-            const V4<T> la = atom_at(lig, a);
-#pragma unroll
-            for (int j = 0; j < KPL; ++j) {
-              const T dx = la.x - px[j], dy = la.y - py[j], dz = la.z - pz[j];
-              const T d2 = dx * dx + dy * dy + dz * dz;
-              T t, u;
-              if constexpr (PREC == kFP64) {
-                t = fmax(1.0 - d2 / 81.0, 0.0);
-                u = 1.0 - 0.5 * d2 / 81.0;
-              } else {
-                t = fmaxf(fmaf(d2, -1.0f / 81.0f, 1.0f), 0.0f);
-                u = fmaf(d2, -0.5f / 81.0f, 1.0f);
-              }
-              hpc[k] += ph[j] * (t * t * t * u);
-            }
-          }
-        }
-      }
-      {
-#pragma unroll
-        for (int k = 0; k < AB; ++k) {
-          const int a = a0 + k;
-          if (a >= L) break;
-          const T S = warp_sum(hpc[k]);
-          const int lt = GD_AT(lgrp[GD_AT(a, L, kSiteLgrp)].x, kLigTypes, kSiteTab);
-          const T h2 = (S - (T)par->hpl0[lt]) / (T)par->hpl1[lt];
-          ehpc += (T)0.5 * h2 * h2 - (T)par->hpl2[lt];
-        }
-      }
-    }
-    // the atom-pair form's restraint terms sit on one lane per atom
-  }
-
-  T vdw, ele, pmf, psp, hdb;
-  if constexpr (PREC == kFP32Kahan) {
-    vdw = warp_sum_comp(s_vdw, c_vdw);
-    ele = warp_sum_comp(s_ele, c_ele);
-    pmf = warp_sum_comp(s_pmf, c_pmf);
-    psp = warp_sum(s_psp);
-    hdb = warp_sum(s_hdb);
-  } else {
-    vdw = warp_sum(s_vdw);
-    ele = warp_sum(s_ele);
-    pmf = warp_sum(s_pmf);
-    psp = warp_sum(s_psp);
-    hdb = warp_sum(s_hdb);
-  }
-  // the FP32 hydrogen-bond sum carries the table's factor c (see DevParams)
-  if constexpr (PREC != kFP64) hdb *= par->hdb_cinv;
-
-  // ---- KDE, energy_kde_v1.cu:183-274: per atom, mean of exp(kde2 d^2) over
-  // the KDE points of the same type; atoms with no such point contribute 0.
-  // The atom-pair form walks the job's slots (below); the per-type-group form:
-  // one type group at a time, lane k holds KDE point k of the group's type and
-  // sums over the group's atoms, then scales by 1 / (points of the type).  A
-  // replica split over G warps deals the slots or the type groups out to its
-  // warps in turn.
-  T kacc = 0;
-  {
-    const T kde2 = par->kde2;
-    int tg = 0;
-    for (int a = 0; a < L; ++tg) {
-      const int2 grp = lgrp[GD_AT(a, L, kSiteLgrp)];
-      const int lt = GD_AT(grp.x, kLigTypes, kSiteTab), aend = grp.y;
-      const int cnt = J.kcnt[lt];
-      if (cnt > 0 && (G == 1 || tg % G == my_sub)) {
-        const int beg = J.kbeg[lt];
-        const T inv = (T)1 / (T)cnt;
-        for (int k = beg + lane; k < beg + cnt; k += 32) {
-          const float4 q = kde[GD_AT(k, J.nkde, kSiteKde)];
-          T s = 0;
-          for (int b = a; b < aend; ++b) {
-            const V4<T> la = atom_at(lig, b);
-            const T dx = la.x - (T)q.x, dy = la.y - (T)q.y, dz = la.z - (T)q.z;
-            const T d2 = dx * dx + dy * dy + dz * dz;
-            if constexpr (PREC == kFP64) s += exp(kde2 * d2);
-            else s += ex2_approx((kde2 * kLog2e) * d2);
-          }
-          kacc += s * inv;
-        }
-      }
-      a = aend;
-    }
-  }
-  T ekde;
-  if constexpr (PREC == kFP64) ekde = warp_sum(kacc) / (double)par->kde3;
-  else ekde = warp_sum(kacc) * par->kde3_inv;
-
-
-  // ---- MCS, energy_mcs_v1.cu:277-320
-  T macc = 0;
-  {
-    const int M = J.nmcs;
-    if (M <= 16) {
-      // two half-warps share each template: lane and lane + 16 take its even and odd atoms
-      const int m = lane & 15, h = lane >> 4;
-      T s = 0;
-      int n = 0;
-      // a replica split over G warps deals the templates out to its warps
-      const bool mine = m < M && (G == 1 || m % G == my_sub);
-      if (mine) {
-        for (int a = h; a < L; a += 2) {
-          const float4 q = J.mcs[GD_AT((size_t)a * M + m, (size_t)L * M, kSiteMcs)];
-          if (q.w != 0.0f) {
-            const V4<T> la = atom_at(lig, a);
-            const T dx = la.x - (T)q.x, dy = la.y - (T)q.y, dz = la.z - (T)q.z;
-            s += dx * dx + dy * dy + dz * dz;
-            ++n;
-          }
-        }
-      }
-      s += __shfl_xor_sync(0xffffffffu, s, 16);
-      n += __shfl_xor_sync(0xffffffffu, n, 16);
-      if (mine && h == 0) macc += (T)J.tcc[GD_AT(m, M, kSiteTcc)] * sqrt(s / (T)n);
-    } else
-    for (int m0 = 32 * my_sub; m0 < M; m0 += 32 * G) {
-      const int m = m0 + lane;
-      if (m < M) {
-        T s = 0;
-        int n = 0;
-        for (int a = 0; a < L; ++a) {
-          const float4 q = J.mcs[GD_AT((size_t)a * M + m, (size_t)L * M, kSiteMcs)];
-          if (q.w != 0.0f) {
-            const V4<T> la = atom_at(lig, a);
-            const T dx = la.x - (T)q.x, dy = la.y - (T)q.y, dz = la.z - (T)q.z;
-            s += dx * dx + dy * dy + dz * dz;
-            ++n;
-          }
-        }
-        macc += (T)J.tcc[GD_AT(m, M, kSiteTcc)] * sqrt(s / (T)n);
-      }
-    }
-  }
-  T elhm = warp_sum(macc);
-
-
-  // ---- distance to the pocket centre, kernel_cuda_l1_montecarlo.cu:439-454
-  const float *pc = J.pcenter + 3 * GD_AT(iprt, J.nprt, kSitePrtConf);
-  T dst = 0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const T t = ((T)lc[i] + (T)mm[i]) - (T)pc[i];
-    dst += t * t;
-  }
-
-  T r9[9];
-  r9[0] = vdw;
-  r9[1] = ele;
-  r9[2] = pmf;
-  r9[3] = psp;
-  r9[4] = hdb * (PREC == kFP64 ? (T)kSqrt2PiInvNegD : (T)kSqrt2PiInvNeg);
-  r9[5] = ehpc;
-  r9[6] = ekde;
-  r9[7] = log(elhm / (T)J.nmcs);
-  r9[8] = sqrt(dst);
-
-  // normalisation and weighted total, kernel_cuda_l1_montecarlo.cu:460-476
-  if (lane == 0) {
-    T tot = 0;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      out->raw[i] = (double)r9[i];
-      T v = r9[i];
-      if (i < 7) v = v / (T)L;
-      v = (T)par->a_para[i] * v + (T)par->b_para[i];
-      out->e[i] = (double)v;
-      tot += (T)par->w[i] * v;
-    }
-    out->e[9] = (double)tot;
-  }
   __syncwarp();
 }
 
@@ -796,8 +334,36 @@ __device__ bool load_item(const KArgs &A, const DevJob &J, const WorkItem &wi, u
     }
     prev_job = wi.job;
     prev_prt = wi.prt;
+    __syncthreads();
   }
+  return true;
+}
+
+// The next work item's index: from the queue, or (mode 2, no item list) the CTA's
+// turn; and the item.  Mode 2 poses of one CTA may have any protein conformation:
+// nothing of a conformation is staged, and after the first turn nothing is shared
+// between a CTA's warps (or teams) that a turn writes.
+template <int MODE>
+__device__ __forceinline__ int next_item(const KArgs &A, int turn, int *s_item)
+{
+  if constexpr (MODE == 2) return blockIdx.x + turn * gridDim.x;
+  if (threadIdx.x == 0) *s_item = atomicAdd(A.queue, 1);
   __syncthreads();
+  return *s_item;
+}
+template <int MODE>
+__device__ __forceinline__ WorkItem work_item(const KArgs &A, int it, int R)
+{
+  if constexpr (MODE == 2) return WorkItem{0, 0, it * R, min(R, A.n_poses - it * R)};
+  return A.items[it];
+}
+
+// Mode 2: a pose whose conformations are out of range gets NaN and the error flag.
+__device__ __forceinline__ bool bad_pose(const KArgs &A, const DevJob &J, int r, int ilig, int iprt, bool tell)
+{
+  if (ilig >= 0 && ilig < J.nlig && iprt >= 0 && iprt < J.nprt) return false;
+  if (tell && lane_id() < 10) A.out[10 * (size_t)r + lane_id()] = __int_as_float(0x7fc00000);
+  if (tell && lane_id() == 0) atomicOr(A.err, kErrSize);
   return true;
 }
 
@@ -860,12 +426,10 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
   uint32_t phase = 0;
   int prev_job = -1, prev_prt = -1;
 
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(A.queue, 1);
-    __syncthreads();
-    const int it = s_item;
+  for (int turn = 0;; ++turn) {
+    const int it = next_item<MODE>(A, turn, &s_item);
     if (it >= A.n_items) break;
-    const WorkItem wi = A.items[it];
+    const WorkItem wi = work_item<MODE>(A, it, blockDim.x >> 5);
     const DevJob &J = A.jobs[wi.job];
     if (!load_item<PREC>(A, J, wi, smem, sl, &bar, phase, prev_job, prev_prt)) return;
     const float4 *apt = reinterpret_cast<const float4 *>(smem + sl.apt);
@@ -887,12 +451,17 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
 
     if (warp < wi.count) {
       const int r = wi.rep0 + warp;  // job-local index
-      if constexpr (MODE == 1) {
+      if constexpr (MODE >= 1) {
         // ---- pose evaluation
         const int ilig = A.conf[2 * r], iprt = A.conf[2 * r + 1];
+        if constexpr (MODE == 2) {
+          if (bad_pose(A, J, r, ilig, iprt, true)) continue;  // no barrier follows in this mode
+          pos = J.pos + (size_t)iprt * J.npoint_pad;
+          aux = J.aux + (size_t)iprt * J.npoint_pad;
+        }
         if (lane < 6) esc->mm[lane] = A.mm[6 * r + lane];
         __syncwarp();
-        energy_warp<PREC, KPL, AB>(J, par, pos, aux, lgrp, apt, aph, ahd, ligbuf, ilig, iprt, esc);
+        energy_warp<PREC, KPL, AB, MODE == 2>(J, par, pos, aux, lgrp, apt, aph, ahd, ligbuf, ilig, iprt, esc);
         if (lane < 10) {
           A.out[10 * (size_t)r + lane] = (float)esc->e[lane];
           if (A.out64) A.out64[10 * (size_t)r + lane] = esc->e[lane];
@@ -949,7 +518,7 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
             esc->mm[lane] = __fmaf_rn(par->move_scale[lane], 0.0f, srep->movematrix[lane]);
           }
           __syncwarp();
-          energy_warp<PREC, KPL, AB>(J, par, pos, aux, lgrp, apt, aph, ahd, ligbuf, ilig, iprt, esc);
+          energy_warp<PREC, KPL, AB, false>(J, par, pos, aux, lgrp, apt, aph, ahd, ligbuf, ilig, iprt, esc);
           const float etot = (float)esc->e[9];
 
           // Metropolis test in FP64, kernel_cuda_l1_montecarlo.cu:485-507
@@ -978,7 +547,7 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
         reinterpret_cast<int *>(J.rep + r)[lane] = sw[lane];
       }
     }
-    __syncthreads();
+    if constexpr (MODE != 2) __syncthreads();
   }
 }
 
@@ -1068,57 +637,6 @@ __global__ void exchange_jobs_kernel(const DevJob *jobs)
 __global__ void advance_step_kernel(int *d_step, int n) { *d_step += n; }
 __global__ void set_step_kernel(int *d_step, int v) { *d_step = v; }
 
-// Pose evaluation that reads the packed job straight from global memory (no
-// shared-memory staging, no work items): warp w of the grid evaluates poses
-// w, w + (number of warps), ...  Used by the allocation-free entry point.
-template <int PREC, int KPL, int AB>
-__global__ void __launch_bounds__(256) eval_global_kernel(const DevJob *jobp, const int *conf, const float *mm,
-                                                          int n, float *out, float *raw, int *err)
-{
-  extern __shared__ __align__(128) unsigned char smem[];
-  if (err != nullptr && *(volatile int *)err != 0) return;  // the job was not packed
-  const DevJob &J = *jobp;
-  const int warp = threadIdx.x >> 5, lane = lane_id();
-  const uint32_t lig_bytes = (uint32_t)kMaxAtoms * 32u;
-  unsigned char *wb = smem + (size_t)warp * (lig_bytes + sizeof(EnergyScratch));
-  EnergyScratch *esc = reinterpret_cast<EnergyScratch *>(wb + lig_bytes);
-  const int nwarps = gridDim.x * (blockDim.x >> 5);
-  for (int i = blockIdx.x * (blockDim.x >> 5) + warp; i < n; i += nwarps) {
-    const int ilig = conf[2 * i], iprt = conf[2 * i + 1];
-    if (ilig < 0 || ilig >= J.nlig || iprt < 0 || iprt >= J.nprt) {
-      if (lane < 10) out[10 * (size_t)i + lane] = __int_as_float(0x7fc00000);
-      if (lane == 0) atomicOr(err, kErrSize);
-      continue;
-    }
-    if (lane < 6) esc->mm[lane] = mm[6 * (size_t)i + lane];
-    __syncwarp();
-    const size_t P = (size_t)J.npoint_pad;
-    // KPL = 1: the per-type-group form, which needs no per-work-item tables
-    energy_typed<PREC, KPL, AB>(J, J.par, J.pos + iprt * P, J.aux + iprt * P, J.kde, J.lgrp, nullptr, nullptr, nullptr,
-                               wb, ilig, iprt, esc->mm, esc);
-    if (lane < 10) out[10 * (size_t)i + lane] = (float)esc->e[lane];
-    if (raw && lane < 9) raw[9 * (size_t)i + lane] = (float)esc->raw[lane];
-    __syncwarp();
-  }
-}
-
-cudaError_t launch_eval_global(int precision, const DevJob *d_job, const int *conf, const float *mm, int n,
-                               float *out, float *raw, int *err, int grid, cudaStream_t st)
-{
-  const int threads = 256;
-  const size_t smem = (size_t)(threads / 32) * ((size_t)kMaxAtoms * 32 + sizeof(EnergyScratch));
-  if (n <= 0) return cudaSuccess;
-  if (precision == kFP32)
-    eval_global_kernel<kFP32, 1, 8><<<grid, threads, smem, st>>>(d_job, conf, mm, n, out, raw, err);
-  else if (precision == kFP32Kahan)
-    eval_global_kernel<kFP32Kahan, 1, 8><<<grid, threads, smem, st>>>(d_job, conf, mm, n, out, raw, err);
-  else if (precision == kFP64)
-    eval_global_kernel<kFP64, 1, 8><<<grid, threads, smem, st>>>(d_job, conf, mm, n, out, raw, err);
-  else
-    return cudaErrorInvalidValue;
-  return cudaGetLastError();
-}
-
 // ---------------------------------------------------------- launchers --
 size_t kernel_smem_bytes(int P, int Pall, int lig_slots, int precision, const TileConfig &tc)
 {
@@ -1136,9 +654,11 @@ static McKernel pick_kernel(const TileConfig &tc)
   if (tc.group > 1) return team_kernel<MODE, PREC, false>;
   if constexpr (PREC == kFP64) return tc.kpl == 1 && tc.ab == 8 ? mc_kernel<MODE, PREC, 1, 8> : nullptr;
   else {
-    if (tc.kpl == 2 && tc.ab == 4) return mc_kernel<MODE, PREC, 2, 4>;
-    if (tc.kpl == 2 && tc.ab == 8) return mc_kernel<MODE, PREC, 2, 8>;
-    if (tc.kpl == 4 && tc.ab == 4) return mc_kernel<MODE, PREC, 4, 4>;
+    if constexpr (MODE != 2) {  // mode 2 has one shape
+      if (tc.kpl == 2 && tc.ab == 4) return mc_kernel<MODE, PREC, 2, 4>;
+      if (tc.kpl == 2 && tc.ab == 8) return mc_kernel<MODE, PREC, 2, 8>;
+      if (tc.kpl == 4 && tc.ab == 4) return mc_kernel<MODE, PREC, 4, 4>;
+    }
     if (tc.kpl == 4 && tc.ab == 8) return mc_kernel<MODE, PREC, 4, 8>;
     return nullptr;
   }
@@ -1150,6 +670,10 @@ static McKernel pick_kernel(int mode, int precision, const TileConfig &tc)
     if (precision == kFP32) return pick_kernel<0, kFP32>(tc);
     if (precision == kFP32Kahan) return pick_kernel<0, kFP32Kahan>(tc);
     if (precision == kFP64) return pick_kernel<0, kFP64>(tc);
+  } else if (mode == 2) {
+    if (precision == kFP32) return pick_kernel<2, kFP32>(tc);
+    if (precision == kFP32Kahan) return pick_kernel<2, kFP32Kahan>(tc);
+    if (precision == kFP64) return pick_kernel<2, kFP64>(tc);
   } else {
     if (precision == kFP32) return pick_kernel<1, kFP32>(tc);
     if (precision == kFP32Kahan) return pick_kernel<1, kFP32Kahan>(tc);

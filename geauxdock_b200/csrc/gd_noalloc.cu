@@ -21,11 +21,17 @@
 // All calls on a device share the array and it keeps the last call's
 // contents, so calls whose GPU work overlaps (different streams, or different
 // host threads) race on it: issue them one after another.
+//
+// The poses run in the batched kernels' mode 2 (gd_mc.cu, gd_team.cuh): no work
+// items or queue, the pair tables built per CTA, the conformations read through
+// L1, and the pocket-specific cells 4 bytes each, which fit where the dense
+// potential was.  4096 poses of 40 atoms x 1500 points x 11 conformations in FP32:
+// the former kernel, one type group of atoms at a time in scalar arithmetic, 991
+// us, now 417 us (bound by the pair loop as the Monte Carlo kernel is); the whole
+// call 1.24 -> 0.45 ms.
 #include <algorithm>
-#include <cstring>
 #include <mutex>
 
-#include "gd_device.cuh"
 #include "gd_pack.h"
 
 namespace gd {
@@ -45,12 +51,12 @@ struct NoAllocScratch {
   float pcenter[GD_MAX_CONF_PRT * 3];
   float tcc[GD_MAX_MCS_ROW];
   float4 lig[GD_MAX_CONF_LIG * GD_MAXLIG];
-  float4 kde[GD_MAXKDE];
+  int4 kslot[2 * GD_MAXKDE];
   float4 mcs[GD_MAXLIG * GD_MAX_MCS_ROW];
   float4 pos[GD_MAX_CONF_PRT * GD_MAXPRO];
   float2 aux[GD_MAX_CONF_PRT * GD_MAXPRO];
-  float psp[GD_MAX_CONF_PRT * kLigTypes * GD_MAXPRO];
-  uint32_t pspmask[GD_MAX_CONF_PRT * GD_MAXPRO];
+  int pcell4[GD_MAX_CONF_PRT * kLigTypes * GD_MAXPRO];
+  int pcell_cnt[GD_MAX_CONF_PRT];
   float4 ref4[kLigTypes * kTabCols];
 };
 
@@ -61,6 +67,51 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoAllocS
 namespace {
 std::mutex g_na_mu;
 void *g_na_ptr[kNaMaxDevices] = {nullptr};
+
+// Launch shape of n poses: chosen for the caps (the sizes are on the GPU), so it
+// depends on the device, the precision and n alone.  The occupancies behind it
+// are looked up once per device and precision.
+struct NaShapes {
+  bool known = false;
+  int nsm = 0;
+  int wave[5][17] = {};  // [log2 warps per pose][poses per CTA]: CTAs one wave holds
+};
+NaShapes g_na_shape[kNaMaxDevices][3];
+
+TileConfig na_tile(int precision, int lg, int R)
+{
+  TileConfig t{R << lg, precision == kFP64 ? 1 : 4, 8, 0, 1 << lg};
+  return t;
+}
+
+int noalloc_shape(int dev, int precision, int n, TileConfig &tc, int &n_items, int &grid)
+{
+  std::lock_guard<std::mutex> lk(g_na_mu);
+  NaShapes &s = g_na_shape[dev][precision];
+  if (!s.known) {
+    GD_CUDA(cudaDeviceGetAttribute(&s.nsm, cudaDevAttrMultiProcessorCount, dev));
+    for (int lg = 0; lg < 5; ++lg)
+      for (int R = 1; R << lg <= kMaxCtaThreads / 32; ++R) {
+        const TileConfig t = na_tile(precision, lg, R);
+        const size_t smem = kernel_smem_bytes(0, GD_MAXPRO, GD_MAXLIG, precision, t);
+        s.wave[lg][R] = smem > kSmemLimit ? 0 : kernel_occupancy(2, precision, t, smem) * s.nsm;
+      }
+    s.known = true;
+  }
+  // as choose_team: the most warps per pose for which one wave holds all, else 8 poses a CTA
+  for (int lg = 4; lg >= 1; --lg)
+    for (int R = 1; R << lg <= kMaxCtaThreads / 32; ++R)
+      if ((n + R - 1) / R <= s.wave[lg][R]) {
+        tc = na_tile(precision, lg, R);
+        grid = n_items = (n + R - 1) / R;
+        return GD_OK;
+      }
+  if (s.wave[0][8] < 1) return fail(GD_E_CUDA, "the pose kernel cannot launch");
+  tc = na_tile(precision, 0, 8);
+  n_items = (n + 7) / 8;
+  grid = std::min(n_items, s.wave[0][8]);
+  return GD_OK;
+}
 
 // The device packer's destination: the scratch array's members.
 PackDst scratch_dst(NoAllocScratch *S)
@@ -75,13 +126,14 @@ PackDst scratch_dst(NoAllocScratch *S)
   D.pcenter = S->pcenter;
   D.tcc = S->tcc;
   D.lig = S->lig;
-  D.kde = S->kde;
+  D.kslot = S->kslot;
   D.mcs = S->mcs;
   D.pos = S->pos;
   D.aux = S->aux;
   D.ncdc = S->ncdc;
-  D.psp = S->psp;
-  D.pspmask = S->pspmask;
+  D.pcell4 = S->pcell4;
+  D.pcell_cnt = S->pcell_cnt;
+  D.pcell_stride = kLigTypes * GD_MAXPRO;
   D.kde_cap = GD_MAXKDE;
   D.Ppad = 0;
   D.nkde_expect = -1;
@@ -123,7 +175,7 @@ extern "C" int gd_eval_poses_noalloc(const Complex *d_complex, int n, const int 
   if (!d_complex || n < 0 || (n > 0 && (!d_conf || !d_mm || !d_out))) return fail(GD_E_INVALID, "null argument");
   if (precision < GD_PREC_FP32 || precision > GD_PREC_FP64) return fail(GD_E_INVALID, "precision = %d", precision);
   cudaStream_t st = (cudaStream_t)stream;
-  int nsm = 0, dev = 0;
+  int dev = 0;
   GD_CUDA(cudaGetDevice(&dev));
   if (st != nullptr) {
     // the scratch address below is the current device's: the stream must belong to it
@@ -135,12 +187,25 @@ extern "C" int gd_eval_poses_noalloc(const Complex *d_complex, int n, const int 
   }
   NoAllocScratch *S = nullptr;
   GD_TRY(noalloc_scratch(&S));
-  GD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  TileConfig tc{8, 4, 8};
+  KArgs a{};
+  int grid = 0;
+  if (n > 0) GD_TRY(noalloc_shape(dev, precision, n, tc, a.n_items, grid));
   // the failure flag and its details must start at zero on every call
   GD_CUDA(cudaMemsetAsync(S->err, 0, sizeof(S->err), st));
   GD_CUDA(device_pack(d_complex, scratch_dst(S), st));
-  const int grid = std::max(1, std::min((n + 7) / 8, nsm * 8));
-  GD_CUDA(launch_eval_global(precision, &S->job, d_conf, d_mm, n, d_out, d_raw, &S->err[0], grid, st));
+  if (n > 0) {
+    a.jobs = &S->job;
+    a.err = &S->err[0];
+    a.Pall = GD_MAXPRO;
+    a.lig_slots = GD_MAXLIG;
+    a.n_poses = n;
+    a.conf = d_conf;
+    a.mm = d_mm;
+    a.out = d_out;
+    a.raw = d_raw;
+    GD_CUDA(launch_kernel(2, precision, tc, a, grid, st));
+  }
   int h[4] = {0, 0, 0, 0};
   GD_CUDA(cudaMemcpyAsync(h, S->err, sizeof(h), cudaMemcpyDeviceToHost, st));
   GD_CUDA(cudaStreamSynchronize(st));

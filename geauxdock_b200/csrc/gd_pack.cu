@@ -677,6 +677,7 @@ int pack_job_impl(const JobData &jd, const DevPocket &pk, const EnePara &ep, boo
   J.pcell = (const int4 *)(b + o_pc);
   J.pcell_cnt = (const int *)(b + o_pcn);
   J.pcell_stride = cstride;
+  for (int t = 0; t < kLigTypes; ++t) J.trange[t] = tbeg[t] | (tend[t] << 16);
   J.nkde = (int)kidx.size();
   J.nkslot = nkslot;
   J.kslot = (const int4 *)(b + o_ks);

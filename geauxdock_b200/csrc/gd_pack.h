@@ -152,8 +152,9 @@ struct PackDst {
   int *ncdc;
   float *psp;
   uint32_t *pspmask;
-  int4 *pcell;         // pocket-specific cells (nullptr: none; only the per-type-group form reads the job)
-  int4 *kslot;         // KDE slots, kde_cap of them (nullptr: none, as pcell)
+  int4 *pcell;         // pocket-specific cells, or
+  int *pcell4;         // the same in 4 bytes each (pcell null)
+  int4 *kslot;         // KDE slots, kde_cap of them
   int *pcell_cnt;
   int pcell_stride;    // cells per conformation the array holds
   int kde_cap;         // KDE points the kde array holds
@@ -172,7 +173,7 @@ struct PackDst {
 enum { kPackFailCapacity = 1, kPackFailInput = 2, kPackFailShape = 3 };
 enum { kFieldNLig = 1, kFieldNPrt, kFieldNatom, kFieldNatomConf, kFieldNpoint, kFieldKde, kFieldMcs, kFieldLigType,
        kFieldPrtType, kFieldSeq3r, kFieldMcsRow, kFieldP1a, kFieldNTmp, kFieldReplica, kFieldPcell };
-// Launches the packer on `st` (setup, pocket, ligand kernels); failures stay in D.err.
+// Launches the packer on `st` (one kernel); failures stay in D.err.  kde, psp and pspmask may be null.
 cudaError_t device_pack(const Complex *d_cx, const PackDst &D, cudaStream_t st);
 const char *pack_field_name(int field);
 

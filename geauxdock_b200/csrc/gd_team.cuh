@@ -80,12 +80,13 @@ __device__ __forceinline__ double to_double(float x)
 }
 
 // Term k of the KDE (which = 0) or pocket-specific walk.
-template <int PREC>
+template <int PREC, bool C4>
 __device__ __forceinline__ WalkTerm<RealOf<PREC>> team_walk_term(const DevJob &J, const DevParams *par,
                                                               const LigOf<PREC> *lig, int which, int iprt, int k)
 {
   if (which == 0) return kde_slot<PREC>(J.kslot, J.nkde, J.natom, kde_exponent<PREC>(par), lig, k);
-  return psp_cell<PREC>(J.pcell + (size_t)iprt * J.pcell_stride * 2, J.pcell_stride, J.natom, lig, k);
+  if constexpr (C4) return psp_cell4<PREC>(J, iprt, lig, k);
+  else return psp_cell<PREC>(J.pcell + (size_t)iprt * J.pcell_stride * 2, J.pcell_stride, J.natom, lig, k);
 }
 
 __device__ __forceinline__ int walk_length(const DevJob &J, int which, int iprt)
@@ -95,7 +96,7 @@ __device__ __forceinline__ int walk_length(const DevJob &J, int which, int iprt)
 
 // Task `task` of `ntask` of a walk: the terms of its chunks or, without chunks,
 // the lanes' sums of the share that is the task.
-template <int PREC>
+template <int PREC, bool C4>
 __device__ __forceinline__ void team_walk(const DevJob &J, const DevParams *par, const TeamArea<PREC> &A,
                                           const LigOf<PREC> *lig, int which, int iprt, int task, int ntask, int chunks)
 {
@@ -106,7 +107,7 @@ __device__ __forceinline__ void team_walk(const DevJob &J, const DevParams *par,
 #pragma unroll 1
   for (int c = task; 32 * c < n && (chunks == 0 || c < chunks); c += ntask) {
     WalkTerm<T> t{0, 0};
-    if (32 * c + lane < n) t = team_walk_term<PREC>(J, par, lig, which, iprt, 32 * c + lane);
+    if (32 * c + lane < n) t = team_walk_term<PREC, C4>(J, par, lig, which, iprt, 32 * c + lane);
     if (chunks) {
       w[64 * c + lane] = t.x;
       w[64 * c + 32 + lane] = t.w;
@@ -141,7 +142,7 @@ __device__ __forceinline__ void kahan_add_any(double &s, float &, double x) { s 
 // lane i < 9 of every warp holds term i, normalised in e and before that in raw,
 // and every lane the total.  What the next call writes before its first barrier
 // nobody reads after this call's second.
-template <int PREC, bool WIDE>
+template <int PREC, bool WIDE, bool C4>
 __device__ __forceinline__ RealOf<PREC> team_energy(const DevJob &J, const ItemData &D, const TeamArea<PREC> &A,
                                                     LigOf<PREC> *lig, int team, int sub, int G, int V, int chunks,
                                                     int ilig, int iprt, float pm, RealOf<PREC> &e, RealOf<PREC> &raw)
@@ -195,7 +196,7 @@ __device__ __forceinline__ RealOf<PREC> team_energy(const DevJob &J, const ItemD
       if ((lane & 3) == 0 && a < L) A.contact[v * kMaxAtoms + a] = S;
     } else {
       const int which = t - t1 > nw;
-      team_walk<PREC>(J, D.par, A, lig, which, iprt, t - t1 - 1 - which * nw, nw, chunks);
+      team_walk<PREC, C4>(J, D.par, A, lig, which, iprt, t - t1 - 1 - which * nw, nw, chunks);
     }
   }
   team_sync(team, G);
@@ -238,7 +239,7 @@ __device__ __forceinline__ RealOf<PREC> team_energy(const DevJob &J, const ItemD
           if (32 * k + lane < n) s = fma_(w[64 * k], w[64 * k + 32], s);
 #pragma unroll 1
         for (int k = 32 * chunks + lane; k < n; k += 32) {  // past the chunks kept
-          const WalkTerm<T> x = team_walk_term<PREC>(J, D.par, lig, i == 3, iprt, k);
+          const WalkTerm<T> x = team_walk_term<PREC, C4>(J, D.par, lig, i == 3, iprt, k);
           s = fma_(x.x, x.w, s);
         }
       }
@@ -308,12 +309,10 @@ __global__ void __maxnreg__(PREC == kFP64 || WIDE ? 128 : 80) team_kernel(KArgs 
   float *draw = reinterpret_cast<float *>(wbase + sl.lig_bytes);
   double *logu = reinterpret_cast<double *>(draw + 8 * kDrawSteps);
 
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(A.queue, 1);
-    __syncthreads();
-    const int it = s_item;
+  for (int turn = 0;; ++turn) {
+    const int it = next_item<MODE>(A, turn, &s_item);
     if (it >= A.n_items) break;
-    const WorkItem wi = A.items[it];
+    const WorkItem wi = work_item<MODE>(A, it, (blockDim.x >> 5) / G);
     const DevJob &J = A.jobs[wi.job];
     if (!load_item<PREC>(A, J, wi, smem, sl, &bar, phase, prev_job, prev_prt)) return;
     ItemData D;
@@ -328,11 +327,16 @@ __global__ void __maxnreg__(PREC == kFP64 || WIDE ? 128 : 80) team_kernel(KArgs 
 
     if (team < wi.count) {
       const int r = wi.rep0 + team;  // job-local index
-      if constexpr (MODE == 1) {
+      if constexpr (MODE >= 1) {
         const int ilig = A.conf[2 * r], iprt = A.conf[2 * r + 1];
+        if constexpr (MODE == 2) {
+          if (bad_pose(A, J, r, ilig, iprt, sub == 0)) continue;  // the team alike; no CTA barrier follows
+          D.pos = J.pos + (size_t)iprt * J.npoint_pad;
+          D.aux = J.aux + (size_t)iprt * J.npoint_pad;
+        }
         const float pm = lane < 6 ? A.mm[6 * r + lane] : 0.0f;
         T et, raw;
-        const T tot = team_energy<PREC, WIDE>(J, D, T_, lig, team, sub, G, V, chunks, ilig, iprt, pm, et, raw);
+        const T tot = team_energy<PREC, WIDE, MODE == 2>(J, D, T_, lig, team, sub, G, V, chunks, ilig, iprt, pm, et, raw);
         if (sub == 0) {
           const double e = (double)(lane < 9 ? et : tot);
           if (lane < 10) {
@@ -394,7 +398,7 @@ __global__ void __maxnreg__(PREC == kFP64 || WIDE ? 128 : 80) team_kernel(KArgs 
           }
           T et, raw;
           const float etot =
-              (float)team_energy<PREC, WIDE>(J, D, T_, lig, team, sub, G, V, chunks, ilig, iprt, pm, et, raw);
+              (float)team_energy<PREC, WIDE, MODE == 2>(J, D, T_, lig, team, sub, G, V, chunks, ilig, iprt, pm, et, raw);
           // Metropolis test in FP64, kernel_cuda_l1_montecarlo.cu:485-507, the same in every warp
           int accept = 1;
           if (!initial) accept = logu[ks] < (to_double(etot) - to_double(ecur)) * mbeta;
@@ -425,7 +429,7 @@ __global__ void __maxnreg__(PREC == kFP64 || WIDE ? 128 : 80) team_kernel(KArgs 
         }
       }
     }
-    __syncthreads();
+    if constexpr (MODE != 2) __syncthreads();
   }
 }
 
