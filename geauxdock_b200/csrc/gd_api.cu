@@ -1086,9 +1086,9 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
     sconf[2 * i + 1] = conf[2 * ord[i] + 1];
     for (int k = 0; k < 6; ++k) smm[6 * i + k] = mm[6 * (size_t)ord[i] + k];
   }
-  // A team of warps per pose where one wave holds the poses, else one warp each, with the
-  // pocket staged in shared memory or read through L1 and the poses per CTA that keep the most
-  // poses in flight (ties: staged, 8 poses).  A 64-atom ligand against 3000 points staged is
+  // A team of warps per pose where one wave holds the poses; else one warp each, spread over the
+  // SMs where one wave holds that (gd_shape.cu); else with the pocket staged in shared memory or read through L1 and the poses
+  // per CTA that keep the most poses in flight (ties: staged, 8 poses).  A 64-atom ligand against 3000 points staged is
   // 136 KB a CTA, so one CTA of 8 warps per SM: 16384 poses 6.26 ms; through L1 three CTAs
   // fit, 24 warps: 3.96 ms (FP64, 2048 poses on 8 and 16 warps: 8.89 and 5.12 ms).
   ShapeQuery q;
@@ -1104,7 +1104,8 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
     return m;
   };
   int grid = 0;
-  if (n > 16 * q.nsm || !choose_team(q, tc, grid)) {  // one wave holds at most 12 teams of two per SM
+  // (one wave holds at most 12 teams of two and 24 warps per SM)
+  if ((n > 16 * q.nsm || !choose_team(q, tc, grid)) && (n > 32 * q.nsm || !choose_spread(q, tc, grid))) {
     long long flight = 0;
     int occ = 0;
     for (const int staged : {1, 0})

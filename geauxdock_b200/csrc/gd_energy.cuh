@@ -115,6 +115,12 @@ struct PairConst {
   }
 };
 
+// The same in FP64, and the exponential's table.
+struct PairConst64 {
+  double lj0, lj01, el0, el1, inv_el1, ea, eb;
+  const double *tab;
+};
+
 // -------------------------------------------- pair loop, FP32 (pass 1) --
 // Protein-ligand pair terms but the hydrophobic contact, energy_prt_v1.cu:56-139.
 //
@@ -393,13 +399,63 @@ struct RowSums {
 };
 
 // ------------------------------------------------------ pair loop, FP64 --
+// Reciprocal and reciprocal square root in FP64: the PTX approximation (about 20
+// bits) and one step of the third-order Newton (Halley) iteration, which cubes its
+// error; measured within 2.3e-16 and 2.7e-16 relative.  x positive, normal and
+// finite, as every argument below is.
+__device__ __forceinline__ double rcp64(double x)
+{
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma_(-x, y, 1.0);
+  return fma_(y, fma_(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt64(double x)
+{
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma_(mul_(-x, y), y, 1.0);
+  return fma_(mul_(y, e), fma_(0.375, e, 0.5), y);
+}
+
+// exp(x) in FP64 after Tang (Table-driven implementation of the exponential
+// function in IEEE floating-point arithmetic, ACM TOMS 15, 1989): x = (32 m + j)
+// ln2/32 + r, |r| <= ln2/64, exp(x) = 2^m 2^(j/32) exp(r), the last from its Taylor
+// series to r^6 (remainder below 4e-18), 2^(j/32) from tab[32].  Measured within
+// 4.0e-16 relative of exp() on [-700, 700].  Beyond it 0 and 2^1000, whose
+// reciprocals act as those of exp() would; NaN stays NaN.
+__device__ __forceinline__ double exp64(double x, const double *tab)
+{
+  const double kMagic = 6755399441055744.0;  // 1.5 2^52: the nearest integer in the low word
+  const double k = fma_(x, 46.16624130844683, kMagic);
+  const int n = __double2loint(k);
+  const double kn = sub_(k, kMagic);
+  const double r = fma_(kn, -7.247021293269686e-19, fma_(kn, -0.02166084939249829, x));
+  double p = fma_(r, 1.0 / 720.0, 1.0 / 120.0);
+  p = fma_(p, r, 1.0 / 24.0);
+  p = fma_(p, r, 1.0 / 6.0);
+  p = fma_(p, r, 0.5);
+  p = fma_(p, r, 1.0);
+  p = fma_(p, r, 1.0);
+  const double v = mul_(p, tab[n & 31]);
+  int hi = __double2hiint(v) + ((n >> 5) << 20), lo = __double2loint(v);
+  const int xh = __double2hiint(x), mag = xh & 0x7fffffff;
+  if (mag > 0x4085e000) {  // |x| > 700, infinite or NaN
+    hi = mag > 0x7ff00000 ? 0x7ff80000 : xh < 0 ? 0 : 0x7e700000;
+    lo = 0;
+  }
+  return __hiloint2double(hi, lo);
+}
+
 // Per work item, the FP64 kernel's (ligand type group, point type) entries in
 // shared memory: pk = (1/p1a, -p2a/p1a), pf = (-pmf0, pmf1, hdb0, hdb1), the
-// hydrogen-bond entries zero where hdb0 <= 0.1.  Padding point types get
-// 1/p1a = +inf, which makes every term exactly 0.
-__device__ __forceinline__ void build_pair_tables64(const DevJob &J, const int2 *lg, double2 *pk, float4 *pf)
+// hydrogen-bond entries zero where hdb0 <= 0.1; and tab = 2^(j/32), j < 32.
+// Padding point types get 1/p1a = 1e200 and 0 else: at their distance (over 1e3)
+// their Lennard-Jones term is below 1e-227, the others exactly 0.
+__device__ __forceinline__ void build_pair_tables64(const DevJob &J, const int2 *lg, double2 *pk, float4 *pf, double *tab)
 {
   const int L = J.natom;
+  for (int j = threadIdx.x; j < 32; j += blockDim.x) tab[j] = exp2((double)j / 32.0);
   int g = 0;
   for (int a = 0; a < L; ++g) {
     const int lt = GD_AT(lg[GD_AT(a, L, kSiteLgrp)].x, kLigTypes, kSiteTab);
@@ -407,8 +463,8 @@ __device__ __forceinline__ void build_pair_tables64(const DevJob &J, const int2 
       const float4 r = J.ref4[lt * kTabCols + pt], t = J.par->tab4[lt][pt];
       const bool real = pt < kPadType;
       pk[g * kTabCols + pt] = real ? make_double2(1.0 / (double)r.x, -(double)r.y / (double)r.x)
-                                   : make_double2((double)INFINITY, 0.0);
-      pf[g * kTabCols + pt] = make_float4(t.z, t.w, r.z, r.w);
+                                   : make_double2(1.0e200, 0.0);
+      pf[g * kTabCols + pt] = real ? make_float4(t.z, t.w, r.z, r.w) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     a = lg[a].y;
   }
@@ -417,34 +473,36 @@ __device__ __forceinline__ void build_pair_tables64(const DevJob &J, const int2 
 // Terms of the atoms [a, aend) of one type against the lane's two points, the
 // reference's formulas with the Lennard-Jones term divided through by p1 (as in
 // FP32), which leaves one reciprocal square root, two reciprocals and one
-// exponential per pair in place of a square root, five divisions and an
-// exponential: 2048 poses of 64 atoms x 3000 points 5.12 -> 2.73 ms.  Bound by
-// the FP64 pipe; two points per lane keep two chains in flight.
+// exponential per pair.  Bound by the FP64 pipe (2.04 cycles a warp operation and
+// scheduler, ~50 a pair): 199 cycles per 32 pairs with CUDA's rsqrt, __drcp_rn and
+// exp, 154 with the Newton steps, 140 with the table-driven exponential too, at 16
+// warps per SM; 2048 poses of 64 atoms x 3000 points 2.73 -> 2.16 ms.  1e-300 keeps
+// d > 0 where a point and an atom coincide.
 template <bool HDB>
 __device__ __forceinline__ void pair_atoms64(const V4<double> *lig, int a, int aend, int L, const double (&px)[2],
                                              const double (&py)[2], const double (&pz)[2], const double2 (&k)[2],
-                                             const float4 (&f)[2], double lj0, double lj01, double el0, double el1,
-                                             double inv_el1, double ea, double eb, double (&vdw)[2], double (&ele)[2],
-                                             double (&pmf)[2], double (&hdb)[2])
+                                             const float4 (&f)[2], const PairConst64 &c, double (&vdw)[2],
+                                             double (&ele)[2], double (&pmf)[2], double (&hdb)[2])
 {
 #pragma unroll 1
   for (; a < aend; ++a) {
     const V4<double> la = lig[GD_AT(a, L, kSiteLig)];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const double d2 = dist2(sub_(la.x, px[j]), sub_(la.y, py[j]), sub_(la.z, pz[j]));
-      const double r = rsqrt(d2);
+      const double dx = sub_(la.x, px[j]), dy = sub_(la.y, py[j]), dz = sub_(la.z, pz[j]);
+      const double d2 = fma_(dx, dx, fma_(dy, dy, fma_(dz, dz, 1.0e-300)));
+      const double r = rsqrt64(d2);
       const double d = mul_(d2, r);
       const double d3 = mul_(d2, d);
-      const double den = fma_(mul_(mul_(d3, d3), d3), k[j].x, fma_(lj01, d2, lj0));
-      vdw[j] = fma_(fma_(k[j].y, d3, 1.0), __drcp_rn(den), vdw[j]);
-      const double g = mul_(el1, d) < 1.0 ? fma_(d2, fma_(eb, d, ea), el0) : mul_(r, inv_el1);
+      const double den = fma_(mul_(mul_(d3, d3), d3), k[j].x, fma_(c.lj01, d2, c.lj0));
+      vdw[j] = fma_(fma_(k[j].y, d3, 1.0), rcp64(den), vdw[j]);
+      const double g = mul_(c.el1, d) < 1.0 ? fma_(d2, fma_(c.eb, d, c.ea), c.el0) : mul_(r, c.inv_el1);
       ele[j] = fma_(la.w, g, ele[j]);
-      const double e1 = add_(1.0, exp(mul_(fma_(-0.5, d, 6.0), add_(d, (double)f[j].x))));
-      pmf[j] = fma_((double)f[j].y, __drcp_rn(e1), pmf[j]);
+      const double e1 = add_(1.0, exp64(mul_(fma_(-0.5, d, 6.0), add_(d, (double)f[j].x)), c.tab));
+      pmf[j] = fma_((double)f[j].y, rcp64(e1), pmf[j]);
       if constexpr (HDB) {
         const double h3 = mul_(sub_(d, (double)f[j].z), (double)f[j].w);
-        hdb[j] = fma_((double)f[j].w, exp(mul_(mul_(-0.5, h3), h3)), hdb[j]);
+        hdb[j] = fma_((double)f[j].w, exp64(mul_(mul_(-0.5, h3), h3), c.tab), hdb[j]);
       }
     }
   }
@@ -452,13 +510,19 @@ __device__ __forceinline__ void pair_atoms64(const V4<double> *lig, int a, int a
 
 // Pass 1 over the 128 points from `row` in FP64, two points per lane at a time.
 __device__ __forceinline__ void pass1_row64(const V4<double> *lig, int L, const int2 *lgrp, const DevParams *par,
-                                            const double2 *pk, const float4 *pf, int row, int P, const float4 *pos,
-                                            const float2 *aux, double (&h)[4])
+                                            const double2 *pk, const float4 *pf, const double *tab, int row, int P,
+                                            const float4 *pos, const float2 *aux, double (&h)[4])
 {
   const int lane = lane_id();
-  const double lj0 = par->lj0, lj01 = mul_((double)par->lj0, (double)par->lj1), el0 = par->el0, el1 = par->el1;
-  const double ea = mul_(mul_((double)par->a1, el1), el1), eb = mul_(mul_(mul_((double)par->b1, el1), el1), el1);
-  const double inv_el1 = __drcp_rn(el1);
+  PairConst64 c;
+  c.lj0 = par->lj0;
+  c.lj01 = mul_(c.lj0, (double)par->lj1);
+  c.el0 = par->el0;
+  c.el1 = par->el1;
+  c.ea = mul_(mul_((double)par->a1, c.el1), c.el1);
+  c.eb = mul_(mul_(mul_((double)par->b1, c.el1), c.el1), c.el1);
+  c.inv_el1 = __drcp_rn(c.el1);
+  c.tab = tab;
   double vdw[2] = {0, 0}, pmf[2] = {0, 0}, hdb[2] = {0, 0}, qe = 0;
 #pragma unroll 1
   for (int sub = 0; sub < kRowPoints; sub += 64) {
@@ -486,9 +550,9 @@ __device__ __forceinline__ void pass1_row64(const V4<double> *lig, int L, const 
         f[j] = pf[g * kTabCols + pt[j]];
       }
       if (par->hdbmask[GD_AT(grp.x, kLigTypes, kSiteTab)] & ptbits)
-        pair_atoms64<true>(lig, a, aend, L, px, py, pz, k, f, lj0, lj01, el0, el1, inv_el1, ea, eb, vdw, ele, pmf, hdb);
+        pair_atoms64<true>(lig, a, aend, L, px, py, pz, k, f, c, vdw, ele, pmf, hdb);
       else
-        pair_atoms64<false>(lig, a, aend, L, px, py, pz, k, f, lj0, lj01, el0, el1, inv_el1, ea, eb, vdw, ele, pmf, hdb);
+        pair_atoms64<false>(lig, a, aend, L, px, py, pz, k, f, c, vdw, ele, pmf, hdb);
       a = aend;
     }
     qe = fma_(pe[1], ele[1], fma_(pe[0], ele[0], qe));

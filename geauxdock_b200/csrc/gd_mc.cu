@@ -151,7 +151,8 @@ __host__ __device__ inline SmemLayout smem_layout(int P, int Pall, int lig_slots
   off = align16(off + 16u * (uint32_t)P);
   s.aux = off;
   off = align16(off + 8u * (uint32_t)P);
-  // FP32: per (atom pair, point type) tables of the atom-pair pair loop; FP64: per (type group, point type)
+  // FP32: per (atom pair, point type) tables of the atom-pair pair loop and a header per pair; FP64: per (type group,
+  // point type), and the exponential's table in the place of the headers
   const uint32_t npairs = (uint32_t)(lig_slots + 1) / 2u;
   const uint32_t entries = (uint32_t)kTabCols * (fp64 ? (uint32_t)(lig_slots < kLigTypes ? lig_slots : kLigTypes) : npairs);
   s.apt = off;
@@ -159,7 +160,7 @@ __host__ __device__ inline SmemLayout smem_layout(int P, int Pall, int lig_slots
   s.aph = off;
   off = align16(off + 16u * entries);
   s.ahd = off;
-  if (!fp64) off = align16(off + 16u * npairs);
+  off = align16(off + (fp64 ? 8u * 32u : 16u * npairs));
   s.lig_bytes = (uint32_t)lig_slots * (fp64 ? 32u : 16u);  // V4<double> per atom, or LigPair per two atoms
   // per replica: ReplicaMC state, EnergyScratch (192 B), WarpStats (64 B); per warp the rotated ligand
   const uint32_t state = (uint32_t)sizeof(ReplicaMC) + 192u + 64u;
@@ -212,7 +213,8 @@ __device__ __noinline__ void energy_warp(const DevJob &J, const DevParams *__res
   if constexpr (PREC == kFP64) {
     for (int row = 0; row < P; row += kRowPoints) {
       double h[4];
-      pass1_row64(lig, L, lgrp, par, reinterpret_cast<const double2 *>(apt), aph, row, P, pos, aux, h);
+      pass1_row64(lig, L, lgrp, par, reinterpret_cast<const double2 *>(apt), aph, reinterpret_cast<const double *>(ahd), row,
+                  P, pos, aux, h);
 #pragma unroll
       for (int t = 0; t < 4; ++t) rs.add(t, h[t]);
     }
@@ -327,7 +329,8 @@ __device__ bool load_item(const KArgs &A, const DevJob &J, const WorkItem &wi, u
     if (wi.job != prev_job) {
       const int2 *lg = reinterpret_cast<const int2 *>(smem + sl.lgrp);
       if constexpr (PREC == kFP64)
-        build_pair_tables64(J, lg, reinterpret_cast<double2 *>(smem + sl.apt), reinterpret_cast<float4 *>(smem + sl.aph));
+        build_pair_tables64(J, lg, reinterpret_cast<double2 *>(smem + sl.apt), reinterpret_cast<float4 *>(smem + sl.aph),
+                            reinterpret_cast<double *>(smem + sl.ahd));
       else
         build_pair_tables(J.natom, J.par, lg, reinterpret_cast<float4 *>(smem + sl.apt),
                           reinterpret_cast<float4 *>(smem + sl.aph), reinterpret_cast<int4 *>(smem + sl.ahd));

@@ -159,7 +159,8 @@ __device__ __forceinline__ RealOf<PREC> team_energy(const DevJob &J, const ItemD
     if constexpr (PREC == kFP64) {
       T *o = A.rows + 128 * t + lane;
       double h[4];
-      pass1_row64(lig, L, D.lgrp, D.par, reinterpret_cast<const double2 *>(D.apt), D.aph, t * row, P, D.pos, D.aux, h);
+      pass1_row64(lig, L, D.lgrp, D.par, reinterpret_cast<const double2 *>(D.apt), D.aph,
+                  reinterpret_cast<const double *>(D.ahd), t * row, P, D.pos, D.aux, h);
 #pragma unroll
       for (int k = 0; k < 4; ++k) o[32 * k] = h[k];
     } else {
