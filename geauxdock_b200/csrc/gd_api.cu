@@ -1482,6 +1482,7 @@ int gd_ensemble_autotune(gd_ensemble_t *e, int steps, char *report, int report_l
   const int shapes[][2] = {{1, 8}, {2, 4}, {2, 8}, {4, 4}, {4, 8}};
   const int warps[] = {4, 6, 8, 10, 12, 14, 16};
   const int group = e->tc.group;  // kept
+  const int cluster = e->tc.cluster;  // kept by the candidates of one replica per CTA
   const TileConfig smallest{std::max(4, group), e->tc.kpl, e->tc.ab, 1, group, e->tc.split};
   const bool can_stage = smem_for(e, smallest) <= kSmemLimit;
   cudaEvent_t a, b;
@@ -1496,7 +1497,7 @@ int gd_ensemble_autotune(gd_ensemble_t *e, int steps, char *report, int report_l
       if (rc != GD_OK) break;
       // the warps per replica are kept; the candidates are the multiples of it
       if (w % group) continue;
-      TileConfig tc{w, sh[0], sh[1], stage, group, e->tc.split};
+      TileConfig tc{w, sh[0], sh[1], stage, group, e->tc.split, w == group ? cluster : 1};
       if (configure(e, tc) != GD_OK || e->tc.stage != stage) continue;
       // a strided sample of the work items (heaviest-first order kept), about two
       // waves of the grid, so that a candidate runs the full chunk length

@@ -171,8 +171,7 @@ __device__ __forceinline__ void mbar_complete_tx(uint64_t *bar, uint32_t bytes)
 // combines it with __syncthreads_and.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64_t limit_ns)
 {
-  const uint64_t t0 = global_ns();
-  for (;;) {
+  for (uint64_t t0 = 0;;) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -182,7 +181,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64
         : "r"(smem_addr(bar)), "r"(parity)
         : "memory");
     if (done) return true;
-    if (global_ns() - t0 > limit_ns) return false;
+    const uint64_t t = global_ns();
+    if (t0 == 0) t0 = t;
+    else if (t - t0 > limit_ns) return false;
   }
 }
 

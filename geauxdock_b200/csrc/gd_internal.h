@@ -187,6 +187,8 @@ struct WorkItem {
 };
 
 // Kernel configuration chosen by the autotuner.
+constexpr int kMaxCluster = 16;  // CTAs of a cluster (above 8 not portable between GPUs; this one takes 16)
+
 struct TileConfig {
   int warps_per_cta;   // replicas per CTA (one warp each)
   int kpl;             // pocket points per lane per row (2 or 4; FP64: 1, its only shape)
@@ -196,6 +198,8 @@ struct TileConfig {
   int split = 1;       // order the sums are combined in: 1 the one-warp kernel's, 2, 4 or 8 the order of a replica
                        // split over that many warps (option replica_warps; group > 1); whatever the group, a
                        // replica's results depend on this alone
+  int cluster = 1;     // more than one (Monte Carlo, one team of 8 or 16 warps per CTA): CTAs of a cluster, which share a
+                       // replica's chunk (gd_spec.cuh)
 };
 
 // Pair-tile shape where the caller leaves it to the library (option value 0).
@@ -256,6 +260,9 @@ size_t kernel_smem_bytes(int P, int Pall, int lig_slots, int precision, const Ti
 
 // Resident CTAs per SM of the batched kernel for this configuration (0 if it cannot launch).
 int kernel_occupancy(int mode, int precision, const TileConfig &tc, size_t smem);
+
+// Clusters of the shape (tc.cluster CTAs each) that the GPU holds at once (0 if it cannot launch).
+int cluster_occupancy(int precision, const TileConfig &tc, size_t smem);
 
 // mode 0: Monte Carlo chunk over the work items; mode 1: pose evaluation over
 // work items; mode 2: pose evaluation of jobs[0] without an item list or queue

@@ -172,7 +172,7 @@ __host__ __device__ inline SmemLayout smem_layout(int P, int Pall, int lig_slots
     // walks' terms (chunks) or sums per lane
     const uint32_t real = fp64 ? 8u : 4u, V = (uint32_t)split;
     const uint32_t walk = 64u * (V > 1 ? 0u : (uint32_t)team_chunks(group)) + 32u * V;
-    s.parts = (uint32_t)sizeof(ReplicaMC) + 64u + real * 72u;
+    s.parts = (uint32_t)sizeof(ReplicaMC) + 64u + real * 84u;
     s.team_bytes = align16(s.parts + real * ((uint32_t)team_row_reals(group, split, fp64) * (uint32_t)(Pall / team_row(split)) + V * (uint32_t)kMaxAtoms + 2u * walk));
     off += s.team_bytes * (uint32_t)(warps / group);
   }
@@ -557,6 +557,7 @@ __global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
 }  // namespace gd
 
 #include "gd_team.cuh"
+#include "gd_spec.cuh"
 
 namespace gd {
 
@@ -685,16 +686,64 @@ static McKernel pick_kernel(int mode, int precision, const TileConfig &tc)
   return nullptr;
 }
 
+// The kernel of a chunk on clusters (gd_spec.cuh); teams of 8 and 16 warps only.
+static McKernel pick_spec(int precision)
+{
+  if (precision == kFP32) return spec_kernel<kFP32, true>;
+  if (precision == kFP32Kahan) return spec_kernel<kFP32Kahan, true>;
+  if (precision == kFP64) return spec_kernel<kFP64, false>;
+  return nullptr;
+}
+
+struct SpecLaunch {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  cudaError_t prepare(McKernel k, const TileConfig &tc, int items, size_t smem, cudaStream_t st)
+  {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = tc.cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(items * tc.cluster));
+    cfg.blockDim = dim3((unsigned)(tc.warps_per_cta * 32));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess || tc.cluster <= 8) return e;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }
+};
+
+int cluster_occupancy(int precision, const TileConfig &tc, size_t smem)
+{
+  const McKernel f = pick_spec(precision);
+  SpecLaunch l;
+  int n = 0;
+  if (!f || l.prepare(f, tc, 1, smem, nullptr) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, (const void *)f, &l.cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 cudaError_t launch_kernel(int mode, int precision, const TileConfig &tc, const KArgs &a, int grid, cudaStream_t st)
 {
-  const McKernel k = pick_kernel(mode, precision, tc);
+  const bool spec = mode == 0 && tc.cluster > 1 && a.nsteps > 1 && !(a.flags & kMcInitial);
+  const McKernel k = spec ? pick_spec(precision) : pick_kernel(mode, precision, tc);
   if (!k) return cudaErrorInvalidValue;
   const size_t smem = kernel_smem_bytes(a.P, a.Pall, a.lig_slots, precision, tc);
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   KArgs b = a;
   b.group = (uint8_t)tc.group;
   b.split = (uint8_t)tc.split;
+  if (spec) {
+    SpecLaunch l;
+    const cudaError_t e = l.prepare(k, tc, a.n_items, smem, st);
+    return e != cudaSuccess ? e : cudaLaunchKernelEx(&l.cfg, k, b);
+  }
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
   k<<<grid, tc.warps_per_cta * 32, smem, st>>>(b);
   return cudaGetLastError();
 }

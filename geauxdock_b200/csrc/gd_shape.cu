@@ -5,6 +5,26 @@
 
 namespace gd {
 
+// SMs that no replica's team needs evaluate the steps that may follow
+// (gd_spec.cuh): the largest cluster for which one wave holds a cluster per
+// replica.  Measured on clusters of 1, 2, 4, 8 and 16: 400 steps of one replica of
+// 24 atoms x 600 points on 8 warps' sums 3.41 / 2.34 / 1.65 / 1.27 / 1.01 ms,
+// a Dock call of 200 steps 1.65 / 1.16 / 0.85 / 0.67 / 0.61 ms, of 51 replicas x
+// 100 steps (34 x 344) 1.01 / 0.79 ms; sizes between lie between (10: 1.17 and
+// 0.67 ms).  Two teams of 8 warps in a CTA, for twice the nodes, are slower at
+// every size (16 nodes on 8 SMs: 1.52 and 0.81 ms).
+static void choose_cluster(const ShapeQuery &q, TileConfig &tc, long long items)
+{
+  if (q.mode != 0 || tc.group < 8 || tc.warps_per_cta != tc.group) return;
+  TileConfig t = tc;
+  t.cluster = (int)std::min<long long>(kMaxCluster, q.nsm / std::max(1LL, items));
+  for (; t.cluster > 1; --t.cluster)
+    if (items <= cluster_occupancy(q.precision, t, q.smem(t))) {
+      tc = t;
+      return;
+    }
+}
+
 // A team is the best use of a warp that no replica needs.  Measured per step of
 // an ensemble of n replicas (40 atoms x 1500 points) on 1, 2, 4, 8 and 16 warps
 // each, where one wave holds the teams: n = 48 128 / 77 / 44 / 22 / 19 us;
@@ -29,6 +49,7 @@ bool choose_team(const ShapeQuery &q, TileConfig &tc, int &grid)
       const long long items = q.items(R), wave = (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm;
       if (items > wave) continue;
       tc = t;
+      choose_cluster(q, tc, items);
       grid = (int)std::max(1LL, items);
       return true;
     }

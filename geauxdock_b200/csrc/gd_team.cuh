@@ -21,10 +21,13 @@
 // A step of 24 atoms x 600 points takes 7.1 us on 16 warps (one warp 36 us, the
 // former split over 8 warps 17 us), of 34 x 344 over 51 replicas 7.5 us (42 us).
 // It is bound by one SM's special-function and issue rate for the rows (~9,300
-// of 14,300 cycles, ten half rows on four schedulers) and by the two barriers'
-// serial parts (combining ~2,300, rotation 850, finishing 1,200).  FP32 <-> FP64
+// of 13,900 cycles, ten half rows on four schedulers) and by the two barriers'
+// serial parts (combining ~2,300, rotation 1,000, finishing 500).  FP32 <-> FP64
 // conversions are kept out of the step's common path: every warp finishing the
-// terms through doubles cost 2,500 cycles.
+// terms through doubles cost 2,500 cycles.  In the split order of 8 the 49 sums of
+// shares go up to four to a warp through one butterfly (one after the other 1,000
+// cycles a step more), and the warp with the templates sits out the first turns of
+// the other tasks (3,000 less where the templates end last).
 #pragma once
 
 #include "gd_energy.cuh"
@@ -53,7 +56,8 @@ struct TeamArea {
   using T = RealOf<PREC>;
   ReplicaMC *rep;
   WarpStats *stats;
-  T *part;     // [9][8] the terms: scaled sums of 0..6 and the MCS sums (V = 1: the term) per share, the distance term
+  T *part;     // [9][8] the terms: the scaled sum of each share, or (V = 1, and the distance) the term as it is and normalised
+  T *mcs;      // MCS sums of the shares, and in [8] the squared distance of the centres
   T *rows;     // pass 1 per lane: [rows][4][32] vdw, ele, pmf, hdb, or [rows][2][7][32] the components (HalfRow)
   T *contact;  // [V][kMaxAtoms] hydrophobic-contact sums
   T *walk[2];  // KDE, pocket-specific: [chunks][32][2] terms, then [V][32] sums
@@ -62,6 +66,7 @@ struct TeamArea {
     rep = reinterpret_cast<ReplicaMC *>(base);
     stats = reinterpret_cast<WarpStats *>(base + sizeof(ReplicaMC));
     part = reinterpret_cast<T *>(base + sizeof(ReplicaMC) + sizeof(WarpStats));
+    mcs = part + 72;
     rows = reinterpret_cast<T *>(base + sl.parts);
     contact = rows + row_reals * nrows;
     walk[0] = contact + V * kMaxAtoms;
@@ -137,12 +142,48 @@ __device__ __forceinline__ void team_half_sums(const LigPair *lig, int npairs, i
 __device__ __forceinline__ void kahan_add_any(float &s, float &c, float x) { kahan_add(s, c, x); }
 __device__ __forceinline__ void kahan_add_any(double &s, float &, double x) { s = add_(s, x); }
 
+// Task t of combining a team's units: share v of term i (the contact, 5, has one).
+__device__ __forceinline__ void team_task(int t, int V, int &i, int &v)
+{
+  const int q = t >> (31 - __clz(V));  // V is a power of two
+  i = t == 6 * V ? 5 : q == 5 ? 6 : q;
+  v = t == 6 * V ? 0 : t - q * V;
+}
+
+// A finished term: as it is, and normalised.
+template <int PREC>
+__device__ __forceinline__ void team_term(RealOf<PREC> *part, int i, RealOf<PREC> raw, const DevParams *par, int L)
+{
+  part[8 * i] = raw;
+  part[8 * i + 1] = norm_term(i, raw, par, L);
+}
+
+// A level of two butterflies at once: a lane whose bit o is clear goes on with the
+// first pair (s0, c0), the others with the second, in (s0, c0); with the same
+// pair twice, a level of warp_sum_pair (FP64: warp_sum).
+__device__ __forceinline__ void sum_merge(float &s0, float &c0, float s1, float c1, int o)
+{
+  const bool hi = (lane_id() & o) != 0;
+  const float s = hi ? s1 : s0, c = hi ? c1 : c0;
+  const float so = __shfl_xor_sync(0xffffffffu, hi ? s0 : s1, o), co = __shfl_xor_sync(0xffffffffu, hi ? c0 : c1, o);
+  const float t = add_(s, so), bp = sub_(t, s);
+  c0 = add_(add_(c, co), add_(sub_(s, sub_(t, bp)), sub_(so, bp)));
+  s0 = t;
+}
+__device__ __forceinline__ void sum_merge(double &s0, float &, double s1, float, int o)
+{
+  const bool hi = (lane_id() & o) != 0;
+  const double s = hi ? s1 : s0;
+  s0 = add_(s, __shfl_xor_sync(0xffffffffu, hi ? s0 : s1, o));
+}
+
 // Energy of ligand conformation ilig at the pose in pm (lane k < 6 holds
 // movematrix[k]) in protein conformation iprt by the team's warps: on return
 // lane i < 9 of every warp holds term i, normalised in e and before that in raw,
-// and every lane the total.  What the next call writes before its first barrier
-// nobody reads after this call's second.
-template <int PREC, bool WIDE, bool C4>
+// and every lane the total (SOLO: of the first warp alone; the finishing of 16
+// warps costs them each other's issue slots).  What the next call writes before
+// its first barrier nobody but the first warp reads after this call's second.
+template <int PREC, bool WIDE, bool C4, bool SOLO = false>
 __device__ __forceinline__ RealOf<PREC> team_energy(const DevJob &J, const ItemData &D, const TeamArea<PREC> &A,
                                                     LigOf<PREC> *lig, int team, int sub, int G, int V, int chunks,
                                                     int ilig, int iprt, float pm, RealOf<PREC> &e, RealOf<PREC> &raw)
@@ -182,14 +223,18 @@ __device__ __forceinline__ RealOf<PREC> team_energy(const DevJob &J, const ItemD
   const int nb = (L + kContactBlock - 1) / kContactBlock;
   const int crows = contact_rows(J, iprt), nv = min(V, max(1, crows / kHalfPoints));  // shares with a contact row
   const int nw = chunks ? 4 : V;  // tasks of a walk
-  const int t1 = nb * nv, t2 = t1 + 2 * nw, busy = nrt % G;
-  for (int t = sub >= busy ? sub - busy : t2 + 1; t <= t2; t += G - busy) {
+  // task 0 takes as long as four or five of the others, so its warp sits out the first four turns of those
+  const int t1 = nb * nv, t2 = t1 + 2 * nw, busy = nrt % G, W = G - busy, x = sub - busy;
+  for (int turn = 0, next = 1; x >= 0 && next <= t2; ++turn) {
+    const int first = turn < 4 ? 1 : 0, t = turn == 0 && x == 0 ? 0 : x < first ? t2 + 1 : next + x - first;
+    next += W - first;
+    if (t > t2) continue;
     if (t == 0) {
       // the longest of them
-      const T m = mcs_sums<PREC>(J, lig, V, A.part + 8 * 7), dst = centre_dist2<T>(J, ilig, iprt, pm);
+      const T m = mcs_sums<PREC>(J, lig, V, A.mcs), dst = centre_dist2<T>(J, ilig, iprt, pm);
       if (lane == 0) {
-        if (V == 1) A.part[8 * 7] = raw_term<PREC>(7, m, J.nmcs);
-        A.part[8 * 8] = raw_term<PREC>(8, dst, J.nmcs);
+        if (V == 1) A.mcs[0] = m;
+        A.mcs[8] = dst;
       }
     } else if (t <= t1) {
       const int v = (t - 1) / nb, a0 = kContactBlock * (t - 1 - v * nb), a = a0 + (lane >> 2);
@@ -202,89 +247,197 @@ __device__ __forceinline__ RealOf<PREC> team_energy(const DevJob &J, const ItemD
   }
   team_sync(team, G);
 
-  // terms 0..6 from their units: per share of V the lanes' sums (the rows' with the
-  // compensation c) and one butterfly, dealt out to the warps
+  // terms 0..6 from their units, dealt out to the warps: per share of V the lanes' sums (the rows' with the
+  // compensation c) and a butterfly, up to four of a warp's in one
+  for (int t0 = sub; t0 < 6 * V + 1; t0 += 4 * G) {
+    T s4[4] = {0, 0, 0, 0};
+    float c4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-  for (int t = sub; t < 6 * V + 1; t += G) {
-    const int q = t / V, i = t == 6 * V ? 5 : q == 5 ? 6 : q, v = t == 6 * V ? 0 : t - q * V;
-    const bool comp = PREC == kFP32Kahan && i < 3;  // the dense terms are compensated
-    T s = 0;
-    float c = 0.f;
-    if (i < 5 && i != 3) {
-      // the rows' sums; the two components of a row joined as pass1_row does
-      const T *u = A.rows + (halves ? 32 * (i == 1 ? 3 : i >> 1) : 32 * (i == 4 ? 3 : i)) + lane;
+    for (int q = 0; q < 4 && t0 + q * G < 6 * V + 1; ++q) {
+      int i, v;
+      team_task(t0 + q * G, V, i, v);
+      T s = 0;
+      float c = 0.f;
+      if (i < 5 && i != 3) {
+        // the rows' sums; the two components of a row joined as pass1_row does
+        const T *u = A.rows + (halves ? 32 * (i == 1 ? 3 : i >> 1) : 32 * (i == 4 ? 3 : i)) + lane;
 #pragma unroll 2
-      for (int r = v; r < nr; r += V) {
-        T h;
-        if (!halves) {
-          h = u[128 * r];
-        } else if (i != 1) {
-          h = add_(u[448 * r], u[448 * r + 224]);
-        } else {
-          h = 0;
+        for (int r = v; r < nr; r += V) {
+          T h;
+          if (!halves) {
+            h = u[128 * r];
+          } else if (i != 1) {
+            h = add_(u[448 * r], u[448 * r + 224]);
+          } else {
+            h = 0;
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            h = fma_((T)D.pos[r * row + 32 * j + lane].w, add_(u[448 * r + 32 * j], u[448 * r + 224 + 32 * j]), h);
+            for (int j = 0; j < 4; ++j)
+              h = fma_((T)D.pos[r * row + 32 * j + lane].w, add_(u[448 * r + 32 * j], u[448 * r + 224 + 32 * j]), h);
+          }
+          // a plain sum is the compensated one without c
+          kahan_add_any(s, c, h);
         }
-        // a plain sum is the compensated one without c
-        kahan_add_any(s, c, h);
-      }
-    } else if (i != 5) {
-      const T *w = A.walk[i == 3] + lane;
-      if (chunks == 0) {
-        s = w[32 * v];
-      } else {
-        const int n = walk_length(J, i == 3, iprt);
+      } else if (i != 5) {
+        const T *w = A.walk[i == 3] + lane;
+        if (chunks == 0) {
+          s = w[32 * v];
+        } else {
+          const int n = walk_length(J, i == 3, iprt);
 #pragma unroll 2
-        for (int k = 0; k < chunks && 32 * k < n; ++k)
-          if (32 * k + lane < n) s = fma_(w[64 * k], w[64 * k + 32], s);
+          for (int k = 0; k < chunks && 32 * k < n; ++k)
+            if (32 * k + lane < n) s = fma_(w[64 * k], w[64 * k + 32], s);
 #pragma unroll 1
-        for (int k = 32 * chunks + lane; k < n; k += 32) {  // past the chunks kept
-          const WalkTerm<T> x = team_walk_term<PREC, C4>(J, D.par, lig, i == 3, iprt, k);
-          s = fma_(x.x, x.w, s);
+          for (int k = 32 * chunks + lane; k < n; k += 32) {  // past the chunks kept
+            const WalkTerm<T> x = team_walk_term<PREC, C4>(J, D.par, lig, i == 3, iprt, k);
+            s = fma_(x.x, x.w, s);
+          }
         }
+      } else {
+        // a lane's atoms and their order: those of the one-warp kernel's blocks, or one lane per atom
+        const bool blocks = V == 1;
+        if (!blocks || (lane & 3) == 0)
+#pragma unroll 1
+          for (int a = blocks ? lane >> 2 : lane; a < L; a += blocks ? kContactBlock : 32) {
+            T S = A.contact[a];
+            for (int k = 1; k < nv; ++k) S = add_(S, A.contact[k * kMaxAtoms + a]);
+            s = add_(s, contact_restraint(D.par, D.lgrp, a, L, S));
+          }
       }
-    } else {
-      // a lane's atoms and their order: those of the one-warp kernel's blocks, or one lane per atom
-      const bool blocks = V == 1;
-      if (!blocks || (lane & 3) == 0)
-#pragma unroll 1
-        for (int a = blocks ? lane >> 2 : lane; a < L; a += blocks ? kContactBlock : 32) {
-          T S = A.contact[a];
-          for (int k = 1; k < nv; ++k) S = add_(S, A.contact[k * kMaxAtoms + a]);
-          s = add_(s, contact_restraint(D.par, D.lgrp, a, L, S));
-        }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        s4[k] = q == k ? s : s4[k];
+        c4[k] = q == k ? c : c4[k];
+      }
     }
-    if constexpr (PREC == kFP32Kahan) {
-      warp_sum_pair(s, c);
-      if (comp) s = add_(s, c);
-    } else {
-      s = warp_sum(s);
+    sum_merge(s4[0], c4[0], s4[1], c4[1], 16);
+    sum_merge(s4[2], c4[2], s4[3], c4[3], 16);
+    sum_merge(s4[0], c4[0], s4[2], c4[2], 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) sum_merge(s4[0], c4[0], s4[0], c4[0], o);
+    const int t = t0 + (2 * ((lane >> 3) & 1) + (lane >> 4)) * G;
+    if ((lane & 7) == 0 && t < 6 * V + 1) {
+      int i, v;
+      team_task(t, V, i, v);
+      T x = s4[0];
+      if (PREC == kFP32Kahan && i < 3) x = add_(x, (T)c4[0]);  // the dense terms are compensated
+      x = scaled_sum<PREC>(i, x, D.par);
+      if (V > 1) A.part[8 * i + v] = x;
+      else team_term<PREC>(A.part, i, i == 4 ? raw_term<PREC>(4, x, J.nmcs) : x, D.par, L);
     }
-    if (lane == 0) A.part[8 * i + v] = scaled_sum<PREC>(i, s, D.par);
+  }
+  if (sub == G - 1) {
+    if (lane < V) {
+      if (V > 1) A.part[8 * 7 + lane] = A.mcs[lane];
+      else team_term<PREC>(A.part, 7, raw_term<PREC>(7, A.mcs[0], J.nmcs), D.par, L);
+    }
+    if (lane == 8) team_term<PREC>(A.part, 8, raw_term<PREC>(8, A.mcs[8], J.nmcs), D.par, L);
   }
   team_sync(team, G);
+  if (SOLO && sub > 0) return 0;
 
-  // every warp: lane i adds term i's shares in order (dense terms compensated) and
-  // finishes it; the weighted total in term order
+  // every warp: lane i has term i, finished where it was summed, or (V > 1) adds its shares in order (dense terms
+  // compensated) and finishes it; the weighted total in term order
   const int i = min(lane, 8);
   const T *p = A.part + 8 * i;
-  T x = p[0];
-  float c = 0.f;
-  if (V > 1) {
+  raw = p[0];
+  e = p[1];
+  if (V > 1 && i != 8) {
+    T x = raw;
+    float c = 0.f;
 #pragma unroll
     for (int v = 1; v < 8; ++v)
-      if (v < V && i != 5 && i != 8) kahan_add_any(x, c, p[v]);
+      if (v < V && i != 5) kahan_add_any(x, c, p[v]);
     if (PREC == kFP32Kahan && i < 3) x = add_(x, (T)c);
-    if (i == 7) x = raw_term<PREC>(7, x, J.nmcs);
+    raw = i == 4 || i == 7 ? raw_term<PREC>(i, x, J.nmcs) : x;
+    e = norm_term(i, raw, D.par, L);
   }
-  raw = i == 4 ? raw_term<PREC>(4, x, J.nmcs) : x;
-  e = norm_term(i, raw, D.par, L);
   T tot = 0;
 #pragma unroll
   for (int k = 0; k < 9; ++k) tot = fma_((T)D.par->w[k], __shfl_sync(0xffffffffu, e, k), tot);
   return tot;
 }
+
+// Random numbers of steps [s, s + kDrawSteps) of replica r by one warp, the counters
+// of the one-warp kernel: lane 2 q + w has word w of step s + q.  Row q of draw:
+// the six moves and two unused words; logu: the logarithm of the acceptance draw.
+__device__ __forceinline__ void draw_steps(const DevJob &J, int r, int s, float *draw, double *logu)
+{
+  const int lane = lane_id();
+  const Philox4 d = philox4x32_10((uint32_t)(s + (lane >> 1)), (uint32_t)(J.rid_base + r), 0u, (uint32_t)(lane & 1),
+                                  J.key0, J.key1);
+  float *o = draw + 8 * (lane >> 1) + 4 * (lane & 1);
+  o[0] = u01(d.v[0]);
+  o[1] = u01(d.v[1]);
+  o[2] = u01(d.v[2]);
+  o[3] = u01(d.v[3]);
+  if (lane & 1) logu[lane >> 1] = log((double)u01(d.v[2]));
+}
+
+// Metropolis test in FP64, kernel_cuda_l1_montecarlo.cu:485-507.
+__device__ __forceinline__ int team_accept(double logu, float etot, float ecur, double mbeta)
+{
+  return logu < (to_double(etot) - to_double(ecur)) * mbeta;
+}
+
+// A replica's state, statistics and Record during a chunk, kept by one warp of its
+// team (state and statistics in shared memory).
+struct TeamRecord {
+  Record *rec;
+  int acc, ne;  // accepted in the step before; Record entries
+
+  __device__ __forceinline__ void begin(const KArgs &A, const DevJob &J, int r, ReplicaMC *srep, WarpStats *wst)
+  {
+    const int lane = lane_id();
+    reinterpret_cast<int *>(srep)[lane] = reinterpret_cast<const int *>(J.rep + r)[lane];
+    if (lane == 0) load_stats(wst, J.stats[r]);
+    rec = (J.rec && (A.flags & kMcRecord)) ? J.rec + r : nullptr;
+    acc = J.run_acc[r];
+    ne = 0;
+    if (J.rec && (A.flags & kMcResetRecord)) {
+      if (lane == 0) J.rec[r].next_entry = 0;
+    } else if (rec) {
+      ne = rec->next_entry;
+    }
+    __syncwarp();
+  }
+  // Before step s: a state that was accepted is recorded, kernel_cuda_l1_montecarlo.cu:290-297.
+  __device__ __forceinline__ void before(ReplicaMC *srep, int s)
+  {
+    if (!acc) return;
+    const int lane = lane_id();
+    if (lane == 0) srep->step = s;
+    __syncwarp();
+    if (rec && ne < GD_STEPS_PER_DUMP)
+      reinterpret_cast<int *>(&rec->replica[ne])[lane] = reinterpret_cast<const int *>(srep)[lane];
+    ++ne;
+  }
+  // After step s: lane k < 9 has term k in et, lane k < 6 word k of the pose in pm.
+  __device__ __forceinline__ void after(ReplicaMC *srep, WarpStats *wst, int s, int accept, float et, float etot, float pm)
+  {
+    const int lane = lane_id();
+    if (accept) {
+      if (lane < 9) srep->energy[lane] = et;
+      if (lane == 9) srep->energy[9] = etot;
+      if (lane < 6) srep->movematrix[lane] = pm;
+    }
+    __syncwarp();
+    if (lane == 0) step_stats(wst, accept, (double)srep->energy[9], s, srep->movematrix);
+    acc = accept;
+  }
+  __device__ __forceinline__ void end(const KArgs &A, const DevJob &J, int r, ReplicaMC *srep, const WarpStats *wst,
+                                      int nsteps)
+  {
+    const int lane = lane_id();
+    if (lane == 0) {
+      J.run_acc[r] = acc;
+      if (A.flags & kMcStoreAccept) srep->is_accept = acc;
+      if (rec) rec->next_entry = ne;
+      store_stats(J.stats[r], wst, nsteps);
+    }
+    __syncwarp();
+    reinterpret_cast<int *>(J.rep + r)[lane] = reinterpret_cast<const int *>(srep)[lane];
+  }
+};
 
 // WIDE: teams of 8 and 16 warps, one CTA per SM: 128 registers, deep pair loops.
 template <int MODE, int PREC, bool WIDE>
@@ -349,85 +502,37 @@ __global__ void __maxnreg__(PREC == kFP64 || WIDE ? 128 : 80) team_kernel(KArgs 
       } else {
         // ---- Monte Carlo chunk for replica r; the team's first warp keeps its state
         const bool lead = sub == 0;
-        const int gr = J.rid_base + r;
         const ReplicaMC *grep = J.rep + GD_AT(r, J.nrep, kSiteRep);
-        ReplicaMC *srep = T_.rep;
-        WarpStats *wst = T_.stats;
-        int *sw = reinterpret_cast<int *>(srep);
         float cur = lane < 6 ? grep->movematrix[lane] : 0.0f;  // every warp's copy of the pose and its total
         float ecur = grep->energy[9];
         const int ilig = grep->idx_lig, iprt = grep->idx_prt;
         const double mbeta = (double)J.minus_beta[GD_AT(grep->idx_tmp, J.ntmp, kSiteTmp)];
-        Record *rec = (J.rec && (A.flags & kMcRecord)) ? J.rec + r : nullptr;
-        int acc = 0, ne = 0;
-        if (lead) {
-          sw[lane] = reinterpret_cast<const int *>(grep)[lane];
-          if (lane == 0) load_stats(wst, J.stats[r]);
-          acc = J.run_acc[r];
-          if (J.rec && (A.flags & kMcResetRecord)) {
-            if (lane == 0) J.rec[r].next_entry = 0;
-          } else if (rec) {
-            ne = rec->next_entry;
-          }
-          __syncwarp();
-        }
+        TeamRecord R;
+        if (lead) R.begin(A, J, r, T_.rep, T_.stats);
         const bool initial = (A.flags & kMcInitial) != 0;
         const int s0 = (A.d_step ? *A.d_step + A.s_begin : A.s_begin) + J.step0;
         const int nsteps = J.nsteps > 0 ? min(J.nsteps, A.nsteps) : A.nsteps;
         for (int k = 0; k < nsteps; ++k) {
           const int s = s0 + k, ks = k & (kDrawSteps - 1);
           if (ks == 0 && !initial) {
-            // draws of steps s .. s + 15, the counters of the one-warp kernel: lane 2 q + w has word w of step s + q
-            const Philox4 d = philox4x32_10((uint32_t)(s + (lane >> 1)), (uint32_t)gr, 0u, (uint32_t)(lane & 1), J.key0,
-                                            J.key1);
             __syncwarp();
-            float *o = draw + 8 * (lane >> 1) + 4 * (lane & 1);
-            o[0] = u01(d.v[0]);
-            o[1] = u01(d.v[1]);
-            o[2] = u01(d.v[2]);
-            o[3] = u01(d.v[3]);
-            if (lane & 1) logu[lane >> 1] = log((double)u01(d.v[2]));
+            draw_steps(J, r, s, draw, logu);
             __syncwarp();
           }
           const float pm = lane < 6 ? __fmaf_rn(D.par->move_scale[lane], initial ? 0.0f : draw[8 * ks + lane], cur) : 0.0f;
-          if (lead && acc) {
-            // record the old state, kernel_cuda_l1_montecarlo.cu:290-297
-            if (lane == 0) srep->step = s;
-            __syncwarp();
-            if (rec && ne < GD_STEPS_PER_DUMP) reinterpret_cast<int *>(&rec->replica[ne])[lane] = sw[lane];
-            ++ne;
-          }
+          if (lead) R.before(T_.rep, s);
           T et, raw;
           const float etot =
               (float)team_energy<PREC, WIDE, MODE == 2>(J, D, T_, lig, team, sub, G, V, chunks, ilig, iprt, pm, et, raw);
-          // Metropolis test in FP64, kernel_cuda_l1_montecarlo.cu:485-507, the same in every warp
           int accept = 1;
-          if (!initial) accept = logu[ks] < (to_double(etot) - to_double(ecur)) * mbeta;
+          if (!initial) accept = team_accept(logu[ks], etot, ecur, mbeta);
           if (accept) {
             ecur = etot;
             cur = pm;
           }
-          if (lead) {
-            if (accept) {
-              if (lane < 9) srep->energy[lane] = (float)et;
-              if (lane == 9) srep->energy[9] = etot;
-              if (lane < 6) srep->movematrix[lane] = pm;
-            }
-            __syncwarp();
-            if (lane == 0) step_stats(wst, accept, (double)srep->energy[9], s, srep->movematrix);
-            acc = accept;
-          }
+          if (lead) R.after(T_.rep, T_.stats, s, accept, (float)et, etot, pm);
         }
-        if (lead) {
-          if (lane == 0) {
-            J.run_acc[r] = acc;
-            if (A.flags & kMcStoreAccept) srep->is_accept = acc;
-            if (rec) rec->next_entry = ne;
-            store_stats(J.stats[r], wst, nsteps);
-          }
-          __syncwarp();
-          reinterpret_cast<int *>(J.rep + r)[lane] = sw[lane];
-        }
+        if (lead) R.end(A, J, r, T_.rep, T_.stats, nsteps);
       }
     }
     if constexpr (MODE != 2) __syncthreads();
