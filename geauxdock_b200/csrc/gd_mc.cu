@@ -37,6 +37,9 @@
 // across lanes with a compensated butterfly; the FP64 variant evaluates the
 // reference's forms in double.
 #include <cstdio>
+#include <map>
+#include <mutex>
+#include <tuple>
 #include <type_traits>
 
 #include "gd_device.cuh"
@@ -715,17 +718,47 @@ struct SpecLaunch {
   }
 };
 
-int cluster_occupancy(int precision, const TileConfig &tc, size_t smem)
+// Occupancies of this process: they depend on the device, the kernel and the launch
+// alone, and a small pose call looks up more of them (45 us) than its kernel
+// takes.  Emptied when it has grown past any set of shapes in use.
+static int known_occupancy(McKernel f, int cluster, const TileConfig &tc, size_t smem, int (*look)(McKernel, const TileConfig &, size_t))
 {
-  const McKernel f = pick_spec(precision);
-  SpecLaunch l;
-  int n = 0;
-  if (!f || l.prepare(f, tc, 1, smem, nullptr) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, (const void *)f, &l.cfg) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return 0;
+  struct Key {
+    McKernel f;
+    size_t smem;
+    int dev, warps, cluster;
+    bool operator<(const Key &o) const
+    {
+      return std::tie(f, smem, dev, warps, cluster) < std::tie(o.f, o.smem, o.dev, o.warps, o.cluster);
+    }
+  };
+  static std::mutex mu;
+  static std::map<Key, int> known;
+  Key k{f, smem, 0, tc.warps_per_cta, cluster};
+  if (!f || cudaGetDevice(&k.dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto it = known.find(k);
+  if (it != known.end()) return it->second;
+  const int n = look(f, tc, smem);
+  if (n > 0) {  // a failure may be of the moment
+    if (known.size() >= 4096) known.clear();
+    known[k] = n;
   }
   return n;
+}
+
+int cluster_occupancy(int precision, const TileConfig &tc, size_t smem)
+{
+  return known_occupancy(pick_spec(precision), tc.cluster, tc, smem, [](McKernel f, const TileConfig &t, size_t bytes) {
+    SpecLaunch l;
+    int n = 0;
+    if (l.prepare(f, t, 1, bytes, nullptr) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, (const void *)f, &l.cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    return n;
+  });
 }
 
 cudaError_t launch_kernel(int mode, int precision, const TileConfig &tc, const KArgs &a, int grid, cudaStream_t st)
@@ -750,12 +783,12 @@ cudaError_t launch_kernel(int mode, int precision, const TileConfig &tc, const K
 
 int kernel_occupancy(int mode, int precision, const TileConfig &tc, size_t smem)
 {
-  const McKernel f = pick_kernel(mode, precision, tc);
-  if (!f) return 0;
-  if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-  int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, tc.warps_per_cta * 32, smem) != cudaSuccess) return 0;
-  return nb;
+  return known_occupancy(pick_kernel(mode, precision, tc), 1, tc, smem, [](McKernel f, const TileConfig &t, size_t bytes) {
+    int nb = 0;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, t.warps_per_cta * 32, bytes) != cudaSuccess) return 0;
+    return nb;
+  });
 }
 
 cudaError_t launch_exchange_all(const DevJob *d_jobs, const int *d_xoff, int njob, int total, int x,

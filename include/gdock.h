@@ -113,7 +113,10 @@ int Dock(Complex *ch, Record *rh, Complex **cd, Record **rd, ParaT **pt, gd_rng_
  * cudaHostRegister with mapping -- the kernels write each Record entry into it
  * as the chunk runs and no copy follows; entries at and past a Record's
  * next_entry keep what rh held; 0, or pageable rh: the Records go to rd[g] and
- * the whole array is copied to rh after each chunk), "device_base" (the
+ * the whole array is copied to rh after each chunk), "eval_cache" (1:
+ * gd_eval_poses keeps its device block and stream for the next call, at most
+ * four of at most 32 MiB each; 0: it keeps none, and those kept are freed),
+ * "device_base" (the
  * drop-in API's GPU g is CUDA device device_base + g, for one process per GPU;
  * set it before SetDevice/DeviceAlloc and keep it), "wait_limit"
  * (microseconds, on the GPU's global timer, that the kernel's bounded
