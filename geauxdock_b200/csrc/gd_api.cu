@@ -200,14 +200,19 @@ int configure(gd_ensemble *e, TileConfig tc)
 }
 
 // Work items of R replicas at most (build_items).
+long long count_items(const std::vector<int> &pr, int R)
+{
+  long long items = 0;
+  for (size_t r = 0, k; r < pr.size(); r += k) {
+    for (k = 1; r + k < pr.size() && (int)k < R && pr[r + k] == pr[r]; ++k) {}
+    ++items;
+  }
+  return items;
+}
 long long count_items(const gd_ensemble *e, int R)
 {
   long long items = 0;
-  for (const std::vector<int> &pr : e->rep_prt)
-    for (size_t r = 0, k; r < pr.size(); r += k) {
-      for (k = 1; r + k < pr.size() && (int)k < R && pr[r + k] == pr[r]; ++k) {}
-      ++items;
-    }
+  for (const std::vector<int> &pr : e->rep_prt) items += count_items(pr, R);
   return items;
 }
 
@@ -220,6 +225,10 @@ ShapeQuery shape_query(const gd_ensemble *e, int stage_opt, int nsm)
   q.nsm = nsm;
   q.stage_opt = stage_opt;
   q.items = [e](int R) { return count_items(e, R); };
+  q.loads = [e](int R, std::vector<std::pair<double, long long>> &out) {
+    for (size_t j = 0; j < e->jobs.size(); ++j)
+      out.emplace_back((double)e->jobs[j].dj.natom * e->jobs[j].dj.npoint_pad, count_items(e->rep_prt[j], R));
+  };
   return q;
 }
 
@@ -233,8 +242,10 @@ int choose_warps(gd_ensemble *e, TileConfig base, int stage_opt = -1)
   GD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device));
   int grid = 0;
   const ShapeQuery q = shape_query(e, stage_opt, nsm);
-  if (e->kernel == GD_KERNEL_BATCHED && choose_team(q, base, grid)) return configure(e, base);
-  if (base.group == 1 && choose_spread(q, base, grid)) return configure(e, base);
+  if ((e->kernel == GD_KERNEL_BATCHED && choose_team(q, base, grid)) || (base.group == 1 && choose_spread(q, base, grid))) {
+    if (e->kernel == GD_KERNEL_BATCHED) choose_waves(q, base, grid);
+    return configure(e, base);
+  }
   double best = 1e300;
   const int G = e->kernel == GD_KERNEL_PLAIN ? 1 : std::max(1, base.group);
   int best_w = std::max(8, G), best_stage = 1;
@@ -272,6 +283,10 @@ int choose_warps(gd_ensemble *e, TileConfig base, int stage_opt = -1)
   tc.warps_per_cta = best_w;
   tc.stage = best_stage;
   tc.group = G;
+  if (e->kernel == GD_KERNEL_BATCHED && smem_for(e, tc) <= kSmemLimit) {
+    grid = (int)std::min(count_items(e, best_w / G), (long long)kernel_occupancy(0, e->precision, tc, smem_for(e, tc)) * nsm);
+    choose_waves(q, tc, grid);
+  }
   return configure(e, tc);
 }
 

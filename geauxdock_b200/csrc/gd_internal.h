@@ -200,6 +200,7 @@ struct TileConfig {
                        // replica's results depend on this alone
   int cluster = 1;     // more than one (Monte Carlo, one team of 8 or 16 warps per CTA): CTAs of a cluster, which share a
                        // replica's chunk (gd_spec.cuh)
+  bool wide = false;   // one warp per replica in FP32, 16 or fewer per SM: the kernel with 128 registers
 };
 
 // Pair-tile shape where the caller leaves it to the library (option value 0).

@@ -416,8 +416,11 @@ __device__ __forceinline__ void store_stats(RepStats &S, const WarpStats *w, int
   for (int i = 0; i < 6; ++i) S.best_mm[i] = w->best_mm[i];
 }
 
-template <int MODE, int PREC, int KPL, int AB>
-__global__ void __maxnreg__(PREC == kFP64 ? 128 : 80) mc_kernel(KArgs A)
+// 80 registers keep 24 warps on an SM.  WIDE, for launches that have 16 or fewer for each: with 128 the points of a row
+// overlap further, which counts where few warps hide each other's latency (80 atoms x 2200 points, a step beside 8 and
+// 16 warps per SM 402 -> 353 us and 570 -> 543 us).
+template <int MODE, int PREC, int KPL, int AB, bool WIDE = false>
+__global__ void __maxnreg__(PREC == kFP64 || WIDE ? 128 : 80) mc_kernel(KArgs A)
 {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar;
@@ -666,7 +669,7 @@ static McKernel pick_kernel(const TileConfig &tc)
       if (tc.kpl == 2 && tc.ab == 8) return mc_kernel<MODE, PREC, 2, 8>;
       if (tc.kpl == 4 && tc.ab == 4) return mc_kernel<MODE, PREC, 4, 4>;
     }
-    if (tc.kpl == 4 && tc.ab == 8) return mc_kernel<MODE, PREC, 4, 8>;
+    if (tc.kpl == 4 && tc.ab == 8) return tc.wide ? mc_kernel<MODE, PREC, 4, 8, true> : mc_kernel<MODE, PREC, 4, 8>;
     return nullptr;
   }
 }

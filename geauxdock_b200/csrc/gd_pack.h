@@ -185,6 +185,8 @@ struct ShapeQuery {
   int nsm = 0;
   int stage_opt = -1;            // pocket staged: 1 always, 0 never, -1 by the shape
   std::function<long long(int)> items;  // work items of at most R replicas
+  // per job: atoms x points of a replica, and its work items of at most R replicas (unset: one job)
+  std::function<void(int, std::vector<std::pair<double, long long>> &)> loads;
   size_t smem(const TileConfig &tc) const
   {
     return kernel_smem_bytes(tc.stage ? Pmax : 0, Pmax, lig_slots, precision, tc);
@@ -194,6 +196,8 @@ struct ShapeQuery {
 // or one: false where one wave does not hold the replicas.
 bool choose_team(const ShapeQuery &q, TileConfig &tc, int &grid);
 bool choose_spread(const ShapeQuery &q, TileConfig &tc, int &grid);
+// Instead of the shape given, teams in more than one wave where that ends sooner.
+void choose_waves(const ShapeQuery &q, TileConfig &tc, int &grid);
 
 void free_pocket(DevPocket &p);
 void free_job(DevJobBuf &j);

@@ -280,15 +280,21 @@ void round_shape(gd_server *s, const std::vector<ServeReq *> &act, long long nre
     for (const ServeReq *r : act) n += r->items[R];
     return n;
   };
+  q.loads = [&act](int R, std::vector<std::pair<double, long long>> &out) {
+    for (const ServeReq *r : act) out.emplace_back((double)r->jd.L * r->buf.dj.npoint_pad, r->items[R]);
+  };
   if (s->cfg.warps == 0 && (choose_team(q, tc, grid) || (tc.group == 1 && choose_spread(q, tc, grid)))) {
+    choose_waves(q, tc, grid);
     s->rtc = tc;
     s->rgrid = grid;
     return;
   }
   // the shape chosen at creation, at this round's sizes
   if (tc.stage && q.smem(tc) > kSmemLimit) tc.stage = 0;
+  grid = std::max(1, kernel_occupancy(0, s->precision, tc, q.smem(tc))) * s->nsm;
+  if (s->cfg.warps == 0) choose_waves(q, tc, grid);
   s->rtc = tc;
-  s->rgrid = std::max(1, kernel_occupancy(0, s->precision, tc, q.smem(tc))) * s->nsm;
+  s->rgrid = grid;
 }
 
 int enqueue_round(gd_server *s, long long k, std::vector<ServeReq *> &finishing, bool &enqueued)

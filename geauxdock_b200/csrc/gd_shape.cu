@@ -1,5 +1,10 @@
 // gd_shape.cu -- launch shapes of the batched kernel: the warps a replica gets.
 #include <algorithm>
+#include <cmath>
+#include <functional>
+#include <queue>
+#include <utility>
+#include <vector>
 
 #include "gd_pack.h"
 
@@ -70,15 +75,80 @@ bool choose_spread(const ShapeQuery &q, TileConfig &tc, int &grid)
     t.stage = q.stage_opt > 0 ? 1 : 0;
     const size_t smem = q.smem(t);
     if (smem > kSmemLimit) continue;
-    const long long items = q.items(w);
-    if (items > (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm) continue;
-    const long long load = (items + q.nsm - 1) / q.nsm * w;
+    const long long items = q.items(w), load = (items + q.nsm - 1) / q.nsm * w;
     if (best >= 0 && load >= best) continue;
+    t.wide = load <= 16 && q.precision != kFP64 && t.kpl == 4 && t.ab == 8;
+    if (items > (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm) continue;
     best = load;
     tc = t;
     grid = (int)std::max(1LL, items);
   }
   return best >= 0;
+}
+
+// How long a step of the launch takes by a model of it: the work items, heaviest
+// first, on `slots` CTAs.  An atom pair against 32 points takes a warp 150 + 62 w
+// cycles beside w warps on its scheduler (80 atoms x 2200 points, 8, 9-12, 16 and
+// 24 warps per SM: 278, 338, 394 and 606 of them; with 128 registers 120 + 64 w);
+// a team of 2 or 4 takes 1.3 times
+// its share of that (8 x 2 warps 465 / 2, 4 x 4 warps 514 / 4).
+static double step_cycles(const ShapeQuery &q, const TileConfig &tc, long long slots)
+{
+  std::vector<std::pair<double, long long>> load;
+  q.loads(tc.warps_per_cta / tc.group, load);
+  std::sort(load.begin(), load.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+  long long items = 0;
+  for (const auto &l : load) items += l.second;
+  slots = std::max(1LL, std::min(slots, items));
+  const double w = std::ceil((double)((slots + q.nsm - 1) / q.nsm * tc.warps_per_cta) / 4.0);
+  const double alone = tc.wide && tc.group == 1 ? 120.0 + 64.0 * w : 150.0 + 62.0 * w;
+  const double per = alone * (tc.group > 1 ? 1.3 : 1.0) / tc.group / 64.0;
+  std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+  for (long long i = 0; i < slots; ++i) free_at.push(0.0);
+  double last = 0.0;
+  for (const auto &l : load)
+    for (long long i = 0; i < l.second; ++i) {
+      const double t = free_at.top() + l.first * per;
+      free_at.pop();
+      free_at.push(t);
+      last = std::max(last, t);
+    }
+  return last;
+}
+
+// Jobs of uneven sizes: with one warp per replica a step of the whole launch takes
+// what the largest replica takes one warp, while the warps of the small ones have
+// long finished; teams in several waves, largest first, share it out.  400
+// replicas each of 20, 33, 45 and 80 atoms against 2200 points, one wave of one
+// warp 493 us a step, 2 or 4 teams of 4 per CTA 333 us; of 8, 14, 25 and 70 atoms
+// 431 and 217 us, against 800 points 140 and 106 us; but of 40, 42 and 45 atoms
+// 266 and 305 us, of 80 alone 493 and 543 us.  So by the model above, where it
+// says an eighth less (teams of 8 and 16 are not: their few half rows per warp
+// follow no such rule).
+void choose_waves(const ShapeQuery &q, TileConfig &tc, int &grid)
+{
+  if (q.mode != 0 || !q.loads || tc.group > 4 || (tc.split == 1 && q.precision != kFP64 && (tc.kpl != 4 || tc.ab != 8)))
+    return;
+  if (q.items(1) > 32LL * q.nsm) return;  // long past one wave even of one warp each
+  double best = 0.875 * step_cycles(q, tc, grid);
+  const TileConfig base = tc;
+  for (const int G : {4, 2})
+    for (const int warps : {16, 8}) {
+      TileConfig t = base;
+      t.group = G;
+      t.warps_per_cta = warps;
+      t.stage = q.stage_opt > 0 ? 1 : 0;
+      if (t.stage && q.smem(t) > kSmemLimit) t.stage = 0;
+      const size_t smem = q.smem(t);
+      if (smem > kSmemLimit) continue;
+      const long long slots = (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm;
+      if (slots < 1) continue;
+      const double c = step_cycles(q, t, slots);
+      if (c >= best) continue;
+      best = c;
+      tc = t;
+      grid = (int)std::max(1LL, std::min(slots, q.items(warps / G)));
+    }
 }
 
 }  // namespace gd
