@@ -30,6 +30,14 @@ static void choose_cluster(const ShapeQuery &q, TileConfig &tc, long long items)
     }
 }
 
+// CTAs that the registers of the GPU's SMs could hold: a launch with more is not asked about, since the first question
+// about a kernel loads its code.
+static long long register_wave(const ShapeQuery &q, const TileConfig &tc)
+{
+  const int regs = q.precision == kFP64 || tc.group >= 8 || tc.wide ? 128 : 80;  // gd_mc.cu, gd_team.cuh
+  return 65536LL / (regs * 32 * tc.warps_per_cta) * q.nsm;
+}
+
 // A team is the best use of a warp that no replica needs.  Measured per step of
 // an ensemble of n replicas (40 atoms x 1500 points) on 1, 2, 4, 8 and 16 warps
 // each, where one wave holds the teams: n = 48 128 / 77 / 44 / 22 / 19 us;
@@ -51,8 +59,8 @@ bool choose_team(const ShapeQuery &q, TileConfig &tc, int &grid)
       if (t.stage && q.smem(t) > kSmemLimit) t.stage = 0;
       const size_t smem = q.smem(t);
       if (smem > kSmemLimit) continue;
-      const long long items = q.items(R), wave = (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm;
-      if (items > wave) continue;
+      const long long items = q.items(R);
+      if (items > register_wave(q, t) || items > (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm) continue;
       tc = t;
       choose_cluster(q, tc, items);
       grid = (int)std::max(1LL, items);
@@ -78,7 +86,7 @@ bool choose_spread(const ShapeQuery &q, TileConfig &tc, int &grid)
     const long long items = q.items(w), load = (items + q.nsm - 1) / q.nsm * w;
     if (best >= 0 && load >= best) continue;
     t.wide = load <= 16 && q.precision != kFP64 && t.kpl == 4 && t.ab == 8;
-    if (items > (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm) continue;
+    if (items > register_wave(q, t) || items > (long long)kernel_occupancy(q.mode, q.precision, t, smem) * q.nsm) continue;
     best = load;
     tc = t;
     grid = (int)std::max(1LL, items);
@@ -90,8 +98,8 @@ bool choose_spread(const ShapeQuery &q, TileConfig &tc, int &grid)
 // first, on `slots` CTAs.  An atom pair against 32 points takes a warp 150 + 62 w
 // cycles beside w warps on its scheduler (80 atoms x 2200 points, 8, 9-12, 16 and
 // 24 warps per SM: 278, 338, 394 and 606 of them; with 128 registers 120 + 64 w);
-// a team of 2 or 4 takes 1.3 times
-// its share of that (8 x 2 warps 465 / 2, 4 x 4 warps 514 / 4).
+// a team of 2 or 4 takes 1.3 times its share of that (8 x 2 warps 465 / 2, 4 x 4
+// warps 514 / 4).
 static double step_cycles(const ShapeQuery &q, const TileConfig &tc, long long slots)
 {
   std::vector<std::pair<double, long long>> load;
