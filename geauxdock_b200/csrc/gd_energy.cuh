@@ -117,7 +117,7 @@ struct PairConst {
 
 // The same in FP64, and the exponential's table.
 struct PairConst64 {
-  double lj0, lj01, el0, el1, inv_el1, ea, eb;
+  double lj0, lj01, el0, inv_el1, ed2, ea, eb;
   const double *tab;
 };
 
@@ -418,27 +418,27 @@ __device__ __forceinline__ double rsqrt64(double x)
   return fma_(mul_(y, e), fma_(0.375, e, 0.5), y);
 }
 
+constexpr int kExpTab = 256;
+
 // exp(x) in FP64 after Tang (Table-driven implementation of the exponential
-// function in IEEE floating-point arithmetic, ACM TOMS 15, 1989): x = (32 m + j)
-// ln2/32 + r, |r| <= ln2/64, exp(x) = 2^m 2^(j/32) exp(r), the last from its Taylor
-// series to r^6 (remainder below 4e-18), 2^(j/32) from tab[32].  Measured within
+// function in IEEE floating-point arithmetic, ACM TOMS 15, 1989): x = (256 m + j)
+// ln2/256 + r, |r| <= ln2/512, exp(x) = 2^m 2^(j/256) exp(r), the last from its Taylor
+// series to r^4 (remainder below 4e-17), 2^(j/256) from tab[256].  Measured within
 // 4.0e-16 relative of exp() on [-700, 700].  Beyond it 0 and 2^1000, whose
 // reciprocals act as those of exp() would; NaN stays NaN.
 __device__ __forceinline__ double exp64(double x, const double *tab)
 {
   const double kMagic = 6755399441055744.0;  // 1.5 2^52: the nearest integer in the low word
-  const double k = fma_(x, 46.16624130844683, kMagic);
+  const double k = fma_(x, 8 * 46.16624130844683, kMagic);
   const int n = __double2loint(k);
   const double kn = sub_(k, kMagic);
-  const double r = fma_(kn, -7.247021293269686e-19, fma_(kn, -0.02166084939249829, x));
-  double p = fma_(r, 1.0 / 720.0, 1.0 / 120.0);
-  p = fma_(p, r, 1.0 / 24.0);
-  p = fma_(p, r, 1.0 / 6.0);
+  const double r = fma_(kn, -7.247021293269686e-19 / 8, fma_(kn, -0.02166084939249829 / 8, x));
+  double p = fma_(r, 1.0 / 24.0, 1.0 / 6.0);
   p = fma_(p, r, 0.5);
   p = fma_(p, r, 1.0);
   p = fma_(p, r, 1.0);
-  const double v = mul_(p, tab[n & 31]);
-  int hi = __double2hiint(v) + ((n >> 5) << 20), lo = __double2loint(v);
+  const double v = mul_(p, tab[n & (kExpTab - 1)]);
+  int hi = __double2hiint(v) + ((n >> 8) << 20), lo = __double2loint(v);
   const int xh = __double2hiint(x), mag = xh & 0x7fffffff;
   if (mag > 0x4085e000) {  // |x| > 700, infinite or NaN
     hi = mag > 0x7ff00000 ? 0x7ff80000 : xh < 0 ? 0 : 0x7e700000;
@@ -449,13 +449,14 @@ __device__ __forceinline__ double exp64(double x, const double *tab)
 
 // Per work item, the FP64 kernel's (ligand type group, point type) entries in
 // shared memory: pk = (1/p1a, -p2a/p1a), pf = (-pmf0, pmf1, hdb0, hdb1), the
-// hydrogen-bond entries zero where hdb0 <= 0.1; and tab = 2^(j/32), j < 32.
+// hydrogen-bond entries zero where hdb0 <= 0.1; and tab = 2^(j/256),
+// j < 256.
 // Padding point types get 1/p1a = 1e200 and 0 else: at their distance (over 1e3)
 // their Lennard-Jones term is below 1e-227, the others exactly 0.
 __device__ __forceinline__ void build_pair_tables64(const DevJob &J, const int2 *lg, double2 *pk, float4 *pf, double *tab)
 {
   const int L = J.natom;
-  for (int j = threadIdx.x; j < 32; j += blockDim.x) tab[j] = exp2((double)j / 32.0);
+  for (int j = threadIdx.x; j < kExpTab; j += blockDim.x) tab[j] = exp2((double)j / kExpTab);
   int g = 0;
   for (int a = 0; a < L; ++g) {
     const int lt = GD_AT(lg[GD_AT(a, L, kSiteLgrp)].x, kLigTypes, kSiteTab);
@@ -474,10 +475,13 @@ __device__ __forceinline__ void build_pair_tables64(const DevJob &J, const int2 
 // reference's formulas with the Lennard-Jones term divided through by p1 (as in
 // FP32), which leaves one reciprocal square root, two reciprocals and one
 // exponential per pair.  Bound by the FP64 pipe (2.04 cycles a warp operation and
-// scheduler, ~50 a pair): 199 cycles per 32 pairs with CUDA's rsqrt, __drcp_rn and
-// exp, 154 with the Newton steps, 140 with the table-driven exponential too, at 16
-// warps per SM; 2048 poses of 64 atoms x 3000 points 2.73 -> 2.16 ms.  1e-300 keeps
-// d > 0 where a point and an atom coincide.
+// scheduler, 44 a pair) and the issue of the ~30 others: 199 cycles per 32 pairs with
+// CUDA's rsqrt, __drcp_rn and exp, 154 with the Newton steps, 140 with the
+// exponential from a table of 32 too, at 16 warps per SM; 2048 poses of 64 atoms x
+// 3000 points 2.73 -> 2.16 ms, with the table of 256 and the near field told by d^2
+// 2.03.  (Table entries held in FP64, or converted by integer operations, cost more
+// than the conversions: 2.09, 2.21.)  1e-300 keeps d > 0 where a point and an atom
+// coincide.
 template <bool HDB>
 __device__ __forceinline__ void pair_atoms64(const V4<double> *lig, int a, int aend, int L, const double (&px)[2],
                                              const double (&py)[2], const double (&pz)[2], const double2 (&k)[2],
@@ -496,7 +500,7 @@ __device__ __forceinline__ void pair_atoms64(const V4<double> *lig, int a, int a
       const double d3 = mul_(d2, d);
       const double den = fma_(mul_(mul_(d3, d3), d3), k[j].x, fma_(c.lj01, d2, c.lj0));
       vdw[j] = fma_(fma_(k[j].y, d3, 1.0), rcp64(den), vdw[j]);
-      const double g = mul_(c.el1, d) < 1.0 ? fma_(d2, fma_(c.eb, d, c.ea), c.el0) : mul_(r, c.inv_el1);
+      const double g = d2 < c.ed2 ? fma_(d2, fma_(c.eb, d, c.ea), c.el0) : mul_(r, c.inv_el1);
       ele[j] = fma_(la.w, g, ele[j]);
       const double e1 = add_(1.0, exp64(mul_(fma_(-0.5, d, 6.0), add_(d, (double)f[j].x)), c.tab));
       pmf[j] = fma_((double)f[j].y, rcp64(e1), pmf[j]);
@@ -518,10 +522,11 @@ __device__ __forceinline__ void pass1_row64(const V4<double> *lig, int L, const 
   c.lj0 = par->lj0;
   c.lj01 = mul_(c.lj0, (double)par->lj1);
   c.el0 = par->el0;
-  c.el1 = par->el1;
-  c.ea = mul_(mul_((double)par->a1, c.el1), c.el1);
-  c.eb = mul_(mul_(mul_((double)par->b1, c.el1), c.el1), c.el1);
-  c.inv_el1 = __drcp_rn(c.el1);
+  const double el1 = par->el1;
+  c.ea = mul_(mul_((double)par->a1, el1), el1);
+  c.eb = mul_(mul_(mul_((double)par->b1, el1), el1), el1);
+  c.inv_el1 = __drcp_rn(el1);
+  c.ed2 = __drcp_rn(mul_(el1, el1));
   c.tab = tab;
   double vdw[2] = {0, 0}, pmf[2] = {0, 0}, hdb[2] = {0, 0}, qe = 0;
 #pragma unroll 1

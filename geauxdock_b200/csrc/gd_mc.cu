@@ -163,7 +163,7 @@ __host__ __device__ inline SmemLayout smem_layout(int P, int Pall, int lig_slots
   s.aph = off;
   off = align16(off + 16u * entries);
   s.ahd = off;
-  off = align16(off + (fp64 ? 8u * 32u : 16u * npairs));
+  off = align16(off + (fp64 ? 8u * (uint32_t)kExpTab : 16u * npairs));
   s.lig_bytes = (uint32_t)lig_slots * (fp64 ? 32u : 16u);  // V4<double> per atom, or LigPair per two atoms
   // per replica: ReplicaMC state, EnergyScratch (192 B), WarpStats (64 B); per warp the rotated ligand
   const uint32_t state = (uint32_t)sizeof(ReplicaMC) + 192u + 64u;
