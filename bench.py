@@ -110,7 +110,7 @@ def _args():
                    help="replicas per serving round (0: the server's default, four waves of resident replicas)")
     p.add_argument("--serve-round", type=int, default=STEPS_PER_INTERVAL, help="MC steps per serving round")
     p.add_argument("--serve-replica-warps", type=int, default=1,
-                   help="warps per replica in the server (2, 4, 8: latency mode)")
+                   help="order of the server's energy sums: of a replica on 2, 4 or 8 warps")
     p.add_argument("--partition-intervals", type=int, default=5,
                    help="exchange intervals timed in the multi-GPU partition leg (one complex split across ranks)")
     return p.parse_args()
@@ -341,7 +341,8 @@ def run_single(args, local: int) -> dict:
     cx = synth.to_complex(job, pk, ep, steps_total=args.single_steps, steps_per_dump=200)
     out = {"workload": "1 complex: ligand 24 atoms, pocket 600 points, 200 KDE points, 8 MCS templates, "
                        f"1 temperature, 1 replica, {args.single_steps} MC steps"}
-    # batched kernel with the replica on 1, 2, 4, 8 warps (latency mode), and the plain kernel
+    # batched kernel with its sums in the order of a replica on 1, 2, 4, 8 warps (the launch shape is the library's
+    # choice in each), and the plain kernel
     for name, kern, g in (("batched", 0, 1), ("batched_2_warps", 0, 2), ("batched_4_warps", 0, 4),
                           ("batched_8_warps", 0, 8), ("plain", 1, 1)):
         check(lib.gd_set_option(b"kernel", kern))
