@@ -41,6 +41,7 @@
 #include <mutex>
 #include <tuple>
 #include <type_traits>
+#include <utility>
 
 #include "gd_device.cuh"
 #include "gd_internal.h"
@@ -701,6 +702,23 @@ static McKernel pick_spec(int precision)
   return nullptr;
 }
 
+// Lets kernel f be launched with `bytes` of dynamic shared memory on the current device.  The limit only rises: a thread
+// that asks for less must not take it from under another's launch.
+static cudaError_t allow_smem(McKernel f, size_t bytes)
+{
+  static std::mutex mu;
+  static std::map<std::pair<McKernel, int>, size_t> allowed;
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  size_t &now = allowed[{f, dev}];
+  if (bytes <= now) return cudaSuccess;
+  const cudaError_t s = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (s == cudaSuccess) now = bytes;
+  return s;
+}
+
 struct SpecLaunch {
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[1];
@@ -715,7 +733,7 @@ struct SpecLaunch {
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess || tc.cluster <= 8) return e;
     return cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   }
@@ -778,7 +796,7 @@ cudaError_t launch_kernel(int mode, int precision, const TileConfig &tc, const K
     const cudaError_t e = l.prepare(k, tc, a.n_items, smem, st);
     return e != cudaSuccess ? e : cudaLaunchKernelEx(&l.cfg, k, b);
   }
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   k<<<grid, tc.warps_per_cta * 32, smem, st>>>(b);
   return cudaGetLastError();
@@ -788,7 +806,7 @@ int kernel_occupancy(int mode, int precision, const TileConfig &tc, size_t smem)
 {
   return known_occupancy(pick_kernel(mode, precision, tc), 1, tc, smem, [](McKernel f, const TileConfig &t, size_t bytes) {
     int nb = 0;
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return 0;
+    if (allow_smem(f, bytes) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, t.warps_per_cta * 32, bytes) != cudaSuccess) return 0;
     return nb;
   });
