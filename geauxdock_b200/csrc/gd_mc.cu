@@ -665,9 +665,11 @@ static McKernel pick_kernel(const TileConfig &tc)
   if (tc.group > 1) return team_kernel<MODE, PREC, false>;
   if constexpr (PREC == kFP64) return tc.kpl == 1 && tc.ab == 8 ? mc_kernel<MODE, PREC, 1, 8> : nullptr;
   else {
-    if constexpr (MODE != 2) {  // mode 2 has one shape
-      if (tc.kpl == 2 && tc.ab == 4) return mc_kernel<MODE, PREC, 2, 4>;
+    // mode 2: the default shape, and (2, 8) with compensated sums for gd_noalloc.cu
+    if constexpr (MODE != 2 || PREC == kFP32Kahan)
       if (tc.kpl == 2 && tc.ab == 8) return mc_kernel<MODE, PREC, 2, 8>;
+    if constexpr (MODE != 2) {
+      if (tc.kpl == 2 && tc.ab == 4) return mc_kernel<MODE, PREC, 2, 4>;
       if (tc.kpl == 4 && tc.ab == 4) return mc_kernel<MODE, PREC, 4, 4>;
     }
     if (tc.kpl == 4 && tc.ab == 8) return tc.wide ? mc_kernel<MODE, PREC, 4, 8, true> : mc_kernel<MODE, PREC, 4, 8>;

@@ -27,8 +27,8 @@
 // L1, and the pocket-specific cells 4 bytes each, which fit where the dense
 // potential was.  4096 poses of 40 atoms x 1500 points x 11 conformations in FP32:
 // the former kernel, one type group of atoms at a time in scalar arithmetic, 991
-// us, now 417 us (bound by the pair loop as the Monte Carlo kernel is); the whole
-// call 1.24 -> 0.45 ms.
+// us, now 450 us (bound by the pair loop as the Monte Carlo kernel is); the whole
+// call 1.27 -> 0.49 ms.
 #include <algorithm>
 #include <mutex>
 
@@ -78,10 +78,17 @@ struct NaShapes {
 };
 NaShapes g_na_shape[kNaMaxDevices][3];
 
+// In FP32 the rows of pass 1 are 64 points, one warp per pose or (the split order
+// of 2) a team, and the sums compensated whichever FP32 precision is asked for: rows
+// of 128, the other kernels' order, are 7 % faster (4096 poses of 40 x 1500, 461 us a
+// call against 495) but their longer chains of plain additions lose more: rms error
+// of the raw terms against 64 bits, 40 x 1500, 20 x 400 and 64 x 2048, 1.6, 0.85 and
+// 1.3e-7 against 0.88, 0.62 and 0.79e-7 (the former kernel of this call: 1.9, 0.77
+// and 0.87e-7).
 TileConfig na_tile(int precision, int lg, int R)
 {
-  TileConfig t{R << lg, precision == kFP64 ? 1 : 4, 8, 0, 1 << lg};
-  return t;
+  const bool fp64 = precision == kFP64;
+  return TileConfig{R << lg, fp64 ? 1 : 2, 8, 0, 1 << lg, fp64 || lg == 0 ? 1 : 2};
 }
 
 int noalloc_shape(int dev, int precision, int n, TileConfig &tc, int &n_items, int &grid)
@@ -187,7 +194,8 @@ extern "C" int gd_eval_poses_noalloc(const Complex *d_complex, int n, const int 
   }
   NoAllocScratch *S = nullptr;
   GD_TRY(noalloc_scratch(&S));
-  TileConfig tc{8, 4, 8};
+  if (precision == GD_PREC_FP32) precision = GD_PREC_FP32_KAHAN;  // na_tile
+  TileConfig tc = na_tile(precision, 0, 8);
   KArgs a{};
   int grid = 0;
   if (n > 0) GD_TRY(noalloc_shape(dev, precision, n, tc, a.n_items, grid));

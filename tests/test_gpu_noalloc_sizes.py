@@ -1,7 +1,9 @@
 """gd_eval_poses_noalloc at the sizes where its launch or its packing changes:
 one pose and a few (teams of warps), more than one wave of CTAs, a potential that
 is non-zero everywhere, no KDE point, an odd atom count and one row of points.
-Its sums are combined as gd_eval_poses combines them: the same bits."""
+In FP64 its sums are combined as gd_eval_poses combines them, in FP32 as the
+tile (2, 8) does with compensated sums (one warp per pose) or as a replica split
+over two warps (teams): the same bits."""
 
 import ctypes as C
 
@@ -9,7 +11,7 @@ import numpy as np
 import pytest
 
 from geauxdock_b200 import dock, synth
-from geauxdock_b200._lib import GD_E_INVALID, GD_PREC_FP32, GD_PREC_FP32_KAHAN, GD_PREC_FP64
+from geauxdock_b200._lib import GD_E_INVALID, GD_PREC_FP32, GD_PREC_FP32_KAHAN, GD_PREC_FP64, check
 
 pytestmark = pytest.mark.gpu
 
@@ -37,17 +39,48 @@ def _case(L, P, K, M, nlig, nprt, dense, n):
     return pk, job, conf, synth.config4_poses(n, n, radius=5.0)
 
 
-@pytest.mark.parametrize("prec", [GD_PREC_FP32, GD_PREC_FP32_KAHAN, GD_PREC_FP64])
-@pytest.mark.parametrize("L,P,K,M,nlig,nprt,dense,n", [
-    (24, 600, 200, 8, 1, 1, False, 1), (33, 129, 0, 17, 3, 2, False, 150), (64, 2048, 1000, 40, 2, 3, True, 700),
-    (17, 300, 60, 1, 4, 4, True, 5000)])
-def test_noalloc_equals_eval_poses(lib, enepara, L, P, K, M, nlig, nprt, dense, n, prec):
+SIZES = [(24, 600, 200, 8, 1, 1, False, 1), (33, 129, 0, 17, 3, 2, False, 150), (64, 2048, 1000, 40, 2, 3, True, 600),
+         (17, 300, 60, 1, 4, 4, True, 5000)]
+
+
+@pytest.mark.parametrize("L,P,K,M,nlig,nprt,dense,n", SIZES)
+def test_noalloc_fp64_equals_eval_poses(lib, enepara, L, P, K, M, nlig, nprt, dense, n):
     pk, job, conf, mm = _case(L, P, K, M, nlig, nprt, dense, n)
     cx = synth.to_complex(job, pk, enepara)
-    want, want_raw, _ = dock.eval_poses(cx, conf, mm, prec)
-    rc, out, raw = _call(lib, cx, conf, mm, prec)
+    want, want_raw, _ = dock.eval_poses(cx, conf, mm, GD_PREC_FP64)
+    rc, out, raw = _call(lib, cx, conf, mm, GD_PREC_FP64)
     assert rc == 0
     assert out.tobytes() == want.tobytes() and raw.tobytes() == want_raw.tobytes()
+
+
+@pytest.mark.parametrize("prec", [GD_PREC_FP32, GD_PREC_FP32_KAHAN])
+@pytest.mark.parametrize("L,P,K,M,nlig,nprt,dense,n", SIZES)
+def test_noalloc_fp32_sums(lib, enepara, L, P, K, M, nlig, nprt, dense, n, prec):
+    pk, job, conf, mm = _case(L, P, K, M, nlig, nprt, dense, n)
+    try:
+        if n > 1776:
+            cx = synth.to_complex(job, pk, enepara)
+            check(lib.gd_set_option(b"kpl", 2))
+            want = dock.eval_poses(cx, conf, mm, GD_PREC_FP32_KAHAN)[0]
+        else:
+            # the poses as the initial states of replicas split over two warps
+            ntmp = n // (nlig * nprt)
+            job.temps = np.linspace(0.3, 3.0, ntmp).astype(np.float32)
+            cx = synth.to_complex(job, pk, enepara)
+            reps = cx[0]["replica"][:n]
+            reps["movematrix"] = mm
+            conf = np.stack([reps["idx_lig"], reps["idx_prt"]], axis=1).astype(np.int32)
+            check(lib.gd_set_option(b"replica_warps", 2))
+            with dock.Ensemble.from_complexes([cx], [1]) as e:
+                e.init()
+                e.sync()
+                want = np.ascontiguousarray(e.replicas(0)["energy"])
+    finally:
+        check(lib.gd_set_option(b"kpl", 0))
+        check(lib.gd_set_option(b"replica_warps", 1))
+    rc, out, _ = _call(lib, cx, conf, mm, prec)
+    assert rc == 0
+    assert out.tobytes() == want.tobytes()
 
 
 @pytest.mark.parametrize("n", [40, 4000])
