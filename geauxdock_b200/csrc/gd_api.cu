@@ -1135,14 +1135,14 @@ std::vector<int> eval_order(int n, const int *conf, int nprt)
 {
   std::vector<int> at(nprt + 1, 0), ord;
   bool sorted = true;
-  for (int i = 0; i < n; ++i) {
+  for (size_t i = 0; i < (size_t)n; ++i) {
     ++at[conf[2 * i + 1] + 1];
     sorted &= i == 0 || conf[2 * i + 1] >= conf[2 * i - 1];
   }
   if (sorted) return ord;
   for (int p = 0; p < nprt; ++p) at[p + 1] += at[p];
   ord.resize(n);
-  for (int i = 0; i < n; ++i) ord[at[conf[2 * i + 1]]++] = i;
+  for (int i = 0; i < n; ++i) ord[at[conf[2 * (size_t)i + 1]]++] = i;
   return ord;
 }
 
@@ -1210,16 +1210,16 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
             double *out64, float *raw)
 {
   const DevJob &J = e->jobs[job].dj;
-  for (int i = 0; i < n; ++i)
+  for (size_t i = 0; i < (size_t)n; ++i)
     if (conf[2 * i] < 0 || conf[2 * i] >= J.nlig || conf[2 * i + 1] < 0 || conf[2 * i + 1] >= J.nprt)
-      return fail(GD_E_INVALID, "pose %d: conformation (%d, %d) out of range", i, conf[2 * i], conf[2 * i + 1]);
+      return fail(GD_E_INVALID, "pose %zu: conformation (%d, %d) out of range", i, conf[2 * i], conf[2 * i + 1]);
   const Options o = opts();
   TileConfig tc{8, o.kpl, o.ab};
   default_pair_tile(tc.kpl, tc.ab);
   if (precision == GD_PREC_FP64) tc.kpl = 1, tc.ab = 8;
   const std::vector<int> ord = eval_order(n, conf, J.nprt);
   std::vector<int> count(J.nprt, 0);
-  for (int i = 0; i < n; ++i) ++count[conf[2 * i + 1]];
+  for (size_t i = 0; i < (size_t)n; ++i) ++count[conf[2 * i + 1]];
   ShapeQuery q;
   GD_CUDA(cudaDeviceGetAttribute(&q.nsm, cudaDevAttrMultiProcessorCount, e->device));
   q.mode = 1;
@@ -1228,7 +1228,7 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
   q.lig_slots = e->lig_slots;
   q.items = [&](int R) {
     long long m = 0;
-    for (const int k : count) m += (k + R - 1) / R;
+    for (const long long k : count) m += (k + R - 1) / R;
     return m;
   };
   int grid = 0;
@@ -1248,7 +1248,7 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
   B.send(h, ord, conf, mm);
   WorkItem *it = (WorkItem *)(h + B.items);
   for (int p = 0, r = 0; p < J.nprt; r += count[p++])
-    for (int k = 0; k < count[p]; k += R) *it++ = WorkItem{job, p, r + k, std::min(R, count[p] - k)};
+    for (long long k = 0; k < count[p]; k += R) *it++ = WorkItem{job, p, (int)(r + k), (int)std::min<long long>(R, count[p] - k)};
   GD_CUDA(cudaMemcpyAsync(d, h, B.sent, cudaMemcpyHostToDevice, e->st));
   GD_CUDA(cudaMemsetAsync(e->d_queue, 0, sizeof(int), e->st));
   KArgs a{};
@@ -1527,9 +1527,9 @@ int gd_eval_poses(const Complex *c, int n, const int *conf, const float *mm, int
   if (!c || n < 0 || (n > 0 && (!conf || !mm || !out))) return fail(GD_E_INVALID, "null argument");
   if (precision < GD_PREC_FP32 || precision > GD_PREC_FP64) return fail(GD_E_INVALID, "precision = %d", precision);
   if (n == 0) return GD_OK;
-  for (int i = 0; i < n; ++i)
+  for (size_t i = 0; i < (size_t)n; ++i)
     if (conf[2 * i] < 0 || conf[2 * i] >= c->size.n_lig || conf[2 * i + 1] < 0 || conf[2 * i + 1] >= c->size.n_prt)
-      return fail(GD_E_INVALID, "pose %d: conformation (%d, %d) out of range", i, conf[2 * i], conf[2 * i + 1]);
+      return fail(GD_E_INVALID, "pose %zu: conformation (%d, %d) out of range", i, conf[2 * i], conf[2 * i + 1]);
   int dev = 0;
   GD_CUDA(cudaGetDevice(&dev));
   if (eval_complex(c, n, conf, mm, precision, out, out64, raw)) return GD_OK;

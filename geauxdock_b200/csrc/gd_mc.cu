@@ -462,13 +462,13 @@ __global__ void __maxnreg__(PREC == kFP64 || WIDE ? 128 : 80) mc_kernel(KArgs A)
       const int r = wi.rep0 + warp;  // job-local index
       if constexpr (MODE >= 1) {
         // ---- pose evaluation
-        const int ilig = A.conf[2 * r], iprt = A.conf[2 * r + 1];
+        const int ilig = A.conf[2 * (size_t)r], iprt = A.conf[2 * (size_t)r + 1];
         if constexpr (MODE == 2) {
           if (bad_pose(A, J, r, ilig, iprt, true)) continue;  // no barrier follows in this mode
           pos = J.pos + (size_t)iprt * J.npoint_pad;
           aux = J.aux + (size_t)iprt * J.npoint_pad;
         }
-        if (lane < 6) esc->mm[lane] = A.mm[6 * r + lane];
+        if (lane < 6) esc->mm[lane] = A.mm[6 * (size_t)r + lane];
         __syncwarp();
         energy_warp<PREC, KPL, AB, MODE == 2>(J, par, pos, aux, lgrp, apt, aph, ahd, ligbuf, ilig, iprt, esc);
         if (lane < 10) {

@@ -108,14 +108,14 @@ int noalloc_shape(int dev, int precision, int n, TileConfig &tc, int &n_items, i
   // as choose_team: the most warps per pose for which one wave holds all, else 8 poses a CTA
   for (int lg = 4; lg >= 1; --lg)
     for (int R = 1; R << lg <= kMaxCtaThreads / 32; ++R)
-      if ((n + R - 1) / R <= s.wave[lg][R]) {
+      if ((n - 1) / R < s.wave[lg][R]) {
         tc = na_tile(precision, lg, R);
-        grid = n_items = (n + R - 1) / R;
+        grid = n_items = (n - 1) / R + 1;
         return GD_OK;
       }
   if (s.wave[0][8] < 1) return fail(GD_E_CUDA, "the pose kernel cannot launch");
   tc = na_tile(precision, 0, 8);
-  n_items = (n + 7) / 8;
+  n_items = (n - 1) / 8 + 1;
   grid = std::min(n_items, s.wave[0][8]);
   return GD_OK;
 }

@@ -482,13 +482,13 @@ __global__ void __maxnreg__(PREC == kFP64 || WIDE ? 128 : 80) team_kernel(KArgs 
     if (team < wi.count) {
       const int r = wi.rep0 + team;  // job-local index
       if constexpr (MODE >= 1) {
-        const int ilig = A.conf[2 * r], iprt = A.conf[2 * r + 1];
+        const int ilig = A.conf[2 * (size_t)r], iprt = A.conf[2 * (size_t)r + 1];
         if constexpr (MODE == 2) {
           if (bad_pose(A, J, r, ilig, iprt, sub == 0)) continue;  // the team alike; no CTA barrier follows
           D.pos = J.pos + (size_t)iprt * J.npoint_pad;
           D.aux = J.aux + (size_t)iprt * J.npoint_pad;
         }
-        const float pm = lane < 6 ? A.mm[6 * r + lane] : 0.0f;
+        const float pm = lane < 6 ? A.mm[6 * (size_t)r + lane] : 0.0f;
         T et, raw;
         const T tot = team_energy<PREC, WIDE, MODE == 2>(J, D, T_, lig, team, sub, G, V, chunks, ilig, iprt, pm, et, raw);
         if (sub == 0) {
