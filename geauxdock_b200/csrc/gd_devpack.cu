@@ -506,6 +506,8 @@ __device__ void dp_ligand(const Complex *cx, const PackDst &D, const DpSizes &s,
       R.idx_lig = R.idx_prt = R.idx_tmp = 0;  // in range, whatever reads it before the flag is seen
     }
     D.rep[r] = R;
+    int *words = reinterpret_cast<int *>(D.rep + r);
+    for (int i = kReplicaUsed / 4; i < (int)(sizeof(ReplicaMC) / 4); ++i) words[i] = 0;
     D.run_acc[r] = R.is_accept;
     RepStats S;
     S.e_sum = S.e_sum2 = S.best_e = 0.0;

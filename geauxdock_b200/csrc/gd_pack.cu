@@ -246,6 +246,7 @@ int job_from_complex(const Complex *c, int rep_begin, int rep_end, uint64_t seed
   jd.rid_base = rep_begin;
   jd.nrep_total = sz.n_rep;
   jd.reps.assign(c->replica + rep_begin, c->replica + rep_end + 1);
+  for (ReplicaMC &R : jd.reps) std::memset((unsigned char *)&R + kReplicaUsed, 0, sizeof(R) - kReplicaUsed);
   for (size_t i = 0; i < jd.reps.size(); ++i) {
     const ReplicaMC &R = jd.reps[i];
     if (R.idx_lig < 0 || R.idx_lig >= sz.n_lig || R.idx_prt < 0 || R.idx_prt >= sz.n_prt || R.idx_tmp < 0 ||

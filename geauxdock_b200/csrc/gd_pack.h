@@ -177,6 +177,10 @@ enum { kFieldNLig = 1, kFieldNPrt, kFieldNatom, kFieldNatomConf, kFieldNpoint, k
 cudaError_t device_pack(const Complex *d_cx, const PackDst &D, cudaStream_t st);
 const char *pack_field_name(int field);
 
+// The members of a ReplicaMC end here; the rest of its 128 bytes is padding, which the packers clear: the kernels copy
+// states whole, and a caller's Complex need not have it initialised.
+constexpr size_t kReplicaUsed = offsetof(ReplicaMC, is_accept) + sizeof(int);
+
 // What a launch's shape depends on (gd_shape.cu).
 constexpr size_t kSmemLimit = 227 * 1024;
 struct ShapeQuery {
