@@ -401,14 +401,17 @@ struct RowSums {
 // ------------------------------------------------------ pair loop, FP64 --
 // Reciprocal and reciprocal square root in FP64: the PTX approximation (about 20
 // bits) and one step of the third-order Newton (Halley) iteration, which cubes its
-// error; measured within 2.3e-16 and 2.7e-16 relative.  x positive, normal and
-// finite, as every argument below is.
+// error; measured within 2.3e-16 and 2.7e-16 relative.  x positive and normal, as
+// every argument below is, and that of rsqrt64 finite.  That of rcp64 may be infinite
+// (d^9 of a pose 1e12 A away against a padding point): the approximation is then 0,
+// which the iteration would make NaN of.
 __device__ __forceinline__ double rcp64(double x)
 {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma_(-x, y, 1.0);
-  return fma_(y, fma_(e, e, e), y);
+  const double z = fma_(y, fma_(e, e, e), y);
+  return __double2hiint(x) < 0x7ff00000 ? z : y;
 }
 __device__ __forceinline__ double rsqrt64(double x)
 {
