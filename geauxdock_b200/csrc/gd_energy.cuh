@@ -712,6 +712,8 @@ __device__ __forceinline__ WalkTerm<RealOf<PREC>> psp_cell(const int4 *cell, int
     else d = mul_(d2, rsqrt_approx(d2));
     hits += add_(d, thr) <= (T)0 ? 1 : 0;
   }
+  // (the FP32 loop over these cells has always multiplied; the others added the value of a hit only)
+  if (PREC == kFP64 && hits == 0) return {0, 0};
   return {(T)hits, (T)__int_as_float(c0.w)};
 }
 
@@ -736,6 +738,8 @@ __device__ __forceinline__ WalkTerm<RealOf<PREC>> psp_cell4(const DevJob &J, int
     else d = mul_(d2, rsqrt_approx(d2));
     hits += add_(d, thr) <= (T)0 ? 1 : 0;
   }
+  // a cell without a hit adds nothing, be its value infinite or NaN
+  if (hits == 0) return {0, 0};
   return {(T)hits, (T)J.psp_table[t * GD_MAXPRO + (c >> 16)]};
 }
 
