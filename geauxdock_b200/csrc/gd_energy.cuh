@@ -529,7 +529,7 @@ __device__ __forceinline__ void pass1_row64(const V4<double> *lig, int L, const 
   c.ea = mul_(mul_((double)par->a1, el1), el1);
   c.eb = mul_(mul_(mul_((double)par->b1, el1), el1), el1);
   c.inv_el1 = __drcp_rn(el1);
-  c.ed2 = __drcp_rn(mul_(el1, el1));
+  c.ed2 = el1 > 0.0 ? __drcp_rn(mul_(el1, el1)) : INFINITY;  // el1 d < 1
   c.tab = tab;
   double vdw[2] = {0, 0}, pmf[2] = {0, 0}, hdb[2] = {0, 0}, qe = 0;
 #pragma unroll 1
