@@ -399,48 +399,81 @@ struct RowSums {
 };
 
 // ------------------------------------------------------ pair loop, FP64 --
-// Reciprocal and reciprocal square root in FP64: the PTX approximation (about 20
-// bits) and one step of the third-order Newton (Halley) iteration, which cubes its
-// error; measured within 2.3e-16 and 2.7e-16 relative.  x positive and normal, as
-// every argument below is, and that of rsqrt64 finite.  That of rcp64 may be infinite
-// (d^9 of a pose 1e12 A away against a padding point): the approximation is then 0,
-// which the iteration would make NaN of.
+// Reciprocal in FP64: the PTX approximation (an error of up to 1e-6) and one step
+// of the third-order Newton (Halley) iteration, which cubes that: the rounding of the
+// last operation is what remains (within 1.12e-16 relative).  x positive, normal and
+// finite, as every argument below is.
 __device__ __forceinline__ double rcp64(double x)
 {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma_(-x, y, 1.0);
-  const double z = fma_(y, fma_(e, e, e), y);
-  return __double2hiint(x) < 0x7ff00000 ? z : y;
+  return fma_(y, fma_(e, e, e), y);
 }
-__device__ __forceinline__ double rsqrt64(double x)
+// Square root d of x and half the reciprocal of it, h, in FP64: from the PTX approximation
+// y the pair (x y, y / 2), corrected by one third-order step (Goldschmidt's form of
+// the iteration, whose error e undoes half the rounding of x y: d is within 1.7e-16
+// relative, rms 4.9e-17, where x (1 / sqrt(x)) has 2.2e-16 and 7.0e-17 and sqrt() 1.1e-16
+// and 4.4e-17).  x positive, normal and finite.
+__device__ __forceinline__ void sqrt64(double x, double &d, double &h)
 {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma_(mul_(-x, y), y, 1.0);
-  return fma_(mul_(y, e), fma_(0.375, e, 0.5), y);
+  const double h0 = __hiloint2double(__double2hiint(y) - 0x100000, __double2loint(y));  // y / 2
+  const double g = mul_(x, y);
+  const double e = fma_(-g, h0, 0.5);
+  const double t = fma_(mul_(1.5, e), e, e);
+  h = fma_(h0, t, h0);
+  d = fma_(g, t, g);
 }
 
 constexpr int kExpTab = 256;
 
+// Entry j of the exponential's table: 2^(j / 256) as the sum of two doubles, tab[j] and
+// tab[256 + j], from the product of the 2^(2^b / 256) of j's bits (an error of about 1e-31).
+__device__ __forceinline__ void exp_table_entry(double *tab, int j)
+{
+  constexpr double kPow[8][2] = {{1.0027112750502025, -3.6366159286922639e-17}, {1.0054299011128027, 9.4991865354550318e-17},
+                                 {1.0108892860517005, -1.5234778603368577e-17}, {1.0218971486541166, 5.1092250289734439e-17},
+                                 {1.0442737824274138, 8.5518897055379649e-17}, {1.0905077326652577, -3.0467820798124711e-17},
+                                 {1.189207115002721, 3.9820152314656461e-17}, {1.4142135623730951, -9.6672933134529135e-17}};
+  double hi = 1.0, lo = 0.0;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    if (!((j >> b) & 1)) continue;
+    const double p = mul_(hi, kPow[b][0]);
+    const double e = fma_(hi, kPow[b][0], -p) + fma_(hi, kPow[b][1], mul_(lo, kPow[b][0]));
+    hi = add_(p, e);
+    lo = sub_(e, sub_(hi, p));
+  }
+  tab[j] = hi;
+  tab[kExpTab + j] = lo;
+}
+
 // exp(x) in FP64 after Tang (Table-driven implementation of the exponential
 // function in IEEE floating-point arithmetic, ACM TOMS 15, 1989): x = (256 m + j)
-// ln2/256 + r, |r| <= ln2/512, exp(x) = 2^m 2^(j/256) exp(r), the last from its Taylor
-// series to r^4 (remainder below 4e-17), 2^(j/256) from tab[256].  Measured within
-// 4.0e-16 relative of exp() on [-700, 700].  Beyond it 0 and 2^1000, whose
-// reciprocals act as those of exp() would; NaN stays NaN.
+// ln2/256 + r, |r| <= ln2/512 = a, exp(x) = 2^m 2^(j/256) exp(r), exp(r) - 1 from its
+// Taylor series to r^4 with the coefficient of r^3 raised by (3/4) a^2 / 120, which
+// takes up most of the fifth power (remainder below 1e-17), 2^(j/256) from tab, with its
+// second part (LOW) or without.  Within 1.3e-16 (2.4e-16) relative of the exponential on
+// [-700, 700]; CUDA's exp() was measured within 1.36e-16.  The pmf term takes the
+// form without: its factor 1 / (1 + exp(z)) carries |z| times the rounding of z, 3.8e-16
+// rms, and the second part changes that by a thousandth.  Beyond the range 0 and 2^1000,
+// whose reciprocals act as those of exp() would; NaN stays NaN.
+template <bool LOW>
 __device__ __forceinline__ double exp64(double x, const double *tab)
 {
-  const double kMagic = 6755399441055744.0;  // 1.5 2^52: the nearest integer in the low word
+  constexpr double kMagic = 6755399441055744.0;  // 1.5 2^52: the nearest integer in the low word
+  constexpr double kA = 0.6931471805599453 / 512.0;
   const double k = fma_(x, 8 * 46.16624130844683, kMagic);
   const int n = __double2loint(k);
   const double kn = sub_(k, kMagic);
   const double r = fma_(kn, -7.247021293269686e-19 / 8, fma_(kn, -0.02166084939249829 / 8, x));
-  double p = fma_(r, 1.0 / 24.0, 1.0 / 6.0);
+  double p = fma_(r, 1.0 / 24.0, 1.0 / 6.0 + 0.75 * kA * kA / 120.0);
   p = fma_(p, r, 0.5);
-  p = fma_(p, r, 1.0);
-  p = fma_(p, r, 1.0);
-  const double v = mul_(p, tab[n & (kExpTab - 1)]);
+  const double q = fma_(mul_(p, r), r, r);  // exp(r) - 1
+  const int j = n & (kExpTab - 1);
+  const double t = tab[j], v = LOW ? add_(t, fma_(t, q, tab[kExpTab + j])) : fma_(t, q, t);
   int hi = __double2hiint(v) + ((n >> 8) << 20), lo = __double2loint(v);
   const int xh = __double2hiint(x), mag = xh & 0x7fffffff;
   if (mag > 0x4085e000) {  // |x| > 700, infinite or NaN
@@ -451,23 +484,21 @@ __device__ __forceinline__ double exp64(double x, const double *tab)
 }
 
 // Per work item, the FP64 kernel's (ligand type group, point type) entries in
-// shared memory: pk = (1/p1a, -p2a/p1a), pf = (-pmf0, pmf1, hdb0, hdb1), the
-// hydrogen-bond entries zero where hdb0 <= 0.1; and tab = 2^(j/256),
-// j < 256.
-// Padding point types get 1/p1a = 1e200 and 0 else: at their distance (over 1e3)
-// their Lennard-Jones term is below 1e-227, the others exactly 0.
+// shared memory: pk = (1/p1a, -p2a), pf = (-pmf0, pmf1, hdb0, hdb1), the
+// hydrogen-bond entries zero where hdb0 <= 0.1; and the exponential's table.
+// Padding point types get 1/p1a = 1e30 and 0 else: at their distance (over 1e3)
+// their Lennard-Jones term is below 1e-57, the others exactly 0.
 __device__ __forceinline__ void build_pair_tables64(const DevJob &J, const int2 *lg, double2 *pk, float4 *pf, double *tab)
 {
   const int L = J.natom;
-  for (int j = threadIdx.x; j < kExpTab; j += blockDim.x) tab[j] = exp2((double)j / kExpTab);
+  for (int j = threadIdx.x; j < kExpTab; j += blockDim.x) exp_table_entry(tab, j);
   int g = 0;
   for (int a = 0; a < L; ++g) {
     const int lt = GD_AT(lg[GD_AT(a, L, kSiteLgrp)].x, kLigTypes, kSiteTab);
     for (int pt = threadIdx.x; pt < kTabCols; pt += blockDim.x) {
       const float4 r = J.ref4[lt * kTabCols + pt], t = J.par->tab4[lt][pt];
       const bool real = pt < kPadType;
-      pk[g * kTabCols + pt] = real ? make_double2(1.0 / (double)r.x, -(double)r.y / (double)r.x)
-                                   : make_double2(1.0e200, 0.0);
+      pk[g * kTabCols + pt] = real ? make_double2(1.0 / (double)r.x, -(double)r.y) : make_double2(1.0e30, 0.0);
       pf[g * kTabCols + pt] = real ? make_float4(t.z, t.w, r.z, r.w) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     a = lg[a].y;
@@ -476,15 +507,19 @@ __device__ __forceinline__ void build_pair_tables64(const DevJob &J, const int2 
 
 // Terms of the atoms [a, aend) of one type against the lane's two points, the
 // reference's formulas with the Lennard-Jones term divided through by p1 (as in
-// FP32), which leaves one reciprocal square root, two reciprocals and one
-// exponential per pair.  Bound by the FP64 pipe (2.04 cycles a warp operation and
-// scheduler, 44 a pair) and the issue of the ~30 others: 199 cycles per 32 pairs with
-// CUDA's rsqrt, __drcp_rn and exp, 154 with the Newton steps, 140 with the
-// exponential from a table of 32 too, at 16 warps per SM; 2048 poses of 64 atoms x
-// 3000 points 2.73 -> 2.16 ms, with the table of 256 and the near field told by d^2
-// 2.03.  (Table entries held in FP64, or converted by integer operations, cost more
-// than the conversions: 2.09, 2.21.)  1e-300 keeps d > 0 where a point and an atom
-// coincide.
+// FP32; p = d^3 / p1a in numerator and denominator, so that its rounding cancels where
+// the term decays), which leaves one square root, two reciprocals and one exponential
+// per pair.  Bound by the FP64 pipe (2.04 cycles a warp operation and scheduler, 45 a
+// pair) and the issue of the ~30 others.  2048 poses of 64 atoms x 3000 points: 2.73 ms
+// with CUDA's rsqrt, __drcp_rn and exp, 2.16 with the Newton steps and an exponential
+// from a table of 32, 2.03 with one of 256 and the near field told by d^2, 2.06 in the
+// forms here, which are no less exact than the reference's in double (8,300 poses against
+// 113-bit arithmetic, rms error of the terms vdw, ele, pmf, hdb, hpc relative to their mean:
+// 3.65, 8.50, 0.58, 4.35 and 2.27e-16; formulas as written with CUDA's functions 3.69, 9.13,
+// 0.58, 4.39 and 2.43e-16; d as x (1 / sqrt(x)) and the exponential without its table's
+// second part 4.57e-16 for hdb).  The table's second part for the pmf term's exponential
+// too takes 6 % more, d corrected by its remainder 3 %.  1e-300 keeps d > 0 where a point
+// and an atom coincide.
 template <bool HDB>
 __device__ __forceinline__ void pair_atoms64(const V4<double> *lig, int a, int aend, int L, const double (&px)[2],
                                              const double (&py)[2], const double (&pz)[2], const double2 (&k)[2],
@@ -498,18 +533,21 @@ __device__ __forceinline__ void pair_atoms64(const V4<double> *lig, int a, int a
     for (int j = 0; j < 2; ++j) {
       const double dx = sub_(la.x, px[j]), dy = sub_(la.y, py[j]), dz = sub_(la.z, pz[j]);
       const double d2 = fma_(dx, dx, fma_(dy, dy, fma_(dz, dz, 1.0e-300)));
-      const double r = rsqrt64(d2);
-      const double d = mul_(d2, r);
-      const double d3 = mul_(d2, d);
-      const double den = fma_(mul_(mul_(d3, d3), d3), k[j].x, fma_(c.lj01, d2, c.lj0));
-      vdw[j] = fma_(fma_(k[j].y, d3, 1.0), rcp64(den), vdw[j]);
-      const double g = d2 < c.ed2 ? fma_(d2, fma_(c.eb, d, c.ea), c.el0) : mul_(r, c.inv_el1);
+      double d, h;
+      sqrt64(d2, d, h);
+      const double p = mul_(mul_(d2, d), k[j].x);
+      double d6 = mul_(mul_(d2, d2), d2);
+      // at most 2^450 (from 4e22 A on, where the term is below 1e-130): den stays finite
+      d6 = __hiloint2double(min(__double2hiint(d6), 0x5c100000), __double2loint(d6));
+      const double den = fma_(d6, p, fma_(c.lj01, d2, c.lj0));
+      vdw[j] = fma_(fma_(k[j].y, p, 1.0), rcp64(den), vdw[j]);
+      const double g = d2 < c.ed2 ? fma_(d2, fma_(c.eb, d, c.ea), c.el0) : mul_(h, c.inv_el1);
       ele[j] = fma_(la.w, g, ele[j]);
-      const double e1 = add_(1.0, exp64(mul_(fma_(-0.5, d, 6.0), add_(d, (double)f[j].x)), c.tab));
+      const double e1 = add_(1.0, exp64<false>(mul_(fma_(-0.5, d, 6.0), add_(d, (double)f[j].x)), c.tab));
       pmf[j] = fma_((double)f[j].y, rcp64(e1), pmf[j]);
       if constexpr (HDB) {
         const double h3 = mul_(sub_(d, (double)f[j].z), (double)f[j].w);
-        hdb[j] = fma_((double)f[j].w, exp64(mul_(mul_(-0.5, h3), h3), c.tab), hdb[j]);
+        hdb[j] = fma_((double)f[j].w, exp64<true>(mul_(mul_(-0.5, h3), h3), c.tab), hdb[j]);
       }
     }
   }
@@ -528,7 +566,7 @@ __device__ __forceinline__ void pass1_row64(const V4<double> *lig, int L, const 
   const double el1 = par->el1;
   c.ea = mul_(mul_((double)par->a1, el1), el1);
   c.eb = mul_(mul_(mul_((double)par->b1, el1), el1), el1);
-  c.inv_el1 = __drcp_rn(el1);
+  c.inv_el1 = mul_(2.0, __drcp_rn(el1));  // of half of 1/d
   c.ed2 = el1 > 0.0 ? __drcp_rn(mul_(el1, el1)) : INFINITY;  // el1 d < 1
   c.tab = tab;
   double vdw[2] = {0, 0}, pmf[2] = {0, 0}, hdb[2] = {0, 0}, qe = 0;
@@ -649,13 +687,11 @@ __device__ __forceinline__ RealOf<PREC> contact_block(const LigOf<PREC> *lig, in
           if (a >= L) break;
           const V4<double> la = lig[GD_AT(a, L, kSiteLig)];
           const double d2 = dist2(sub_(la.x, px), sub_(la.y, py), sub_(la.z, pz));
-          const double y = fmax(fma_(d2, -1.0 / 81.0, 1.0), 0.0), yy = mul_(y, y);
-          v[k] = fma_(ph, mul_(yy, add_(y, yy)), v[k]);
+          const double y = fmax(fma_(d2, -1.0 / 81.0, 1.0), 0.0);
+          v[k] = fma_(ph, mul_(mul_(mul_(y, y), y), fma_(d2, -0.5 / 81.0, 1.0)), v[k]);
         }
       }
     }
-#pragma unroll
-    for (int k = 0; k < AB; ++k) v[k] = mul_(0.5, v[k]);
   }
 #pragma unroll
   for (int n = AB, off = 16; n > 1; n >>= 1, off >>= 1) {

@@ -163,7 +163,7 @@ __host__ __device__ inline SmemLayout smem_layout(int P, int Pall, int lig_slots
   s.aph = off;
   off = align16(off + 16u * entries);
   s.ahd = off;
-  off = align16(off + (fp64 ? 8u * (uint32_t)kExpTab : 16u * npairs));
+  off = align16(off + (fp64 ? 16u * (uint32_t)kExpTab : 16u * npairs));
   s.lig_bytes = (uint32_t)lig_slots * (fp64 ? 32u : 16u);  // V4<double> per atom, or LigPair per two atoms
   // per replica: ReplicaMC state, EnergyScratch (192 B), WarpStats (64 B); per warp the rotated ligand
   const uint32_t state = (uint32_t)sizeof(ReplicaMC) + 192u + 64u;
@@ -871,3 +871,31 @@ extern "C" int gd_check_report(int *out4, int reset)
   return gd::fail(GD_E_STATE, "not a bounds-checking build (libgdock_check.so is built with -DGD_CHECK)");
 #endif
 }
+
+#ifdef GD_CHECK
+namespace gd {
+// The FP64 pair loop's functions: out[5 i] the reciprocal of x[i], its square root and half the reciprocal of that
+// (x > 0), and the exponential of z[i] with and without the table's second part.
+__global__ void math64_kernel(int n, const double *x, const double *z, double *out)
+{
+  __shared__ double tab[2 * kExpTab];
+  for (int j = threadIdx.x; j < kExpTab; j += blockDim.x) exp_table_entry(tab, j);
+  __syncthreads();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double *o = out + 5 * (size_t)i;
+    o[0] = rcp64(x[i]);
+    sqrt64(x[i], o[1], o[2]);
+    o[3] = exp64<true>(z[i], tab);
+    o[4] = exp64<false>(z[i], tab);
+  }
+}
+}  // namespace gd
+// The same for device arrays, in the bounds-checking build alone.
+extern "C" int gd_check_math64(int n, const double *d_x, const double *d_z, double *d_out)
+{
+  if (n < 1 || !d_x || !d_z || !d_out) return gd::fail(GD_E_INVALID, "null argument");
+  gd::math64_kernel<<<64, 256>>>(n, d_x, d_z, d_out);
+  GD_CUDA(cudaDeviceSynchronize());
+  return GD_OK;
+}
+#endif
