@@ -1,5 +1,7 @@
 // gd_api.cu -- the C ABI of libgdock.so: resident ensembles, the drop-in
 // Dock family, and pose evaluation.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -10,6 +12,7 @@
 #include <mutex>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "gd_pack.h"
@@ -1276,12 +1279,60 @@ int eval_on(gd_ensemble *e, int job, int n, const int *conf, const float *mm, in
   return check_err(e);
 }
 
+// The driver's calls about contexts, looked up in it; ok: all are there.
+struct ContextCalls {
+  CUresult (*get)(CUcontext *) = nullptr;
+  CUresult (*set)(CUcontext) = nullptr;
+  CUresult (*state)(CUdevice, unsigned *, int *) = nullptr;
+  CUresult (*retain)(CUcontext *, CUdevice) = nullptr;
+  CUresult (*release)(CUdevice) = nullptr;
+  CUresult (*id)(CUcontext, unsigned long long *) = nullptr;
+  bool ok = false;
+  ContextCalls()
+  {
+    auto find = [](const char *name, auto &f) {
+      void *p = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      if (cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &q) != cudaSuccess) p = nullptr;
+      f = reinterpret_cast<std::remove_reference_t<decltype(f)>>(p);
+      return p != nullptr;
+    };
+    ok = find("cuCtxGetCurrent", get) && find("cuCtxSetCurrent", set) && find("cuDevicePrimaryCtxGetState", state) &&
+         find("cuDevicePrimaryCtxRetain", retain) && find("cuDevicePrimaryCtxRelease", release) && find("cuCtxGetId", id);
+  }
+  static const ContextCalls &get_calls()
+  {
+    static const ContextCalls c;
+    return c;
+  }
+};
+
+// The id of device dev's primary context (no two contexts of a process have the same; a reset context's successor has
+// another), 0 where there is none or the driver does not tell.  With `current`, 0 too where the calling thread's context
+// is another one.
+unsigned long long primary_context(int dev, bool current)
+{
+  const ContextCalls &d = ContextCalls::get_calls();
+  unsigned flags = 0;
+  int active = 0;
+  CUcontext c = nullptr, p = nullptr;
+  unsigned long long id = 0;
+  if (!d.ok || d.state(dev, &flags, &active) != CUDA_SUCCESS || !active) return 0;
+  if (current && (d.get(&c) != CUDA_SUCCESS || !c)) return 0;
+  if (d.retain(&p, dev) != CUDA_SUCCESS) return 0;
+  if ((current && c != p) || d.id(p, &id) != CUDA_SUCCESS) id = 0;
+  d.release(dev);
+  return id;
+}
+
 // A device block and a stream for one call, from those that calls before it left (option "eval_cache"): getting and
 // giving back 10 MB and a stream takes 750 us, four times what a call of 64 poses does with them.  At most
-// kEvalSpaces are kept, of kEvalKeep bytes each at most; a call that needs more, or fails, leaves none.
+// kEvalSpaces are kept, of kEvalKeep bytes each at most; a call that needs more, or fails, leaves none, nor
+// does one in another context than the device's primary one.  A block of a context that has been reset is forgotten.
 struct EvalSpace {
   struct Kept {
     int dev;
+    unsigned long long ctx;
     size_t bytes;
     unsigned char *d;
     cudaStream_t st;
@@ -1291,15 +1342,19 @@ struct EvalSpace {
   static std::vector<Kept> kept;
 
   int dev;
+  unsigned long long ctx;  // 0: not one whose blocks are kept
   size_t bytes;
   unsigned char *d = nullptr;
   cudaStream_t st = nullptr;
   bool good = false;  // set by the call when all its work on the stream is done and was right
 
-  EvalSpace(int dev_, size_t need) : dev(dev_), bytes(need)
+  EvalSpace(int dev_, size_t need) : dev(dev_), ctx(0), bytes(need)
   {
-    {
+    ctx = primary_context(dev, true);
+    if (ctx) {
       std::lock_guard<std::mutex> lk(mu);
+      kept.erase(std::remove_if(kept.begin(), kept.end(), [this](const Kept &k) { return k.dev == dev && k.ctx != ctx; }),
+                 kept.end());
       for (size_t i = 0; i < kept.size() && !d; ++i)
         if (kept[i].dev == dev && kept[i].bytes >= need) {
           bytes = kept[i].bytes;
@@ -1311,10 +1366,11 @@ struct EvalSpace {
     if (d) return;
     if (cudaMalloc(&d, bytes) != cudaSuccess) d = nullptr;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) st = nullptr;
+    if (!ctx) ctx = primary_context(dev, true);  // the process's first call: the allocation has made the context
   }
   ~EvalSpace()
   {
-    if (good && bytes <= kEvalKeep && opts().eval_cache) {
+    if (good && ctx && bytes <= kEvalKeep && opts().eval_cache) {
       std::lock_guard<std::mutex> lk(mu);
       // the smallest goes first, so that the sizes in use are the ones kept
       if (kept.size() == kEvalSpaces) {
@@ -1322,27 +1378,35 @@ struct EvalSpace {
         for (size_t i = 1; i < kept.size(); ++i)
           if (kept[i].bytes < kept[k].bytes) k = i;
         if (kept[k].bytes < bytes) {
-          drop(kept[k]);
+          drop_kept(kept[k]);
           kept.erase(kept.begin() + k);
         }
       }
       if (kept.size() < kEvalSpaces) {
-        kept.push_back(Kept{dev, bytes, d, st});
+        kept.push_back(Kept{dev, ctx, bytes, d, st});
         return;
       }
     }
-    drop(Kept{dev, bytes, d, st});
+    drop(d, st);
     (void)cudaGetLastError();  // a failure here is the general path's to report
   }
-  static void drop(const Kept &k)
+  static void drop(unsigned char *d, cudaStream_t st)
   {
-    if (k.st) cudaStreamSynchronize(k.st), cudaStreamDestroy(k.st);
-    if (k.d) cudaFree(k.d);
+    if (st) cudaStreamSynchronize(st), cudaStreamDestroy(st);
+    if (d) cudaFree(d);
+  }
+  static void drop_kept(const Kept &k)
+  {
+    if (primary_context(k.dev, false) != k.ctx) return;
+    CUcontext c = nullptr;
+    const ContextCalls &d = ContextCalls::get_calls();
+    if (d.get(&c) == CUDA_SUCCESS && cudaSetDevice(k.dev) == cudaSuccess) drop(k.d, k.st);
+    d.set(c);
   }
   static void drop_all()
   {
     std::lock_guard<std::mutex> lk(mu);
-    for (const Kept &k : kept) drop(k);
+    for (const Kept &k : kept) drop_kept(k);
     kept.clear();
     (void)cudaGetLastError();
   }

@@ -35,6 +35,7 @@
 // dense terms into the lane totals with compensated summation and reduces
 // across lanes with a compensated butterfly; the FP64 variant evaluates the
 // reference's forms in double.
+#include <algorithm>
 #include <cstdio>
 #include <map>
 #include <mutex>
@@ -703,20 +704,17 @@ static McKernel pick_spec(int precision)
   return nullptr;
 }
 
-// Lets kernel f be launched with `bytes` of dynamic shared memory on the current device.  The limit only rises: a thread
-// that asks for less must not take it from under another's launch.
+// Lets kernel f be launched with `bytes` of dynamic shared memory in the current context.  The limit asked for only
+// rises: a thread that needs less must not take it from under another's launch.  It is set at every launch, since it
+// belongs to the context, and a process may have several or reset one.
 static cudaError_t allow_smem(McKernel f, size_t bytes)
 {
   static std::mutex mu;
-  static std::map<std::pair<McKernel, int>, size_t> allowed;
-  int dev = 0;
-  const cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
+  static std::map<McKernel, size_t> asked;
   std::lock_guard<std::mutex> lk(mu);
-  size_t &now = allowed[{f, dev}];
-  if (bytes <= now) return cudaSuccess;
-  const cudaError_t s = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (s == cudaSuccess) now = bytes;
+  size_t &most = asked[f];
+  const cudaError_t s = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(bytes, most));
+  if (s == cudaSuccess) most = std::max(bytes, most);
   return s;
 }
 
@@ -741,7 +739,7 @@ struct SpecLaunch {
 };
 
 // Occupancies of this process: they depend on the device, the kernel and the launch
-// alone, and a small pose call looks up more of them (45 us) than its kernel
+// alone, whatever the context, and a small pose call looks up more of them (45 us) than its kernel
 // takes.  Emptied when it has grown past any set of shapes in use.
 static int known_occupancy(McKernel f, int cluster, const TileConfig &tc, size_t smem, int (*look)(McKernel, const TileConfig &, size_t))
 {
