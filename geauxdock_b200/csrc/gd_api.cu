@@ -36,7 +36,7 @@ struct Options {
   int replica_warps = 1;     // warps per replica: 1 the library's choice, else fixed at 2, 4 or 8
   int device_base = 0;        // the drop-in API's GPU g is CUDA device device_base + g
   long long wait_limit = 0;   // microseconds of a bounded shared-memory wait (0: one second)
-  int stall_test = 0;         // test hook: staging barriers that never complete (bounded waits run out)
+  int stall_test = 0;         // test hook: staging (1) or cluster (2) barriers that never complete (bounded waits run out)
 };
 Options g_opt;
 int g_ngpu = -1;
@@ -114,7 +114,8 @@ struct gd_ensemble {
   // timing of the Monte Carlo launches
   std::vector<cudaEvent_t> ev;
   int ev_used = 0;
-  uint32_t wait_limit = 0, stall_bytes = 0;  // bounded-wait limit and the test hook (options)
+  uint32_t wait_limit = 0, stall_bytes = 0;  // bounded-wait limit and the test hooks (options)
+  bool stall_nodes = false;
   int launches = 0;      // Monte Carlo kernel launches (or graph replays of one)
   int all_launches = 0;  // every kernel of this library launched on the stream
   // pose evaluation's blocks (EvalBlock)
@@ -339,7 +340,8 @@ int finish_create(gd_ensemble *e)
   e->precision = o.precision;
   e->use_graph = o.graph != 0;
   e->wait_limit = (uint32_t)o.wait_limit;
-  e->stall_bytes = o.stall_test ? 16u : 0u;
+  e->stall_bytes = o.stall_test == 1 ? 16u : 0u;
+  e->stall_nodes = o.stall_test == 2;
   TileConfig tc{o.warps > 0 ? o.warps : 8, o.kpl, o.ab, o.stage != 0 ? 1 : 0, o.replica_warps};
   default_pair_tile(tc.kpl, tc.ab);
   if (e->precision == GD_PREC_FP64) tc.kpl = 1, tc.ab = 8, tc.group = 1;
@@ -413,7 +415,7 @@ KArgs mc_args(gd_ensemble *e, int s_begin, int nsteps, int flags, const int *d_s
   a.err = e->d_err;
   a.s_begin = s_begin;
   a.nsteps = nsteps;
-  a.flags = flags;
+  a.flags = flags | (e->stall_nodes ? kMcStallNodes : 0);
   a.d_step = d_step;
   a.P = e->tc.stage ? e->Pmax : 0;
   a.Pall = e->Pmax;
@@ -801,7 +803,7 @@ int gd_set_option(const char *name, long long v)
     if (v < 0 || v > 0xffffffffLL) return fail(GD_E_INVALID, "wait_limit = %lld", v);
     g_opt.wait_limit = v;
   } else if (n == "stall_test") {
-    if (v != 0 && v != 1) return fail(GD_E_INVALID, "stall_test = %lld", v);
+    if (v < 0 || v > 2) return fail(GD_E_INVALID, "stall_test = %lld", v);
     g_opt.stall_test = (int)v;
   } else if (n == "fail_alloc") {
     if (v < 0 || v > 1000000) return fail(GD_E_INVALID, "fail_alloc = %lld", v);

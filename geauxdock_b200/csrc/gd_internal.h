@@ -222,6 +222,7 @@ enum McFlags {
   kMcResetRecord = 2,    // this launch starts a dump chunk (next_entry = 0)
   kMcStoreAccept = 4,    // write the running accept flag into ReplicaMC.is_accept at the end
   kMcInitial = 8,        // initial-energy evaluation: no move, forced accept
+  kMcStallNodes = 16,    // test hook: a cluster's last CTA (gd_spec.cuh) awaits bytes that nobody sends
 };
 
 // Error flags written by kernels into a device word.

@@ -22,6 +22,12 @@
 // arrive and 900 for the tests.  A cluster barrier in place of the transaction
 // barrier takes 2,200, the tests one after the other along the path 2,600, and all
 // warps finishing the terms 1,200 more.  So a step is 1.8 us (one warp: 36 us).
+//
+// The wait for a round's energies is bounded as the staging waits are, by option
+// wait_limit, but by no less than kNodeWaitNs: it spans other CTAs' work (a CTA without
+// a node waits a whole energy).  A CTA that gives up leaves the rounds; the others
+// miss it in the next one.  They then tell each other how many rounds each has sent,
+// and each waits until all that was sent to it has arrived before it returns.
 #pragma once
 
 namespace gd {
@@ -30,6 +36,7 @@ constexpr int kSpecNodes = kMaxCluster;
 constexpr int kSpecRates = 10;   // rates of acceptance 0.05, 0.15, ...
 constexpr int kSpecRing = 64;    // steps whose random numbers are kept: a round and the next reach 31 steps ahead
 constexpr int kSpecRoot = 255;
+constexpr uint64_t kNodeWaitNs = 10000000ull;  // ten times the energy of 128 atoms x 20,000 points in FP64
 
 // Nodes in the order of their probability, so that the first n are the best n
 // and a node follows those on its path.
@@ -104,6 +111,28 @@ __device__ __forceinline__ void cluster_store_tx(uint32_t a, float v, uint32_t b
                : "memory");
 }
 
+// After some CTA of the cluster gave up (one thread): lets the energies still under way to this CTA arrive.  full: the
+// rounds' barriers, of which this CTA has armed those of the rounds before `mine`; sent[c]: rounds that CTA c has sent
+// (negative where it gave up).
+// The others differ from `mine` by one at most: whoever sent a round had received all of the one before.
+__device__ void spec_drain(uint64_t *full, int mine, bool complete, const int *sent, int ctas, uint32_t extra)
+{
+  int missing = 0, ahead = 0;
+  for (int c = 0; c < ctas; ++c) {
+    missing += abs(sent[c]) < mine;
+    ahead += abs(sent[c]) > mine;
+  }
+  if (!complete) {
+    const int last = mine - 1;
+    if (missing || extra) mbar_complete_tx(&full[last & 1], 40u * missing + extra);
+    (void)mbar_wait(&full[last & 1], (last >> 1) & 1, kWaitLimitNs);
+  }
+  if (ahead) {
+    mbar_expect_tx(&full[mine & 1], 40u * ahead);
+    (void)mbar_wait(&full[mine & 1], (mine >> 1) & 1, kWaitLimitNs);
+  }
+}
+
 // One replica (a work item of one) per cluster; the CTA of rank c has node c.
 template <int PREC, bool WIDE>
 __global__ void __maxnreg__(128) spec_kernel(KArgs A)
@@ -115,7 +144,7 @@ __global__ void __maxnreg__(128) spec_kernel(KArgs A)
   __shared__ double s_logu[kSpecRing];
   __shared__ float s_draw[8 * kSpecRing];
   __shared__ float s_node[2][kSpecNodes][12];  // a round's nodes: nine terms and the total; two rounds in turn
-  __shared__ int s_fail;
+  __shared__ int s_fail, s_sent[kSpecNodes];
   const int G = A.group, V = A.split, chunks = V > 1 ? 0 : team_chunks(G);
   const int sub = threadIdx.x >> 5, lane = lane_id();
   const int ctas = cluster_ctas(), mine = cluster_rank();
@@ -176,12 +205,15 @@ __global__ void __maxnreg__(128) spec_kernel(KArgs A)
       draw_steps(J, r, s0 + kDrawSteps * blocks, s_draw + 8 * kDrawSteps * blocks, s_logu + kDrawSteps * blocks);
   __syncthreads();
 
+  const uint64_t limit = A.wait_limit ? max(wait_limit_ns(A.wait_limit), kNodeWaitNs) : kWaitLimitNs;
+  const uint32_t extra = (A.flags & kMcStallNodes) && mine == ctas - 1 ? 16u : 0u;  // test hook
   bool alive = true;
-  for (int k = 0, round = 0; k < nsteps; ++round) {
+  int round = 0;
+  for (int k = 0; k < nsteps; ++round) {
     const SpecNode *tree = s_tree[max(0, min(kSpecRates - 1, (int)(kSpecRates * nacc / ntry)))];
     float (*nodes)[12] = s_node[round & 1];
     uint64_t *bar2 = &full[round & 1];
-    if (threadIdx.x == 0) mbar_expect_tx(bar2, 40u * ctas);
+    if (threadIdx.x == 0) mbar_expect_tx(bar2, 40u * ctas + extra);
     if (fill)
       // the next round starts at step k + 16 at most and reaches 15 further
       for (; kDrawSteps * blocks <= k + 31; ++blocks) {
@@ -204,7 +236,7 @@ __global__ void __maxnreg__(128) spec_kernel(KArgs A)
     if (sub == 0 && lane < 10)
       for (int c = 0; c < ctas; ++c) cluster_store_tx(cluster_map(&nodes[mine][lane], c), v, cluster_map(bar2, c));
     // one decision for the whole CTA: a warp that gave up and one that did not must not go separate ways
-    alive = __syncthreads_and(mbar_wait(bar2, (round >> 1) & 1, kWaitLimitNs) ? 1 : 0) != 0;
+    alive = __syncthreads_and(mbar_wait(bar2, (round >> 1) & 1, limit) ? 1 : 0) != 0;
     if (!alive) break;
 
     // lane n: the test of node n against the energy that its path leaves
@@ -243,7 +275,14 @@ __global__ void __maxnreg__(128) spec_kernel(KArgs A)
   }
   if (lead && alive) R.end(A, J, r, area.rep, area.stats, nsteps);
   if (!alive && threadIdx.x == 0) atomicOr(A.err, kErrTimeout);
-  cluster_sync();  // no CTA returns while another may still write to its shared memory
+  // no CTA returns while another may still write to its shared memory
+  const int sent = alive ? round : round + 1;
+  if (threadIdx.x < ctas) cluster_store(cluster_map(&s_sent[mine], threadIdx.x), alive ? sent : -sent);
+  cluster_sync();
+  bool all = true;
+  for (int c = 0; c < ctas; ++c) all &= s_sent[c] >= 0;
+  if (all || threadIdx.x > 0) return;
+  spec_drain(full, sent, alive, s_sent, ctas, extra);
 }
 
 }  // namespace gd

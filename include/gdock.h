@@ -120,10 +120,12 @@ int Dock(Complex *ch, Record *rh, Complex **cd, Record **rd, ParaT **pt, gd_rng_
  * drop-in API's GPU g is CUDA device device_base + g, for one process per GPU;
  * set it before SetDevice/DeviceAlloc and keep it), "wait_limit"
  * (microseconds, on the GPU's global timer, that the kernel's bounded
- * shared-memory waits last before they give up and report GD_E_TIMEOUT;
- * 0: one second), "stall_test" (test hook, 0 in normal
- * use: ensembles announce bytes to their staging barriers that no copy
- * delivers, so that the bounded waits run out), "fail_alloc" (test hook, 0 in
+ * shared-memory waits last before they give up and report GD_E_TIMEOUT, the
+ * wait of a cluster's CTAs for each other at least 10 ms; 0: one second),
+ * "stall_test" (test hook, 0 in normal
+ * use: ensembles announce bytes that nothing delivers, 1 to their staging
+ * barriers, 2 to the barriers of one CTA per cluster, so that the bounded
+ * waits run out), "fail_alloc" (test hook, 0 in
  * normal use: the next n device allocations for packing a job report
  * GD_E_NOMEM without calling cudaMalloc).  Applies to objects created
  * afterwards on the calling process. */
