@@ -1844,62 +1844,77 @@ int gd_ensemble_autotune(gd_ensemble_t *e, int steps, char *report, int report_l
     }
   };
   std::string rep;
-  TileConfig best = e->tc;
+  const TileConfig start = e->tc;
+  TileConfig best = start;
   double best_t = 1e300;
   const int shapes[][2] = {{1, 8}, {2, 4}, {2, 8}, {4, 4}, {4, 8}};
   const int warps[] = {4, 6, 8, 10, 12, 14, 16};
-  const int group = e->tc.group;  // kept
-  const int cluster = e->tc.cluster;  // kept by the candidates of one replica per CTA
-  const TileConfig smallest{std::max(4, group), e->tc.kpl, e->tc.ab, 1, group, e->tc.split};
+  const int group = start.group;  // kept
+  const int cluster = start.cluster;  // kept by the candidates of one replica per CTA
+  const TileConfig smallest{std::max(4, group), start.kpl, start.ab, 1, group, start.split};
   const bool can_stage = smem_for(e, smallest) <= kSmemLimit;
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device);
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);
-  for (int stage = can_stage ? 1 : 0; stage >= 0; --stage)
-  for (const auto &sh : shapes) {
-    // FP64 has the shape (1, 8), FP32 the others; a team's kernel has one shape whatever these say
-    if ((e->precision == GD_PREC_FP64) != (sh[0] == 1)) continue;
-    if (group > 1 && (sh[0] != e->tc.kpl || sh[1] != e->tc.ab)) continue;
-    for (int w : warps) {
-      if (rc != GD_OK) break;
-      // the warps per replica are kept; the candidates are the multiples of it
-      if (w % group) continue;
-      TileConfig tc{w, sh[0], sh[1], stage, group, e->tc.split, w == group ? cluster : 1};
-      if (configure(e, tc) != GD_OK || e->tc.stage != stage) continue;
-      // a strided sample of the work items (heaviest-first order kept), about two
-      // waves of the grid, so that a candidate runs the full chunk length
-      const int stride = std::max(1, e->n_items / std::max(1, 2 * e->grid));
-      std::vector<WorkItem> sample;
-      for (int i = 0; i < e->n_items; i += stride) sample.push_back(e->h_items[i]);
-      WorkItem *d_sample = nullptr;
-      if (cudaMalloc(&d_sample, sizeof(WorkItem) * sample.size()) != cudaSuccess ||
-          cudaMemcpyAsync(d_sample, sample.data(), sizeof(WorkItem) * sample.size(), cudaMemcpyHostToDevice,
-                          e->st) != cudaSuccess) {
-        cudaFree(d_sample);
-        rc = fail(GD_E_CUDA, "autotune sample");
-        break;
-      }
-      KArgs ka = mc_args(e, e->step, steps, 0, nullptr);
-      ka.items = d_sample;
-      ka.n_items = (int)sample.size();
-      float t = 0;
+  // times shape tc, already configured, `runs` times and keeps it where the last run is the fastest yet
+  auto time_shape = [&](const TileConfig &tc, int runs) {
+    // a strided sample of the work items (heaviest-first order kept), about two
+    // waves of the grid, so that a candidate runs the full chunk length
+    const int stride = std::max(1, e->n_items / std::max(1, 2 * e->grid));
+    std::vector<WorkItem> sample;
+    for (int i = 0; i < e->n_items; i += stride) sample.push_back(e->h_items[i]);
+    WorkItem *d_sample = nullptr;
+    if (cudaMalloc(&d_sample, sizeof(WorkItem) * sample.size()) != cudaSuccess ||
+        cudaMemcpyAsync(d_sample, sample.data(), sizeof(WorkItem) * sample.size(), cudaMemcpyHostToDevice,
+                        e->st) != cudaSuccess) {
+      cudaFree(d_sample);
+      rc = fail(GD_E_CUDA, "autotune sample");
+      return;
+    }
+    KArgs ka = mc_args(e, e->step, steps, 0, nullptr);
+    ka.items = d_sample;
+    ka.n_items = (int)sample.size();
+    float t = 0;
+    for (int k = 0; k < runs && rc == GD_OK; ++k) {
       cudaMemsetAsync(e->d_queue, 0, sizeof(int), e->st);
       cudaEventRecord(a, e->st);
       const cudaError_t le = launch_kernel(0, e->precision, e->tc, ka, std::min(e->grid, ka.n_items), e->st);
       cudaEventRecord(b, e->st);
       if (le != cudaSuccess || cudaStreamSynchronize(e->st) != cudaSuccess) rc = fail(GD_E_CUDA, "autotune launch");
       cudaEventElapsedTime(&t, a, b);
-      cudaFree(d_sample);
       restore();
-      t *= (float)e->n_items / (float)sample.size();   // per whole launch
-      char line[160];
-      snprintf(line, sizeof line, "warps=%d kpl=%d ab=%d stage=%d grid=%d items=%d: %.3f ms\n", w, sh[0], sh[1],
-               stage, e->grid, e->n_items, t);
-      rep += line;
-      if (t < best_t) {
-        best_t = t;
-        best = tc;
-      }
+    }
+    cudaFree(d_sample);
+    t *= (float)e->n_items / (float)sample.size();   // per whole launch
+    char line[160];
+    snprintf(line, sizeof line, "warps=%d kpl=%d ab=%d stage=%d wide=%d grid=%d items=%d: %.3f ms\n", tc.warps_per_cta,
+             tc.kpl, tc.ab, tc.stage, tc.wide ? 1 : 0, e->grid, e->n_items, t);
+    rep += line;
+    if (rc == GD_OK && t < best_t) {
+      best_t = t;
+      best = tc;
+    }
+  };
+  // the shape that the ensemble has, which the candidates need not contain (its first run warms up for all)
+  if (rc == GD_OK) rc = configure(e, start);
+  if (rc == GD_OK) time_shape(start, 2);
+  for (int stage = can_stage ? 1 : 0; stage >= 0; --stage)
+  for (const auto &sh : shapes) {
+    // FP64 has the shape (1, 8), FP32 the others; a team's kernel has one shape whatever these say
+    if ((e->precision == GD_PREC_FP64) != (sh[0] == 1)) continue;
+    if (group > 1 && (sh[0] != start.kpl || sh[1] != start.ab)) continue;
+    for (int w : warps) {
+      if (rc != GD_OK) break;
+      // the warps per replica are kept; the candidates are the multiples of it
+      if (w % group) continue;
+      TileConfig tc{w, sh[0], sh[1], stage, group, start.split, w == group ? cluster : 1};
+      // the kernel with more registers by choose_spread's rule
+      tc.wide = group == 1 && e->precision != GD_PREC_FP64 && sh[0] == 4 && sh[1] == 8 &&
+                (count_items(e, w) + nsm - 1) / nsm * w <= 16;
+      if (configure(e, tc) != GD_OK || e->tc.stage != stage) continue;
+      time_shape(tc, 1);
     }
   }
   cudaEventDestroy(a);
@@ -1911,8 +1926,8 @@ int gd_ensemble_autotune(gd_ensemble_t *e, int steps, char *report, int report_l
   e->all_launches = 0;
   if (rc == GD_OK) rc = configure(e, best);
   char line[160];
-  snprintf(line, sizeof line, "chosen: warps=%d kpl=%d ab=%d stage=%d\n", best.warps_per_cta, best.kpl, best.ab,
-           best.stage);
+  snprintf(line, sizeof line, "chosen: warps=%d kpl=%d ab=%d stage=%d wide=%d\n", best.warps_per_cta, best.kpl, best.ab,
+           best.stage, best.wide ? 1 : 0);
   rep += line;
   if (report && report_len > 0) {
     std::strncpy(report, rep.c_str(), (size_t)report_len - 1);

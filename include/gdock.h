@@ -270,7 +270,7 @@ int gd_ensemble_cluster(gd_ensemble_t *e, int job, int ref_lig, const float *ref
                         gd_cluster_t *clusters, int max_clusters, int *n_clusters, int *cluster_of,
                         float *rmsd_to_ref);
 /* Choose the tile shape (replicas per CTA, pair tile, pocket staging) by timing
- * candidates on a snapshot of the state (restored after each).  steps: MC
+ * the present one and candidates on a snapshot of the state (restored after each).  steps: MC
  * steps per launch to tune for (the chunk the caller runs, e.g. its exchange
  * interval); each candidate runs them on a strided sample of about two waves
  * of work items. */
