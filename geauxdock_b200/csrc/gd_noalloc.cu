@@ -6,8 +6,8 @@
 // start-up), where a raw cudaMalloc would take memory that allocator has
 // already accounted for; and latency-bound serving loops, where cudaFree
 // synchronises the whole device and would stall every other stream's docking
-// work.  gd_eval_poses() allocates device buffers for each call;
-// gd_eval_poses_noalloc() does the same work with caller-provided device
+// work.  gd_eval_poses() takes host buffers and a device block that it may have
+// to allocate; gd_eval_poses_noalloc() does the same work with caller-provided device
 // buffers for inputs and outputs, and keeps its own scratch (the packed
 // device layout of the Complex, written by the device packer of
 // gd_devpack.cu) in one fixed-size array declared below.
@@ -28,7 +28,8 @@
 // potential was.  4096 poses of 40 atoms x 1500 points x 11 conformations in FP32:
 // the former kernel, one type group of atoms at a time in scalar arithmetic, 991
 // us, now 450 us (bound by the pair loop as the Monte Carlo kernel is); the whole
-// call 1.27 -> 0.49 ms.
+// call 1.27 -> 0.49 ms.  A pose's FP32 sums are combined in one of two orders, by the
+// number of poses sent with it (na_tile, noalloc_shape).
 #include <algorithm>
 #include <mutex>
 
@@ -84,7 +85,12 @@ NaShapes g_na_shape[kNaMaxDevices][3];
 // call against 495) but their longer chains of plain additions lose more: rms error
 // of the raw terms against 64 bits, 40 x 1500, 20 x 400 and 64 x 2048, 1.6, 0.85 and
 // 1.3e-7 against 0.88, 0.62 and 0.79e-7 (the former kernel of this call: 1.9, 0.77
-// and 0.87e-7).
+// and 0.87e-7).  Over eight sizes from 8 x 200 to 64 x 2048, against that kernel's rms
+// error in the same precision (geometric means): FP32 0.75-0.92 times in vdw, ele, pmf,
+// hpc and the total on one warp, 0.77-0.96 in teams; FP32_KAHAN 0.77-1.00 on one warp, in
+// teams vdw 1.18 and the total 1.04 (the two shares' sums are rounded once more before
+// they are added), the others 0.77-1.00; single terms at single sizes up to 1.39 (ele at
+// 20 x 400).
 TileConfig na_tile(int precision, int lg, int R)
 {
   const bool fp64 = precision == kFP64;

@@ -145,7 +145,13 @@ int gd_eval_poses(const Complex *c, int n, const int *conf, const float *mm, int
  * docking call: a process whose device memory belongs to another allocator
  * (a framework's caching allocator, a pool reserved at start-up), or a
  * latency-bound serving loop that cannot afford cudaFree's device-wide
- * synchronisation.  Same result as gd_eval_poses, but every pointer is device
+ * synchronisation.  The energies of gd_eval_poses: the same bits in FP64; in
+ * FP32 equal to rounding, and two calls that send a pose along with different
+ * numbers of others may differ by rounding too: up to about 12 poses per SM (one
+ * wave of teams of warps) the sums are combined in the order of a replica
+ * split over two warps, above that in one warp's, and within each of the two a
+ * pose's bits do not depend on n.  GD_PREC_FP32 runs with compensated sums,
+ * as GD_PREC_FP32_KAHAN, and gives its bits.  Every pointer is device
  * memory the caller owns: d_complex is a reference-layout Complex (for
  * example cd[g] after CopyH2D), d_conf[n][2] / d_mm[n][6] the poses,
  * d_out[n][10] and d_raw[n][9] (may be NULL) the energies; stream is a
