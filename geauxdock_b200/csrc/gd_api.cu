@@ -33,7 +33,7 @@ struct Options {
   int dock_cache = 1;  // Dock keeps its device state per GPU between calls
   int dock_device_pack = 1;  // Dock refills that state on the GPU from the Complex CopyH2D put there
   int dock_record_direct = 1;  // Dock's kernels write Records straight into a GPU-mapped host array
-  int replica_warps = 1;     // warps per replica: 1 the library's choice, else fixed at 2, 4 or 8
+  int replica_warps = 1;     // order of the energy sums: 1 the one-warp kernel's, 2, 4 or 8 that of a replica split over so many
   int device_base = 0;        // the drop-in API's GPU g is CUDA device device_base + g
   long long wait_limit = 0;   // microseconds of a bounded shared-memory wait (0: one second)
   int stall_test = 0;         // test hook: staging (1) or cluster (2) barriers that never complete (bounded waits run out)

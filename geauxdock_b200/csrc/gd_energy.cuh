@@ -5,7 +5,7 @@
 // arithmetic does not depend on who evaluates them -- 128-point rows of the pair
 // loop, 8-atom blocks of the hydrophobic contact, 32-point chunks of the KDE and
 // of the pocket-specific walk -- and the units are combined in the one-warp
-// kernel's order.  Every multiply-add below is written out (__fmaf_rn and the
+// kernel's order (or both times in that of a split, where one is asked for).  Every multiply-add below is written out (__fmaf_rn and the
 // like), so that the compiler's own contraction cannot differ between the two
 // places a function is inlined.
 #pragma once
@@ -299,8 +299,8 @@ __device__ __forceinline__ float4 pass1_row(const LigPair *lp, int npairs, int r
 
 // Component c of pass1_row<4>'s sums, alone: the terms of atoms c, c + 2, ... (of
 // the atom pairs) against the 128 points from `row`, in scalar arithmetic, the
-// same operations in the same order; pass1_join gives pass1_row's sums from the
-// two components.  Two warps then share a row, where a team has warps to spare.
+// same operations in the same order; a team joins the two components to pass1_row's
+// sums where it combines its units.  Two warps then share a row, where a team has warps to spare.
 struct HalfRow {
   float vdw, pmf, hdb, ele[4];
 };

@@ -15,8 +15,8 @@
 //                        tab2[24][32] float2 (hdb1 c, -hdb0 hdb1 c), zero where hdb0 <= 0.1
 //                        ref4[24][32] float4 (p1a, p2a, hdb0, hdb1) as in EnePara (FP64, plain)
 //   ligand conformation  lig[L] float4 (x, y, z, charge), atoms grouped by type; the
-//                        rotated pose of a replica lives in shared memory with
-//                        every value twice (packed f32x2 operands)
+//                        rotated pose of a replica lives in shared memory as atom
+//                        pairs (packed f32x2 operands)
 //   KDE points           kde[K] float4 (x, y, z, type), sorted by type, with
 //                        per-type ranges
 //   MCS templates        mcs[L][M] float4 (x, y, z, valid), atom-major
@@ -64,10 +64,10 @@ __host__ __device__ inline float4 tab4_entry(float p1a, float p2a, float pmf0, f
 }
 __host__ __device__ inline float4 tab4_padding() { return make_float4(INFINITY, 0.f, 0.f, 0.f); }
 
-// The scalar parameters come first and the per-type tables last: the FP32
-// batched kernel stages only the scalar prefix in shared memory (it reads the
-// tables from global memory once per work item to build its per-atom-pair
-// tables); the FP64 and plain kernels stage the whole struct.
+// The scalar parameters come first and the per-type tables last: the batched
+// kernels stage only the scalar prefix in shared memory (they read the tables
+// from global memory once per work item to build their own, per atom pair in
+// FP32, per type group in FP64); the plain kernel stages the whole struct.
 struct alignas(16) DevParams {
   uint32_t hdbmask[kLigTypes];        // bit pt set where (ligand type, point type) has hdb0 > 0.1
   float hpl0[kLigTypes], hpl1[kLigTypes], hpl2[kLigTypes];

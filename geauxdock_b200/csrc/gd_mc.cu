@@ -7,8 +7,8 @@
 // (src/backend_gpu/kernel_cuda_l1_montecarlo.cu:284-527).  Here one warp owns
 // one replica for a whole chunk of steps: the step needs no block barrier,
 // only warp shuffles.  A CTA holds R replica-warps that share one protein
-// conformation; per work item the CTA stages the force-field parameters (in
-// FP64 also the KDE points; when it pays, the conformation itself) into shared
+// conformation; per work item the CTA stages the force-field parameters (when it
+// pays, also the conformation itself) into shared
 // memory with 1-D bulk (TMA) copies, and its replica-warps read them every
 // step.  A persistent grid takes work items from an atomic queue, heaviest
 // first.
@@ -33,8 +33,9 @@
 // the single-instruction PTX approximations (rsqrt/rcp/ex2.approx).  The
 // FP32-Kahan variant (the default) adds each row's partial sums of the three
 // dense terms into the lane totals with compensated summation and reduces
-// across lanes with a compensated butterfly; the FP64 variant evaluates the
-// reference's forms in double.
+// across lanes with a compensated butterfly; the FP64 variant evaluates the same
+// rearrangement of the Lennard-Jones term and the other terms as they stand in
+// double, with special functions of its own (gd_energy.cuh).
 #include <algorithm>
 #include <cstdio>
 #include <map>

@@ -132,7 +132,11 @@ static double step_cycles(const ShapeQuery &q, const TileConfig &tc, long long s
 // 431 and 217 us, against 800 points 140 and 106 us; but of 40, 42 and 45 atoms
 // 266 and 305 us, of 80 alone 493 and 543 us.  So by the model above, where it
 // says an eighth less (teams of 8 and 16 are not: their few half rows per warp
-// follow no such rule).
+// follow no such rule).  The model's constants are those of the FP32 loop; in FP64 it
+// was measured by itself, over eight mixes of ligands x 300, 800 and 2200 points x 4, 8 and
+// 12 temperatures (600 to 4200 replicas): where it chooses waves they are 1.1 to 3 times as
+// fast as the shape before (20, 45 and 80 atoms x 2200, 1200 replicas, 1500 -> 789 us
+// a step; 80 alone, 2400 replicas, 2937 -> 2426), and elsewhere it leaves the shape.
 void choose_waves(const ShapeQuery &q, TileConfig &tc, int &grid)
 {
   if (q.mode != 0 || !q.loads || tc.group > 4 || (tc.split == 1 && q.precision != kFP64 && (tc.kpl != 4 || tc.ab != 8)))
