@@ -1311,7 +1311,7 @@ struct ContextCalls {
 
 // The id of device dev's primary context (no two contexts of a process have the same; a reset context's successor has
 // another), 0 where there is none or the driver does not tell.  With `current`, 0 too where the calling thread's context
-// is another one.
+// is another one (a thread without one gets the primary one from the runtime).
 unsigned long long primary_context(int dev, bool current)
 {
   const ContextCalls &d = ContextCalls::get_calls();
@@ -1320,9 +1320,9 @@ unsigned long long primary_context(int dev, bool current)
   CUcontext c = nullptr, p = nullptr;
   unsigned long long id = 0;
   if (!d.ok || d.state(dev, &flags, &active) != CUDA_SUCCESS || !active) return 0;
-  if (current && (d.get(&c) != CUDA_SUCCESS || !c)) return 0;
+  if (current && d.get(&c) != CUDA_SUCCESS) return 0;
   if (d.retain(&p, dev) != CUDA_SUCCESS) return 0;
-  if ((current && c != p) || d.id(p, &id) != CUDA_SUCCESS) id = 0;
+  if ((c && c != p) || d.id(p, &id) != CUDA_SUCCESS) id = 0;
   d.release(dev);
   return id;
 }
