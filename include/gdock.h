@@ -279,7 +279,7 @@ int gd_ensemble_cluster(gd_ensemble_t *e, int job, int ref_lig, const float *ref
  * the present one and candidates on a snapshot of the state (restored after each).  steps: MC
  * steps per launch to tune for (the chunk the caller runs, e.g. its exchange
  * interval); each candidate runs them on a strided sample of about two waves
- * of work items. */
+ * of work items, the fastest few and the present one on twelve again. */
 int gd_ensemble_autotune(gd_ensemble_t *e, int steps, char *report, int report_len);
 int gd_ensemble_destroy(gd_ensemble_t *e);
 /* Checkpoint and resume of a resident ensemble: every replica's ReplicaMC,

@@ -1,6 +1,7 @@
-"""gd_ensemble_autotune times the shape an ensemble has before its candidates, and
-gives these the kernel with 128 registers where 16 or fewer warps share an SM: tuning
-does not lose a shape that only the library's own choice has."""
+"""gd_ensemble_autotune times the shape an ensemble has before its candidates, gives
+these the kernel with 128 registers where 16 or fewer warps share an SM, and times the
+few that its short samples cannot tell apart on longer ones: tuning does not leave
+an ensemble slower than it was."""
 
 import numpy as np
 import pytest
@@ -10,16 +11,14 @@ from geauxdock_b200 import dock, synth
 pytestmark = pytest.mark.gpu
 
 
-def _tuned(enepara, atoms, points, nlig, nprt, ntmp, steps):
+def _ensemble(enepara, atoms, points, nlig, nprt, ntmp):
     rng = np.random.default_rng(2)
     pk = synth.make_pocket(rng, points, nprt)
     jobs = [synth.make_job(rng, pk, L, nlig, 60, 5, synth.ladder(ntmp, 0.3, 3.0), seed=i) for i, L in enumerate(atoms)]
-    with dock.Ensemble.from_jobs([pk], jobs, enepara) as e:
-        e.init()
-        e.sync()
-        lines = e.autotune(steps).strip().splitlines()
-        again = e.autotune(steps).strip().splitlines()
-    return lines, again
+    e = dock.Ensemble.from_jobs([pk], jobs, enepara)
+    e.init()
+    e.sync()
+    return e
 
 
 def _of(line):
@@ -32,18 +31,44 @@ def _ms(line):
 
 def test_present_shape_is_a_candidate(lib, enepara):
     # 1200 replicas in teams of two
-    lines, again = _tuned(enepara, (60, 60, 60), 700, 10, 5, 8, 6)
-    chosen = _of(lines[-1])
-    # whatever was chosen was the fastest timed, the first among them, and is the first of the next tuning
-    least = min(map(_ms, lines[:-1]))
-    assert any(all(_of(x)[k] == chosen[k] for k in chosen) for x in lines[:-1] if _ms(x) == least)
-    assert all(_of(again[0])[k] == chosen[k] for k in chosen)
+    with _ensemble(enepara, (60, 60, 60), 700, 10, 5, 8) as e:
+        lines = e.autotune(6).strip().splitlines()
+        later = e.autotune(6).strip().splitlines()
+    chosen, again = _of(lines[-1]), [x for x in lines if x.startswith("again:")]
+    keys = ("warps", "kpl", "ab", "stage", "wide")
+    # the present shape is the first of both lists, and stays unless another is 1 % faster on the longer sample
+    assert all(_of(lines[0])[k] == _of(again[0])[k] for k in keys)
+    least = min(map(_ms, again))
+    assert any(all(_of(x)[k] == chosen[k] for k in keys) for x in again if _ms(x) == least) or (
+        all(_of(again[0])[k] == chosen[k] for k in keys) and _ms(again[0]) <= 1.02 * least)
+    # and is the first of the next tuning
+    assert all(_of(later[0])[k] == chosen[k] for k in keys)
 
 
 def test_wide_kernel_stays_where_it_is_faster(lib, enepara):
     # 80 atoms against 2200 points: 402 us a step with 80 registers, 353 with 128 (8 warps per SM)
-    lines, _ = _tuned(enepara, (80, 80, 80), 2200, 10, 5, 8, 10)
+    with _ensemble(enepara, (80, 80, 80), 2200, 10, 5, 8) as e:
+        lines = e.autotune(10).strip().splitlines()
     first = _of(lines[0])
     assert first["wide"] == 1 and first["kpl"] == 4 and first["ab"] == 8
     assert any(_of(x)["wide"] == 1 for x in lines[1:-1])
     assert _of(lines[-1])["wide"] == 1
+
+
+def test_tuned_is_not_slower(lib, enepara):
+    # the screening workload, 512 ligands of 12 to 64 atoms, 204,800 replicas: many waves of uneven work items, whose
+    # launches repeat to 0.2 %
+    pk, jobs = synth.config3(seed=1, nligand=512)
+    with dock.Ensemble.from_jobs([pk], jobs, enepara) as e:
+        def ms():
+            times = []
+            for _ in range(2):
+                e.run(20)
+                times.append(e.sync()[0])
+            return min(times)
+
+        e.init()
+        e.sync()
+        before = ms()
+        e.autotune(50)
+        assert ms() <= 1.01 * before
