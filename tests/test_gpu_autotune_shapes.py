@@ -57,18 +57,16 @@ def test_wide_kernel_stays_where_it_is_faster(lib, enepara):
 
 def test_tuned_is_not_slower(lib, enepara):
     # the screening workload, 512 ligands of 12 to 64 atoms, 204,800 replicas: many waves of uneven work items, whose
-    # launches repeat to 0.2 %
+    # launches repeat to 0.2 %; the tuned ensemble and an untuned one in turn
     pk, jobs = synth.config3(seed=1, nligand=512)
-    with dock.Ensemble.from_jobs([pk], jobs, enepara) as e:
-        def ms():
-            times = []
-            for _ in range(2):
+    with dock.Ensemble.from_jobs([pk], jobs, enepara) as tuned, dock.Ensemble.from_jobs([pk], jobs, enepara) as plain:
+        for e in (tuned, plain):
+            e.init()
+            e.sync()
+        tuned.autotune(50)
+        ms = {tuned: [], plain: []}
+        for _ in range(3):
+            for e, times in ms.items():
                 e.run(20)
                 times.append(e.sync()[0])
-            return min(times)
-
-        e.init()
-        e.sync()
-        before = ms()
-        e.autotune(50)
-        assert ms() <= 1.01 * before
+    assert min(ms[tuned]) <= 1.01 * min(ms[plain])
